@@ -419,6 +419,97 @@ __global__ void __launch_bounds__(256) k_stress_adj_gather3(GamBox b, Range r0, 
 }
 
 
+// Face fluxes of direction D (Fluxes, stress.F90:204-429), one face per
+// thread. The stencil operands are the per-cell products volume*primitive and
+// volume*B of the half state (QdV of Cen8LRs) and the limiter values, read
+// along D through L1 (the callers' unpadded boxes have rows that a TMA copy
+// cannot start on). SAVE (the whole step's forward) also stores the face
+// states in w.fsv.
+template <class R, int D, int MINB, bool SAVE = false>
+__global__ void __launch_bounds__(128, MINB) k_stress_box(GamBox b, DevParams<R> P, Geo<R> g, const R* __restrict__ Blim,
+                                                      Work<R> w, Range r, const GamScalars* sc) {
+    if (sc->halted) return;
+    int ii, jj, kk;
+    if (!thread_ijk(r, ii, jj, kk)) return;
+    const long fs = b.fs;
+    const long c = lidx(b, ii, jj, kk);
+    const long s = D == 0 ? 1L : (D == 1 ? (long)b.sx : b.sk);
+    GAM_BOX_CHECK(c - 4 * s, c + 3 * s, 8 + D);
+    R T[9];
+#pragma unroll
+    for (int n = 0; n < 9; n++) T[n] = g.Tf[(n + 9 * D) * fs + c];
+    const R fa = g.face[D * fs + c];
+    R vol[8];
+#pragma unroll
+    for (int n = 0; n < 8; n++) vol[n] = g.vol[c + (n - 4) * s];
+    const Quot<R> Vi(central8(vol));
+    R MagL[3] = {(R)0, (R)0, (R)0}, MagR[3] = {(R)0, (R)0, (R)0};
+    R Bn = (R)0;
+    double B0[3] = {0.0, 0.0, 0.0}, B0n = 0.0;
+    if (P.doMHD) {
+        Bn = w.Bnf[D * fs + c];
+#pragma unroll
+        for (int x = 0; x < 3; x++) {
+            R q[8], nq[4];
+            const R* qp = w.QB + x * fs + c - 4 * s;
+            const R* lp = Blim + x * fs + c - 2 * s;
+#pragma unroll
+            for (int n = 0; n < 8; n++) q[n] = qp[n * s];
+#pragma unroll
+            for (int m = 0; m < 4; m++) nq[m] = lp[m * s];
+            lrs_from_qdv(P, q, nq, Vi, MagL[x], MagR[x]);
+        }
+        if (P.doBackground) {
+#pragma unroll
+            for (int x = 0; x < 3; x++) B0[x] = g.fcB0[(x + 3 * D) * fs + c];
+            B0n = qdiv(g.bFlux0[D * fs + c], (double)fa);
+        }
+    }
+    R WL[5], WR[5];
+#pragma unroll
+    for (int v = 0; v < 5; v++) {
+        R q[8], nq[4];
+        const R* qp = w.QW + v * fs + c - 4 * s;
+        const R* lp = w.Wn + v * fs + c - 2 * s;
+#pragma unroll
+        for (int n = 0; n < 8; n++) q[n] = qp[n * s];
+#pragma unroll
+        for (int m = 0; m < 4; m++) nq[m] = lp[m * s];
+        lrs_from_qdv(P, q, nq, Vi, WL[v], WR[v]);
+    }
+    R VaD = (R)0, bbD = (R)0;
+    if (P.doMHD) {
+        R mF[3] = {(R)0, (R)0, (R)0};
+        mag_kin_flux<R>(P, (R)-1, WL, MagL, Bn, T, B0, B0n, mF, bbD, VaD);
+        mag_kin_flux<R>(P, (R)1, WR, MagR, Bn, T, B0, B0n, mF, bbD, VaD);
+#pragma unroll
+        for (int x = 0; x < 3; x++) w.mF[(x + 3 * D) * fs + c] = fa * mF[x];
+    }
+    R gF[5] = {(R)0, (R)0, (R)0, (R)0, (R)0}, dW[5] = {(R)0, (R)0, (R)0, (R)0, (R)0};
+    gas_kin_flux(P, (R)-1, WL, T, gF, dW);
+    gas_kin_flux(P, (R)1, WR, T, gF, dW);
+    R gv[5];
+#pragma unroll
+    for (int v = 0; v < 5; v++) gv[v] = gF[v] - (R)1 * P.cHogH * VaD * dW[v];
+#pragma unroll
+    for (int v = 0; v < 5; v++) w.gF[(v + 5 * D) * fs + c] = fa * gv[v];
+    if constexpr (SAVE) {
+        R* o = w.fsv + (long)(GAM_FSV_NC * D) * fs + c;
+#pragma unroll
+        for (int v = 0; v < 5; v++) {
+            o[v * fs] = WL[v];
+            o[(5 + v) * fs] = WR[v];
+            o[(17 + v) * fs] = dW[v];
+        }
+#pragma unroll
+        for (int x = 0; x < 3; x++) {
+            o[(10 + x) * fs] = MagL[x];
+            o[(13 + x) * fs] = MagR[x];
+        }
+        o[16 * fs] = VaD;
+    }
+}
+
 // reverse of edge_lrs (EdgeLRs for faces of direction a along bd): adjoints of
 // bL*Vi, bR*Vi -> the abh (8) and bn (4) stencils
 template <class R, class A>
@@ -1465,13 +1556,13 @@ int flux_call(const gam_params* p, const void* QW, const void* Wn, const void* Q
     };
     const R* Bl = (const R*)Blim;
     if (!dgF && fstates) {
-        k_stress<R, 0, 1, false, true><<<grid(fr[0]), blk, 0, s>>>(b, P, g, Bl, w, fr[0], sc, nullptr, nullptr);
-        k_stress<R, 1, 1, false, true><<<grid(fr[1]), blk, 0, s>>>(b, P, g, Bl, w, fr[1], sc, nullptr, nullptr);
-        k_stress<R, 2, 1, false, true><<<grid(fr[2]), blk, 0, s>>>(b, P, g, Bl, w, fr[2], sc, nullptr, nullptr);
+        k_stress_box<R, 0, 1, true><<<grid(fr[0]), blk, 0, s>>>(b, P, g, Bl, w, fr[0], sc);
+        k_stress_box<R, 1, 1, true><<<grid(fr[1]), blk, 0, s>>>(b, P, g, Bl, w, fr[1], sc);
+        k_stress_box<R, 2, 1, true><<<grid(fr[2]), blk, 0, s>>>(b, P, g, Bl, w, fr[2], sc);
     } else if (!dgF) {
-        k_stress<R, 0, 1><<<grid(fr[0]), blk, 0, s>>>(b, P, g, Bl, w, fr[0], sc, nullptr, nullptr);
-        k_stress<R, 1, 1><<<grid(fr[1]), blk, 0, s>>>(b, P, g, Bl, w, fr[1], sc, nullptr, nullptr);
-        k_stress<R, 2, 1><<<grid(fr[2]), blk, 0, s>>>(b, P, g, Bl, w, fr[2], sc, nullptr, nullptr);
+        k_stress_box<R, 0, 1><<<grid(fr[0]), blk, 0, s>>>(b, P, g, Bl, w, fr[0], sc);
+        k_stress_box<R, 1, 1><<<grid(fr[1]), blk, 0, s>>>(b, P, g, Bl, w, fr[1], sc);
+        k_stress_box<R, 2, 1><<<grid(fr[2]), blk, 0, s>>>(b, P, g, Bl, w, fr[2], sc);
     } else if (fstates) {
         R* rs = (R*)rscratch;
         const long fs40 = 40L * b.fs;

@@ -43,6 +43,8 @@ void gam_geom_dxf(const GamBox& b, const double* xfc, const double* xyzcc, float
 void gam_geom_metric(const GamBox& b, const double* xyz, double* face, double* xfc, double* Tf, double* vol,
                      double* xyzcc, double* dijk, double* dl, double* edge, double* Te, double* Teb,
                      const GamRingGeo& ring, cudaStream_t s);
+void gam_geom_tables_d(const GamBox& b, const double* vol, double* vif, double* rvif, cudaStream_t s);
+void gam_geom_tables_f(const GamBox& b, const double* vol, float* vif, float* rvif, cudaStream_t s);
 void gam_geom_ic_ot(const GamBox& b, const double* xyzcc, const double* face, double* Gas, double* mf, double gamma,
                     cudaStream_t s);
 void gam_geom_ic_case(const GamBox& b, const double* xyz, const double* xyzcc, const double* vol, double* Gas,
@@ -102,6 +104,7 @@ struct gam_handle {
     Ctx<double> cd{};
     Ctx<float> cf{};
     GamScalars* sc = nullptr;   // device
+    GamFluxMapSet fmaps;        // tensor maps of the flux kernels
     double* staging = nullptr;  // device, Fortran-layout transfer buffer
     double* partial = nullptr;  // device, reduction partials
     double* dres = nullptr;     // device, reduction results
@@ -187,6 +190,43 @@ template <class R> static void fill_dev_params(DevParams<R>& P, const gam_params
     P.dtIlo = P.dtIhi = P.dtJlo = P.dtJhi = 1;
 }
 
+// The tensor maps of the flux kernels' boxes (FluxTile): fields of nc
+// components over the box, components fs apart
+template <class R>
+static bool encode_box(const GamBox& b, const R* base, int nc, int bx, int by, int bz, CUtensorMap* m) {
+    typedef CUresult (*Encode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                               const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                               CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+        return false;
+    const cuuint64_t dim[4] = {(cuuint64_t)b.sx, (cuuint64_t)(b.Nj + 1), (cuuint64_t)(b.Nk + 1), (cuuint64_t)nc};
+    const cuuint64_t str[3] = {b.sx * sizeof(R), b.sk * sizeof(R), b.fs * sizeof(R)};
+    const cuuint32_t box[4] = {(cuuint32_t)bx, (cuuint32_t)by, (cuuint32_t)bz, (cuuint32_t)nc}, es[4] = {1, 1, 1, 1};
+    return ((Encode)f)(m, sizeof(R) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
+                       (void*)base, dim, str, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                       CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+template <class R, int D> static bool flux_maps_of(gam_handle* h, Ctx<R>& C) {
+    using T_ = FluxTile<R, D>;
+    const GamBox& b = h->b;
+    const int qy = D == 1 ? T_::QN : (D == 0 ? T_::TN : 1), qz = D == 2 ? T_::QN : 1;
+    const int ly = D == 1 ? T_::LN : (D == 0 ? T_::TN : 1), lz = D == 2 ? T_::LN : 1;
+    for (int cur = 0; cur < 2; cur++) {
+        GamFluxMaps& m = h->fmaps.m[cur][D];
+        const R* Bl = h->p.doLFMLim ? C.st[cur].B : C.w.Bl;
+        if (!encode_box<R>(b, C.w.QW, 5, T_::QX, qy, qz, &m.QW) || !encode_box<R>(b, C.w.QB, 3, T_::QX, qy, qz, &m.QB) ||
+            !encode_box<R>(b, C.w.Wn, 5, T_::QX, ly, lz, &m.Wn) || !encode_box<R>(b, Bl, 3, T_::QX, ly, lz, &m.Bl))
+            return false;
+    }
+    return true;
+}
+template <class R> static bool make_flux_maps(gam_handle* h, Ctx<R>& C) {
+    return flux_maps_of<R, 0>(h, C) && flux_maps_of<R, 1>(h, C) && flux_maps_of<R, 2>(h, C);
+}
+
 template <class R> static int alloc_bulk(gam_handle* h, Ctx<R>& C) {
     cudaError_t e = cudaSuccess;
     const long fs = h->b.fs;
@@ -226,7 +266,18 @@ template <class R> static int alloc_bulk(gam_handle* h, Ctx<R>& C) {
         C.g.vol = vol; C.g.xyzcc = xyzcc; C.g.dl = dl; C.g.face = face; C.g.xfc = xfc; C.g.Tf = Tf;
         C.g.edge = edge; C.g.Te = Te; C.g.Teb = Teb; C.g.dxf = dxf;
     }
+    {
+        // the strict form divides by the interpolated volume, the others
+        // multiply by its reciprocal
+        R *vif = nullptr, *rvif;
+        if (h->p.strict) A(vif, 3);
+        A(rvif, 3);
+        C.g.vif = vif;
+        C.g.rvif = rvif;
+    }
 #undef A
+    if (!make_flux_maps(h, C)) return fail(h, GAM_ECUDA, "cuTensorMapEncodeTiled failed");
+    C.fmaps = &h->fmaps;
     C.g.fcB0 = h->bg.fcB0;
     C.g.bFlux0 = h->bg.bFlux0;
     C.g.edgB0 = h->bg.edgB0;
@@ -417,8 +468,13 @@ template <class R> static int down_r(gam_handle* h, const R* src, double* dst, b
 }
 
 // FP32 form: round the FP64 metric once into the FP32 copies
-static void sync_geo_f32(gam_handle* h) {
-    if (!h->f32) return;
+// the compute form's copies and tables of a geometry just set
+static void sync_geo(gam_handle* h) {
+    if (!h->f32) {
+        const Geo<double>& g = h->cd.g;
+        gam_geom_tables_d(h->b, h->gd.vol, (double*)g.vif, (double*)g.rvif, h->s);
+        return;
+    }
     Geo<float>& g = h->cf.g;
     const long fs = h->b.fs;
     gam_geom_d2f(h->gd.vol, (float*)g.vol, fs, h->s);
@@ -431,6 +487,7 @@ static void sync_geo_f32(gam_handle* h) {
     gam_geom_d2f(h->gd.Te, (float*)g.Te, 27 * fs, h->s);
     gam_geom_d2f(h->gd.Teb, (float*)g.Teb, 12 * fs, h->s);
     gam_geom_dxf(h->b, h->gd.xfc, h->gd.xyzcc, (float*)g.dxf, h->s);
+    gam_geom_tables_f(h->b, h->gd.vol, (float*)g.vif, (float*)g.rvif, h->s);
 }
 
 static bool has_lfm(const gam_handle* h) { return h->p.bc[2] == GAM_BC_LFM || h->p.bc[3] == GAM_BC_LFM; }
@@ -544,7 +601,7 @@ extern "C" int gam_set_geometry(gam_handle* h, const double* xyz) {
     GeoD& g = h->gd;
     gam_geom_metric(h->b, g.xyz, g.face, g.xfc, g.Tf, g.vol, g.xyzcc, g.dijk, g.dl, g.edge, g.Te, g.Teb, h->ringGeo,
                     h->s);
-    sync_geo_f32(h);
+    sync_geo(h);
     CK(h, cudaGetLastError());
     CK(h, cudaStreamSynchronize(h->s));
     h->haveGeo = true;
@@ -572,7 +629,7 @@ extern "C" int gam_set_geometry_arrays(gam_handle* h, const double* face, const 
     if ((rc = up_d(h, Te, g.Te, true, 27))) return rc;
     if ((rc = up_d(h, Teb, g.Teb, true, 12))) return rc;
     gam_diag_min3(h->b, g.dijk, g.dl, h->s);
-    sync_geo_f32(h);
+    sync_geo(h);
     CK(h, cudaGetLastError());
     CK(h, cudaStreamSynchronize(h->s));
     h->haveGeo = true;

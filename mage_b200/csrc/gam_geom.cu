@@ -333,6 +333,31 @@ __global__ void k_geo_teb(GamBox b, const double* __restrict__ face, const doubl
     Teb[(c0 + 1 + 4 * dNorm) * fs + c] = dyT / dScl;
 }
 
+// Geometry-only operands of the step's reconstructions, in FP64 and in the
+// step's evaluation order, rounded once to T: the 8CENT interpolant of the
+// volumes along d at the faces of direction d, and its reciprocal
+__device__ __forceinline__ double cen8(const double* q, long s) {
+    const double w[8] = {-3.0 / 840.0, 29.0 / 840.0, -139.0 / 840.0, 533.0 / 840.0,
+                         533.0 / 840.0, -139.0 / 840.0, 29.0 / 840.0, -3.0 / 840.0};
+    double a = 0.0;
+    for (int n = 0; n < 8; n++) a += w[n] * q[(n - 4) * s];
+    return a;
+}
+template <class T>
+__global__ void k_geo_tables(GamBox b, const double* __restrict__ vol, T* __restrict__ vif, T* __restrict__ rvif) {
+    int ii, jj, kk;
+    if (!tid3(b.Ni, b.Nj, b.Nk, ii, jj, kk)) return;
+    const long c = lidx(b, ii, jj, kk);
+    const int x[3] = {ii, jj, kk}, N[3] = {b.Ni, b.Nj, b.Nk};
+    const long st[3] = {1L, (long)b.sx, b.sk};
+    for (int d = 0; d < 3; d++) {
+        if (x[d] < 4 || x[d] > N[d] - 4) continue;  // cells -4..3 of the face
+        const double v = cen8(vol + c, st[d]);
+        if (vif) vif[d * b.fs + c] = (T)v;
+        rvif[d * b.fs + c] = (T)(1.0 / v);
+    }
+}
+
 // ------------------------------------------------------------ problems
 // initOT2D (prob.F90:74-119) over is..ie+1 (x) js..je+1 (x) ks..ke+1
 __global__ void k_ic_ot(GamBox b, const double* __restrict__ xyzcc, const double* __restrict__ face, double* Gas,
@@ -851,6 +876,14 @@ void gam_geom_metric(const GamBox& b, const double* xyz, double* face, double* x
     }
 }
 
+void gam_geom_tables_d(const GamBox& b, const double* vol, double* vif, double* rvif, cudaStream_t s) {
+    dim3 blk(32, 4, 1);
+    k_geo_tables<double><<<g3(b.Ni, b.Nj, b.Nk, blk), blk, 0, s>>>(b, vol, vif, rvif);
+}
+void gam_geom_tables_f(const GamBox& b, const double* vol, float* vif, float* rvif, cudaStream_t s) {
+    dim3 blk(32, 4, 1);
+    k_geo_tables<float><<<g3(b.Ni, b.Nj, b.Nk, blk), blk, 0, s>>>(b, vol, vif, rvif);
+}
 void gam_geom_ic_ot(const GamBox& b, const double* xyzcc, const double* face, double* Gas, double* mf, double gamma,
                     cudaStream_t s) {
     dim3 blk(32, 4, 1);

@@ -59,8 +59,9 @@ GAMQ_HD bool quot_in_range(double x) {
 struct QuotExact {
     double d, yh, yl;
     bool dok;
-    GAMQ_HD explicit QuotExact(double dd) : d(dd) {
-        yh = 1.0 / dd;
+    GAMQ_HD explicit QuotExact(double dd) : QuotExact(dd, 1.0 / dd) {}
+    // with the divisor's rounded reciprocal r = RN(1/dd) already at hand
+    GAMQ_HD QuotExact(double dd, double r) : d(dd), yh(r) {
         yl = fma(-dd, yh, 1.0) * yh;
         dok = quot_in_range(dd);
     }
@@ -72,6 +73,41 @@ struct QuotExact {
             return a == 0.0 ? a * yh : q;
         }
         return a / d;
+    }
+    // N quotients at once, the same bits as N calls: one branch on whether all
+    // numerators are in range instead of one per numerator, so that the fast
+    // quotients (and the loads around them) schedule together. The sign is
+    // set from the operands, which covers a zero numerator.
+    template <int N> GAMQ_HD void many(const double* a, double* q) const {
+        bool ok = dok;
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+        for (int n = 0; n < N; n++) ok = ok & (quot_in_range(a[n]) | (a[n] == 0.0));
+        if (ok) {
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+            for (int n = 0; n < N; n++) {
+                const double q0 = fma(a[n], yh, a[n] * yl);
+                const double r = fma(-d, q0, a[n]);
+                q[n] = with_sign(fma(r, yh, q0), a[n], d);
+            }
+        } else {
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+            for (int n = 0; n < N; n++) q[n] = a[n] / d;
+        }
+    }
+    // |q| with the sign of a/d
+    static GAMQ_HD double with_sign(double q, double a, double d) {
+#if defined(__CUDA_ARCH__)
+        const int s = (__double2hiint(a) ^ __double2hiint(d)) & (int)0x80000000;
+        return __hiloint2double((__double2hiint(q) & 0x7fffffff) | s, __double2loint(q));
+#else
+        return copysign(q, __builtin_signbit(a) != __builtin_signbit(d) ? -1.0 : 1.0);
+#endif
     }
 };
 

@@ -108,22 +108,32 @@ template <> struct Mth<float> {
 // three fmas and a multiply per numerator), FP32 by plain division.
 // Quot1 is the same for a divisor with a single numerator, where QuotExact
 // would cost more than the division it replaces.
+// many<N> takes N numerators at once (one range check for all of them). The
+// two-argument form takes the divisor's rounded reciprocal from a table.
 template <class R> struct Quot {
 #ifdef GAM_FAST_RECIP
     R r;
     __device__ __forceinline__ explicit Quot(R d) : r((R)1 / d) {}
+    __device__ __forceinline__ Quot(R, R rd) : r(rd) {}
     __device__ __forceinline__ R operator()(R a) const { return a * r; }
 #else
     R d;
     __device__ __forceinline__ explicit Quot(R dd) : d(dd) {}
+    __device__ __forceinline__ Quot(R dd, R) : d(dd) {}
     __device__ __forceinline__ R operator()(R a) const { return a / d; }
 #endif
+    template <int N> __device__ __forceinline__ void many(const R* a, R* o) const {
+#pragma unroll
+        for (int n = 0; n < N; n++) o[n] = (*this)(a[n]);
+    }
 };
 #ifndef GAM_FAST_RECIP
 template <> struct Quot<double> {
     gam::QuotExact q;
     __device__ __forceinline__ explicit Quot(double d) : q(d) {}
+    __device__ __forceinline__ Quot(double d, double rd) : q(d, rd) {}
     __device__ __forceinline__ double operator()(double a) const { return q(a); }
+    template <int N> __device__ __forceinline__ void many(const double* a, double* o) const { q.many<N>(a, o); }
 };
 #endif
 // a/d for a finite nonzero divisor d, equal to the IEEE quotient. A zero
@@ -185,6 +195,36 @@ __device__ __forceinline__ R pdm1(R pdmb, R q0, R q1, R q2, R qI) {
     R s01 = fabs(s0 + s1);
     R dqL = qN - q1;
     return qN - s1 * rmax((R)0, fabs(dqL) - s01 * fabs(dq0));
+}
+// PDM on both sides of a face between the cells v1 and v2, for the
+// interpolants QL and QR (the same one in 8CENT): the values of pdm1, which are
+// pdmLR's too (its right state is its left one with the stencil mirrored; where
+// mirroring a zero difference changes its sign, the term it selects is zero).
+// FP64: the signs of the differences are taken from their bits and twice the
+// limiter difference enters by one fma (exact, since 2|x| is): 15 FP64
+// instructions instead of 22.
+__device__ __forceinline__ double pdm_cut(double pd, double v, double qN, double vd) {
+    // qN - s max(0, |qN - v| - |s + s'| |pd|), s = sign of vd, s' = sign of pd
+    const int sp = __double2hiint(pd), sv = __double2hiint(vd);
+    const double k = __hiloint2double((sp ^ sv) < 0 ? 0 : (int)0xC0000000, 0);  // -2 or 0
+    const double t = fma(k, fabs(pd), fabs(qN - v));
+    const double m = (0.0 < t) ? t : 0.0;
+    return qN - __hiloint2double(__double2hiint(m) ^ (sv & (int)0x80000000), __double2loint(m));
+}
+__device__ __forceinline__ void pdm_both(double pdmb, double v0, double v1, double v2, double v3, double QL, double QR,
+                                         double& L, double& U) {
+    const double d1 = v2 - v1, pd0 = pdmb * (v1 - v0), pd2 = pdmb * (v2 - v3);
+    const bool dn = __double2hiint(d1) < 0;
+    const double hi = dn ? v1 : v2, lo = dn ? v2 : v1;
+    const double qL = rmax(lo, rmin(QL, hi)), qR = rmax(lo, rmin(QR, hi));
+    const double vd = pdmb * d1;
+    L = pdm_cut(pd0, v1, qL, vd);
+    U = pdm_cut(pd2, v2, qR, -vd);
+}
+__device__ __forceinline__ void pdm_both(float pdmb, float v0, float v1, float v2, float v3, float QL, float QR,
+                                         float& L, float& U) {
+    L = pdm1(pdmb, v0, v1, v2, QL);
+    U = pdm1(pdmb, v3, v2, v1, QR);
 }
 template <class R> __device__ __forceinline__ R central8(const R* q) {
     R s = (R)0;
@@ -722,6 +762,24 @@ __global__ void __launch_bounds__(128, MINB) k_vxb(GamBox b, DevParams<R> P, Geo
     }
 }
 
+// Quotient by the volume interpolated to the face c of direction D: from the
+// tables made with the geometry, else from the volumes (differentiation form)
+template <class R> __device__ __forceinline__ Quot<R> face_quot(const GamBox& b, const Geo<R>& g, long c, int D) {
+#ifdef GAM_GEO_TABLES
+#ifdef GAM_FAST_RECIP
+    return Quot<R>((R)0, g.rvif[D * b.fs + c]);
+#else
+    return Quot<R>(g.vif[D * b.fs + c], g.rvif[D * b.fs + c]);
+#endif
+#else
+    const long s = dstride(b, D);
+    R vol[8];
+#pragma unroll
+    for (int n = 0; n < 8; n++) vol[n] = g.vol[c + (n - 4) * s];
+    return Quot<R>(central8(vol));
+#endif
+}
+
 // One-sided Gaussian-moment fluxes for one side q (sgn = -1 LEFT, +1 RIGHT).
 // MagKinFlux (stress.F90:513-599).
 template <class R, bool BORIS = false>
@@ -804,63 +862,156 @@ __device__ __forceinline__ void gas_kin_flux(const DevParams<R>& P, R sgn, const
     dW[4] = dW[4] + sgn * E;
 }
 
+// ----------------------------------------------------------------- TMA
+// Box copies of a (i, j, k, component) field into shared memory and the
+// mbarrier that counts their bytes.
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void tma_bar_init(uint64_t* bar) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+__device__ __forceinline__ void tma_expect(uint64_t* bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void tma_load(void* dst, const CUtensorMap* map, int i, int j, int k, uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
+        "[%6];" ::"r"(smem_u32(dst)), "l"(map), "r"(i), "r"(j), "r"(k), "r"(0), "r"(smem_u32(bar))
+        : "memory");
+}
+// Wait for the first phase; false when it does not complete within the limit
+// (each try waits in hardware for a while)
+__device__ __forceinline__ bool tma_wait(uint64_t* bar) {
+    for (int n = 0; n < (1 << 20); n++) {
+        uint32_t done;
+        asm volatile(
+            "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0; selp.b32 %0, 1, 0, p; }"
+            : "=r"(done)
+            : "r"(smem_u32(bar))
+            : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+
 // Face fluxes of direction D (Fluxes, stress.F90:204-429), one face per
 // thread. The stencil operands are the per-cell products volume*primitive and
-// volume*B of the half state (QdV of Cen8LRs) and the limiter values, read
-// along D through L1; MINB bounds the registers for occupancy. SAVE (the
-// differentiation form's forward) also stores the face states in w.fsv.
-template <class R, int D, int MINB, bool BORIS = false, bool SAVE = false>
-__global__ void __launch_bounds__(128, MINB) k_stress(GamBox b, DevParams<R> P, Geo<R> g, const R* __restrict__ Blim,
-                                                      Work<R> w, Range r, const GamScalars* sc,
-                                                      const R* __restrict__ gasN, const R* __restrict__ gasO) {
+// volume*B of the half state (QdV of Cen8LRs) and the limiter values of 16
+// fields. One thread has the block's tile of all of them copied to shared
+// memory by TMA (four box copies, one mbarrier); the metric's loads are issued
+// meanwhile. What bounds the kernel is the FP64 pipe's issue and the latency of
+// the formulas' chains: with plain loads through L1 (about half of them
+// missing) every variable exposed a memory latency, a third of all stalls.
+// 192^3, I/J/K sweeps, plain loads -> tiles: strict 934/920/957 -> 816/739/808
+// us, FMA form 746/751/811 -> 598/560/563, FP32 386/415/424 -> 295/263/264.
+// MINB bounds the registers for occupancy.
+template <class R, int D, int MINB, bool BORIS = false>
+__global__ void __launch_bounds__(FluxTile<R, D>::NT, MINB)
+    k_stress(GamBox b, DevParams<R> P, Geo<R> g, Work<R> w, Range r, GamScalars* sc, const R* __restrict__ gasN,
+             const R* __restrict__ gasO, const __grid_constant__ GamFluxMaps maps) {
+    using T_ = FluxTile<R, D>;
+    extern __shared__ __align__(128) unsigned char flux_smem[];
+    __shared__ __align__(8) uint64_t bar;
     if (sc->halted) return;
-    int ii, jj, kk;
-    if (!thread_ijk(r, ii, jj, kk)) return;
+    R* sQ = (R*)flux_smem;                // [8][QN][QX]: QW (5), QB (3)
+    R* sL = (R*)(flux_smem + T_::LOFF);   // [8][LN][QX]: Wn (5), limiter B (3)
+    const int tx = threadIdx.x % T_::TX, tn = threadIdx.x / T_::TX;
+    const int i0 = r.i0 + blockIdx.x * T_::TX;
+    const int j0 = r.j0 + blockIdx.y * (D == 2 ? 1 : T_::TN);
+    const int k0 = r.k0 + blockIdx.z * (D == 2 ? T_::TN : 1);
+    if (threadIdx.x == 0) {
+        tma_bar_init(&bar);
+        tma_expect(&bar, P.doMHD ? T_::BYTES : T_::BYTES_GAS);
+        const int qi = D == 0 ? i0 - 4 : i0, qj = D == 1 ? j0 - 4 : j0, qk = D == 2 ? k0 - 4 : k0;
+        const int lj = D == 1 ? j0 - 2 : j0, lk = D == 2 ? k0 - 2 : k0;
+        tma_load(sQ, &maps.QW, qi, qj, qk, &bar);
+        tma_load(sL, &maps.Wn, qi, lj, lk, &bar);
+        if (P.doMHD) {
+            tma_load(sQ + 5 * T_::QN * T_::QX, &maps.QB, qi, qj, qk, &bar);
+            tma_load(sL + 5 * T_::LN * T_::QX, &maps.Bl, qi, lj, lk, &bar);
+        }
+    }
+    const int ii = i0 + tx, jj = D == 2 ? j0 : j0 + tn, kk = D == 2 ? k0 + tn : k0;
     const long fs = b.fs;
-    const long c = lidx(b, ii, jj, kk);
     const long s = D == 0 ? 1L : (D == 1 ? (long)b.sx : b.sk);
-    GAM_BOX_CHECK(c - 4 * s, c + 3 * s, 8 + D);
+    // threads past the range take the range's last face (and store nothing)
+    const bool in = ii <= r.i1 && jj <= r.j1 && kk <= r.k1;
+    const long c = lidx(b, min(ii, r.i1), min(jj, r.j1), min(kk, r.k1));
     R T[9];
 #pragma unroll
     for (int n = 0; n < 9; n++) T[n] = g.Tf[(n + 9 * D) * fs + c];
     const R fa = g.face[D * fs + c];
-    R vol[8];
-#pragma unroll
-    for (int n = 0; n < 8; n++) vol[n] = g.vol[c + (n - 4) * s];
-    const Quot<R> Vi(central8(vol));
+    const Quot<R> Vi = face_quot<R>(b, g, c, D);
     R MagL[3] = {(R)0, (R)0, (R)0}, MagR[3] = {(R)0, (R)0, (R)0};
     R Bn = (R)0;
     double B0[3] = {0.0, 0.0, 0.0}, B0n = 0.0;
     if (P.doMHD) {
         Bn = w.Bnf[D * fs + c];
-#pragma unroll
-        for (int x = 0; x < 3; x++) {
-            R q[8], nq[4];
-            const R* qp = w.QB + x * fs + c - 4 * s;
-            const R* lp = Blim + x * fs + c - 2 * s;
-#pragma unroll
-            for (int n = 0; n < 8; n++) q[n] = qp[n * s];
-#pragma unroll
-            for (int m = 0; m < 4; m++) nq[m] = lp[m * s];
-            lrs_from_qdv(P, q, nq, Vi, MagL[x], MagR[x]);
-        }
         if (P.doBackground) {
 #pragma unroll
             for (int x = 0; x < 3; x++) B0[x] = g.fcB0[(x + 3 * D) * fs + c];
             B0n = qdiv(g.bFlux0[D * fs + c], (double)fa);
         }
     }
+    __syncthreads();  // the barrier's initialisation
+    if (!tma_wait(&bar)) {  // never in a sound step: stop it
+        sc->status = 5;
+        sc->halted = 1;
+        return;
+    }
+    if (!in) return;
+    GAM_BOX_CHECK(c - 4 * s, c + 3 * s, 8 + D);
     R WL[5], WR[5];
+    // reconstruction, GRP variables at a time: their interpolants, one range
+    // check for the quotients, the limiter
+    constexpr int GRP = 4;
+    const R* pQ = sQ + (D == 0 ? tn * T_::QX + tx : tn * T_::TX + tx);
+    const R* pL = sL + (D == 0 ? tn * T_::QX + tx + 2 : tn * T_::TX + tx);
+    constexpr int st = D == 0 ? 1 : T_::TX;
+    const int nvar = P.doMHD ? 8 : 5;
 #pragma unroll
-    for (int v = 0; v < 5; v++) {
-        R q[8], nq[4];
-        const R* qp = w.QW + v * fs + c - 4 * s;
-        const R* lp = w.Wn + v * fs + c - 2 * s;
+    for (int n0 = 0; n0 < 8; n0 += GRP) {
+        if (n0 >= nvar) break;
+        R a[2 * GRP], Qi[2 * GRP];
 #pragma unroll
-        for (int n = 0; n < 8; n++) q[n] = qp[n * s];
+        for (int n = 0; n < GRP; n++) {
+            const R* p = pQ + (n0 + n) * T_::QN * T_::QX;
+            if (!P.up7) {
+                R q[8];
 #pragma unroll
-        for (int m = 0; m < 4; m++) nq[m] = lp[m * s];
-        lrs_from_qdv(P, q, nq, Vi, WL[v], WR[v]);
+                for (int m = 0; m < 8; m++) q[m] = p[m * st];
+                a[n] = central8(q);
+            } else {
+                a[n] = p[0] * Rc<R>(up7c(0));
+                a[GRP + n] = p[7 * st] * Rc<R>(up7c(0));
+#pragma unroll
+                for (int m = 1; m < 7; m++) {
+                    a[n] = a[n] + p[m * st] * Rc<R>(up7c(m));
+                    a[GRP + n] = a[GRP + n] + p[(7 - m) * st] * Rc<R>(up7c(m));
+                }
+            }
+        }
+        Vi.template many<GRP>(a, Qi);
+        if (P.up7) {
+            Vi.template many<GRP>(a + GRP, Qi + GRP);
+        } else {
+#pragma unroll
+            for (int n = 0; n < GRP; n++) Qi[GRP + n] = Qi[n];
+        }
+#pragma unroll
+        for (int n = 0; n < GRP; n++) {
+            const int v = n0 + n;
+            const R* p = pL + v * T_::LN * T_::QX;
+            R l, u;
+            pdm_both(P.pdmb, p[0], p[st], p[2 * st], p[3 * st], Qi[n], Qi[GRP + n], l, u);
+            if (v < 5) {
+                WL[v] = l;
+                WR[v] = u;
+            } else {
+                MagL[v - 5] = l;
+                MagR[v - 5] = u;
+            }
+        }
     }
     R VaD = (R)0, bbD = (R)0;
     if (P.doMHD) {
@@ -919,21 +1070,6 @@ __global__ void __launch_bounds__(128, MINB) k_stress(GamBox b, DevParams<R> P, 
     }
 #pragma unroll
     for (int v = 0; v < 5; v++) w.gF[(v + 5 * D) * fs + c] = fa * gv[v];
-    if constexpr (SAVE) {
-        R* o = w.fsv + (long)(GAM_FSV_NC * D) * fs + c;
-#pragma unroll
-        for (int v = 0; v < 5; v++) {
-            o[v * fs] = WL[v];
-            o[(5 + v) * fs] = WR[v];
-            o[(17 + v) * fs] = dW[v];
-        }
-#pragma unroll
-        for (int x = 0; x < 3; x++) {
-            o[(10 + x) * fs] = MagL[x];
-            o[(13 + x) * fs] = MagR[x];
-        }
-        o[16 * fs] = VaD;
-    }
 }
 
 // E2Flux into the new buffer; faces outside its range are copied. With
@@ -2503,7 +2639,6 @@ template <class R, class F> void for_each_kernel(const Ctx<R>& C, int cur, cudaS
     const int G = GAM_NG;
     const StateBuf<R> S = C.st[cur], O = C.st[1 - cur];
     const dim3 blk(32, 4, 1);
-    const dim3 sblk(16, 8, 1);  // flux kernels: 8 rows per block for the J-direction stencil reuse
     const Range all{0, b.Ni, 0, b.Nj, 0, b.Nk};
     const Range cells{0, b.Ni - 1, 0, b.Nj - 1, 0, b.Nk - 1};
     const int kke = C.P.do25D ? G : G + b.Nkp - 1;  // last active k of the stress sweep
@@ -2546,29 +2681,23 @@ template <class R, class F> void for_each_kernel(const Ctx<R>& C, int cur, cudaS
     const Range fr[3] = {{G, G + b.Nip, G, G + b.Njp - 1, G, kke},
                          {G, G + b.Nip - 1, G, G + b.Njp, G, kke},
                          {G, G + b.Nip - 1, G, G + b.Njp - 1, G, G + b.Nkp}};
-    const R* Blim = C.P.doLFMLim ? S.B : C.w.Bl;
     auto stress = [&](auto Dc) {
         constexpr int D = decltype(Dc)::value;
         const Range& r = fr[D];
-        // K sweep: blocks that extend along k share its 8-point stencil planes
-        // in L1 (16x1x8 measured 5 % faster than 16x8x1 on the K sweep)
-        const dim3 sbk = D != 2           ? sblk
-                         : (C.kvar & 256)  ? sblk
-                         : (C.kvar & 2048) ? dim3(32, 1, 4)
-                         : (C.kvar & 4096) ? dim3(8, 1, 16)
-                                           : dim3(16, 1, 8);
-        if (C.P.doBoris) {
-            k_stress<R, D, sizeof(R) == 4 ? 8 : 6, true><<<grid_for(r, sbk), sbk, 0, s>>>(b, C.P, C.g, Blim, C.w, r, C.sc,
-                                                                                        S.Gas, O.Gas);
-            return;
-        }
-        switch (C.kvar & 3) {
-            case 1: k_stress<R, D, 1><<<grid_for(r, sbk), sbk, 0, s>>>(b, C.P, C.g, Blim, C.w, r, C.sc, S.Gas, O.Gas); break;
-            case 2: k_stress<R, D, 7><<<grid_for(r, sbk), sbk, 0, s>>>(b, C.P, C.g, Blim, C.w, r, C.sc, S.Gas, O.Gas); break;
-            case 3: k_stress<R, D, 8><<<grid_for(r, sbk), sbk, 0, s>>>(b, C.P, C.g, Blim, C.w, r, C.sc, S.Gas, O.Gas); break;
-            // FP64: 8 blocks/SM for the I and J sweeps, 7 for K (measured); FP32: 8
-            default: k_stress<R, D, (sizeof(R) == 4 || D < 2) ? 8 : 7><<<grid_for(r, sbk), sbk, 0, s>>>(b, C.P, C.g, Blim, C.w, r, C.sc, S.Gas, O.Gas); break;
-        }
+        using T_ = FluxTile<R, D>;
+        const dim3 sg((unsigned)((r.i1 - r.i0 + T_::TX) / T_::TX),
+                      (unsigned)(D == 2 ? r.j1 - r.j0 + 1 : (r.j1 - r.j0 + T_::TN) / T_::TN),
+                      (unsigned)(D == 2 ? (r.k1 - r.k0 + T_::TN) / T_::TN : r.k1 - r.k0 + 1));
+        const GamFluxMaps& M = C.fmaps->m[cur][D];
+        // blocks per SM (registers against warps; 192^3, I/J/K sweeps): the strict
+        // form 5 (816/739/808 us; 4: 852/770/775, 7: 895/854/859), the FMA form 5
+        // (598/560/563; 4: 627/576/586, 6: 648/611/636), FP32 5 of 256 threads on
+        // the J and K sweeps (263/264; 4: 269/275) and 7 of 128 on the I sweep
+        constexpr int MB = sizeof(R) == 8 ? 5 : (D == 0 ? 7 : 5);
+        if (C.P.doBoris)
+            k_stress<R, D, sizeof(R) == 8 ? 5 : 3, true><<<sg, T_::NT, T_::SMEM, s>>>(b, C.P, C.g, C.w, r, C.sc, S.Gas, O.Gas, M);
+        else
+            k_stress<R, D, MB><<<sg, T_::NT, T_::SMEM, s>>>(b, C.P, C.g, C.w, r, C.sc, S.Gas, O.Gas, M);
     };
     f(8, [&] { stress(std::integral_constant<int, 0>()); });
     f(9, [&] { stress(std::integral_constant<int, 1>()); });

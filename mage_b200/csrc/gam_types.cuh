@@ -1,6 +1,7 @@
 // Device-side views of the GAMERA Model/Grid/State/Solver data, shared by
 // every build variant of the step kernels and by the C ABI.
 #pragma once
+#include <cuda.h>
 #include "gam_layout.cuh"
 
 // Solar-wind boundary data (apps/wind.F90:206-391) for a constant wind: the
@@ -90,6 +91,12 @@ template <class R> struct Geo {  // Grid_T arrays on the device (gamtypes.F90:16
     // once). Replaces xfc and xyzcc in bFlux2Fld, whose absolute coordinates
     // lose the cell-size differences when rounded to FP32.
     const R* dxf;    // cell, 18
+    // geometry-only operands of the reconstructions, made with the geometry
+    // (gam_geom_tables; null in the differentiation form): the 8CENT interpolant
+    // of the volumes at the faces of each direction and its reciprocal. The
+    // forms that multiply by the reciprocal keep only that one.
+    const R* vif;    // face, 3
+    const R* rvif;   // face, 3
     const double* fcB0;    // face, 9  (background; FP64 in both forms)
     const double* bFlux0;  // face, 3
     const double* edgB0;   // edge, 6: c + 2*d
@@ -133,6 +140,32 @@ struct Range {  // inclusive box-index range
 };
 
 
+// The tile of one block of the flux kernel of direction D, and its stencil
+// boxes in shared memory: TX faces in i by TN along j (D = 0, 1) or k (D = 2);
+// reconstruction operands of cells -4..3 and limiter values of cells -2..1
+// along D. On the I sweep both boxes start 4 cells below the tile's first face
+// (a TMA box starts on a 16-byte boundary: an even cell in FP64, a multiple of
+// 4 in FP32; the flux ranges start at cell 4 and tiles are 16 or 32 wide).
+template <class R, int D> struct FluxTile {
+    static constexpr int TX = D == 0 ? 32 : (sizeof(R) == 8 ? 16 : 32);
+    static constexpr int TN = D == 0 ? 4 : 8;
+    static constexpr int NT = TX * TN;
+    static constexpr int QX = D == 0 ? 40 : TX;
+    static constexpr int QN = D == 0 ? TN : TN + 7, LN = D == 0 ? TN : TN + 3;
+    static constexpr unsigned BYTES = 8u * (QN + LN) * QX * sizeof(R), BYTES_GAS = 5u * (QN + LN) * QX * sizeof(R);
+    static constexpr unsigned LOFF = 8u * QN * QX * sizeof(R), SMEM = BYTES;
+    static_assert(5 * QN * QX * sizeof(R) % 128 == 0 && LOFF % 128 == 0 && 5 * LN * QX * sizeof(R) % 128 == 0,
+                  "TMA destinations are 128-byte aligned");
+};
+// The tensor maps of those boxes for one direction: the reconstruction
+// operands, the limiter primitives and the limiter field
+struct GamFluxMaps {
+    CUtensorMap QW, QB, Wn, Bl;
+};
+struct GamFluxMapSet {
+    GamFluxMaps m[2][3];  // [State buffer][direction]
+};
+
 // Everything one step launch needs.
 template <class R> struct Ctx {
     GamBox b;
@@ -142,6 +175,7 @@ template <class R> struct Ctx {
     R* oomf;             // doAB3: ooState face fluxes (n-2), refreshed from oState by k_update_faces
     Work<R> w;
     GamScalars* sc;
+    const GamFluxMapSet* fmaps;  // host memory, with the handle
     double gamma, gm1;
     int kvar;  // launch-configuration variant for tuning runs (GAM_KVAR); 0 = the tuned default
     // side streams and fork/join events of the step graph (independent
