@@ -1518,7 +1518,7 @@ GamBox torch_box(int Nip, int Njp, int Nkp) {
 template <class R> DevParams<R> dev_params(const gam_params* p) {
     DevParams<R> P;
     memset(&P, 0, sizeof(P));
-    P.gamma = (R)p->gamma; P.gm1 = (R)(p->gamma - 1); P.CFL = (R)p->CFL; P.pdmb = (R)p->pdmb; P.Vd0 = (R)p->Vd0;
+    P.gamma = (R)p->gamma; P.gm1 = (R)(p->gamma - 1); P.rgm1 = (R)1 / P.gm1; P.CFL = (R)p->CFL; P.pdmb = (R)p->pdmb; P.Vd0 = (R)p->Vd0;
     P.cHogH = (R)p->cHogH; P.dFloor = (R)p->dFloor; P.pFloor = (R)p->pFloor;
     P.doMHD = p->doMHD; P.doLFMLim = p->doLFMLim; P.do25D = p->do25D; P.doBackground = p->doBackground;
     P.up7 = p->rmeth == GAM_RECON_7UP;
@@ -1788,7 +1788,7 @@ int predict_call(const gam_params* p, const void* const* st, const void* const* 
         w.QW = (R*)out[0]; w.Wn = (R*)out[1]; w.Dh = (R*)out[2]; w.VdV = (R*)out[3]; w.QB = (R*)out[4];
         w.abh = (R*)out[5]; w.Bnf = (R*)out[6]; w.bn = (R*)out[7];
         const dim3 blk(32, 8, 1);
-        k_predict<R, 1><<<grid3(all, blk), blk, 0, s>>>(b, P, g, cur, old, w, sc, nullptr);
+        k_predict<R, sizeof(R) == 8 ? 3 : 4><<<grid3(all, blk), blk, 0, s>>>(b, P, g, cur, old, w, sc, nullptr);
     } else {
         Work<R> dw;
         memset(&dw, 0, sizeof(dw));
@@ -1823,7 +1823,7 @@ int update_call(const gam_params* p, const void* const* in, const void* const* g
         StateBuf<R> nxt{(R*)out[0], (R*)out[1], (R*)out[2]};
         k_update_faces<R><<<grid3(all, blk), blk, 0, s>>>(b, P, cur, nxt, w, sc, nullptr);
         const double gamma = p->gamma, gm1 = p->gamma - 1;
-        k_update_cells<R, 1><<<grid3(cells, blk), blk, 0, s>>>(b, P, g, cur, nxt, w, sc, gamma, gm1);
+        k_update_cells<R, sizeof(R) == 8 ? 6 : 8><<<grid3(cells, blk), blk, 0, s>>>(b, P, g, cur, nxt, w, sc, gamma, gm1);
     } else {
         k_update_adj_cells<R><<<grid3(cells, blk), blk, 0, s>>>(b, P, g, cur, w, dt, (const R*)din[0], (R*)dst[0],
                                                                  (R*)sU, (R*)sM);

@@ -173,6 +173,7 @@ extern "C" int gam_default_params(gam_params* p, int32_t Nip, int32_t Njp, int32
 template <class R> static void fill_dev_params(DevParams<R>& P, const gam_params& p) {
     P.gamma = (R)p.gamma;
     P.gm1 = (R)(p.gamma - 1);
+    P.rgm1 = (R)1 / P.gm1;
     P.CFL = (R)p.CFL;
     P.pdmb = (R)p.pdmb;
     P.Vd0 = (R)p.Vd0;
@@ -932,6 +933,8 @@ template <class R> static int profile_t(gam_handle* h, Ctx<R>& C, int32_t reps, 
     t.odt = t.time - t.otime;
     t.oodt = t.otime - t.ootime;
     t.pdt = 0.5 * t.dt;
+    t.rodt = 1.0 / t.odt;
+    t.rdt = 1.0 / t.dt;
     if (e == cudaSuccess) e = cudaMemcpyAsync(h->sc, &t, sizeof(t), cudaMemcpyHostToDevice, h->s);
     if (e == cudaSuccess) {
         if (h->f32)

@@ -44,6 +44,7 @@ struct GamRingGeo {
 struct GamScalars {
     double t, dt, dt0, time, otime, tFin, limDT0, CFL;
     double odt, pdt;                   // this step's AB2 spacing and half step
+    double rodt, rdt;                  // 1/odt and 1/dt, rounded
     unsigned long long dtmin_bits;     // running min of the cell dt (bits of a positive double)
     int ts;
     int status;                        // 0 ok, 4 dt bad, 5 dt disaster

@@ -100,6 +100,15 @@ struct QuotExact {
             for (int n = 0; n < N; n++) q[n] = a[n] / d;
         }
     }
+    // The fast quotient alone; ok turns false where it is not the IEEE one (an
+    // operand out of range). A caller that takes all its quotients this way has
+    // no branch between them, and does its work again with a/d if one failed.
+    GAMQ_HD double quick(double a, bool& ok) const {
+        ok = ok & dok & (quot_in_range(a) | (a == 0.0));
+        const double q0 = fma(a, yh, a * yl);
+        const double r = fma(-d, q0, a);
+        return with_sign(fma(r, yh, q0), a, d);
+    }
     // |q| with the sign of a/d
     static GAMQ_HD double with_sign(double q, double a, double d) {
 #if defined(__CUDA_ARCH__)

@@ -136,6 +136,31 @@ template <> struct Quot<double> {
     template <int N> __device__ __forceinline__ void many(const double* a, double* o) const { q.many<N>(a, o); }
 };
 #endif
+// The quotient of code that runs twice at most (strict FP64): first with the
+// branch-free quotients, which note in ok an operand that they do not cover,
+// then, if there was one, with EXACT divisions. The other forms have one kind.
+template <class R, bool EXACT> struct QuotTry : Quot<R> {
+    using Quot<R>::Quot;
+    __device__ __forceinline__ R operator()(R a, bool&) const { return Quot<R>::operator()(a); }
+};
+#ifndef GAM_FAST_RECIP
+template <> struct QuotTry<double, false> : Quot<double> {
+    using Quot<double>::Quot;
+    __device__ __forceinline__ double operator()(double a, bool& ok) const { return this->q.quick(a, ok); }
+};
+template <> struct QuotTry<double, true> {
+    double d;
+    __device__ __forceinline__ explicit QuotTry(double dd) : d(dd) {}
+    __device__ __forceinline__ QuotTry(double dd, double) : d(dd) {}
+    __device__ __forceinline__ double operator()(double a, bool&) const { return a / d; }
+};
+#endif
+// whether a form has the two kinds
+template <class R> struct TwoTries { static constexpr bool v = std::is_same<R, double>::value
+#ifdef GAM_FAST_RECIP
+    && false
+#endif
+    ; };
 // a/d for a finite nonzero divisor d, equal to the IEEE quotient. A zero
 // numerator returns a*d (the signed zero of a/d) without entering the
 // division, whose IEEE routine leaves its fast path for a zero numerator;
@@ -153,6 +178,9 @@ template <class R> struct Quot1 {
     __device__ __forceinline__ R operator()(R a) const { return qdiv(a, d); }
 #endif
 };
+
+// quotients by gamma - 1, with its reciprocal from the parameters
+template <class R> __device__ __forceinline__ Quot<R> gm1_quot(const DevParams<R>& P) { return Quot<R>(P.gm1, P.rgm1); }
 
 // std::max / std::min semantics: max(a,b) = (a < b) ? b : a, min(a,b) = (b < a) ? b : a
 template <class R> __device__ __forceinline__ R rmax(R a, R b) { return (a < b) ? b : a; }
@@ -265,12 +293,15 @@ __device__ __forceinline__ void block_c2p(const DevParams<R>& P, const R* U, R* 
     R D = rmax(U[0], P.dFloor);
     const Quot<R> qD(D);
     R Mx = U[1], My = U[2], Mz = U[3], E = U[4];
-    R KinE = qD((R)0.5 * (Mx * Mx + My * My + Mz * Mz));
+    const R num[4] = {Mx, My, Mz, (R)0.5 * (Mx * Mx + My * My + Mz * Mz)};
+    R quo[4];
+    qD.template many<4>(num, quo);
+    R KinE = quo[3];
     R Pr = rmax(P.gm1 * (E - KinE), P.pFloor);
     W[0] = D;
-    W[1] = qD(Mx);
-    W[2] = qD(My);
-    W[3] = qD(Mz);
+    W[1] = quo[0];
+    W[2] = quo[1];
+    W[3] = quo[2];
     W[4] = Pr;
 }
 // CellC2P (gamutils.F90:301-321)
@@ -278,7 +309,9 @@ template <class R>
 __device__ __forceinline__ void cell_c2p(const DevParams<R>& P, const R* U, R* W) {
     R rho = U[0];
     const Quot<R> qr(rho);
-    R Vx = qr(U[1]), Vy = qr(U[2]), Vz = qr(U[3]);
+    R V[3];
+    qr.template many<3>(U + 1, V);
+    R Vx = V[0], Vy = V[1], Vz = V[2];
     R E = U[4];
     R KinE = (R)0.5 * rho * (Vx * Vx + Vy * Vy + Vz * Vz);
     W[0] = rmax(rho, P.dFloor);
@@ -292,7 +325,7 @@ template <class R>
 __device__ __forceinline__ void cell_p2c(const DevParams<R>& P, const R* W, R* U) {
     R rho = rmax(W[0], P.dFloor);
     R Vx = W[1], Vy = W[2], Vz = W[3];
-    R IntE = rmax(W[4], P.pFloor) / P.gm1;
+    R IntE = gm1_quot(P)(rmax(W[4], P.pFloor));
     R KinE = (R)0.5 * rho * (Vx * Vx + Vy * Vy + Vz * Vz);
     U[0] = rho;
     U[1] = rho * Vx;
@@ -325,21 +358,27 @@ __device__ __forceinline__ double norm2s3(const double* a) {
 #define GAM_SQRT2_R4 ((double)1.41421354f)
 
 // PredictCell (mhdgroup.F90:528-562, AB2, single fluid): the half-step
-// conserved state from State n (Q) and n-1 (oQ)
+// conserved state from the primitives of State n (W) and n-1 (oW)
 template <class R>
-__device__ __forceinline__ void predict_cell(const DevParams<R>& P, const R* Q, const R* oQ, R pdt, const Quot<R>& odt,
+__device__ __forceinline__ void predict_prim(const DevParams<R>& P, const R* W, const R* oW, R pdt, const Quot<R>& odt,
                                              R* pQ) {
-    R W[5], oW[5], pW[5];
-    cell_c2p(P, oQ, oW);
-    cell_c2p(P, Q, W);
+    R dif[5], dQ[5], pW[5];
 #pragma unroll
-    for (int v = 0; v < 5; v++) {
-        R dQ = odt(W[v] - oW[v]);
-        pW[v] = W[v] + pdt * dQ;
-    }
+    for (int v = 0; v < 5; v++) dif[v] = W[v] - oW[v];
+    odt.template many<5>(dif, dQ);
+#pragma unroll
+    for (int v = 0; v < 5; v++) pW[v] = W[v] + pdt * dQ[v];
     pW[0] = rmax(pW[0], P.dFloor);
     pW[4] = rmax(pW[4], P.pFloor);
     cell_p2c(P, pW, pQ);
+}
+template <class R>
+__device__ __forceinline__ void predict_cell(const DevParams<R>& P, const R* Q, const R* oQ, R pdt, const Quot<R>& odt,
+                                             R* pQ) {
+    R W[5], oW[5];
+    cell_c2p(P, oQ, oW);
+    cell_c2p(P, Q, W);
+    predict_prim(P, W, oW, pdt, odt, pQ);
 }
 
 // ExtrapAB3 (mhdgroup.F90:721-731)
@@ -352,28 +391,35 @@ template <class R> __device__ __forceinline__ R extrap_ab3(R dt, R Q, R oQ, R oo
 // PredictCell with doAB3: the third level of the gas is oState's
 // (ooQ = oState%Gas, mhdgroup.F90:500-502), as in the reference
 template <class R>
-__device__ __forceinline__ void predict_cell_ab3(const DevParams<R>& P, const R* Q, const R* oQ, R pdt, R odt, R oodt,
+__device__ __forceinline__ void predict_prim_ab3(const DevParams<R>& P, const R* W, const R* oW, R pdt, R odt, R oodt,
                                                  R* pQ) {
-    R W[5], oW[5], ooW[5], pW[5];
-    cell_c2p(P, oQ, oW);
-    cell_c2p(P, Q, W);
-    cell_c2p(P, oQ, ooW);
+    R pW[5];
 #pragma unroll
-    for (int v = 0; v < 5; v++) pW[v] = extrap_ab3(pdt, W[v], oW[v], ooW[v], odt, oodt);
+    for (int v = 0; v < 5; v++) pW[v] = extrap_ab3(pdt, W[v], oW[v], oW[v], odt, oodt);
     pW[0] = rmax(pW[0], P.dFloor);
     pW[4] = rmax(pW[4], P.pFloor);
     cell_p2c(P, pW, pQ);
+}
+template <class R>
+__device__ __forceinline__ void predict_cell_ab3(const DevParams<R>& P, const R* Q, const R* oQ, R pdt, R odt, R oodt,
+                                                 R* pQ) {
+    R W[5], oW[5];
+    cell_c2p(P, oQ, oW);
+    cell_c2p(P, Q, W);
+    predict_prim_ab3(P, W, oW, pdt, odt, oodt, pQ);
 }
 
 // Boris-limited speed Ca v / sqrt(Ca^2 + v^2) (fields.F90:211-213,
 // gridutils.F90:91-93, gamutils.F90:356-358)
 template <class T> __device__ __forceinline__ T boris_speed(T Ca, T v) { return Ca * v / sqrt(Ca * Ca + v * v); }
 
-// gamCellBxyz (gridutils.F90:648-680) from the six face fluxes of cell c,
-// with the quotient by the cell volume qV
-template <class R>
-__device__ __forceinline__ void cell_bxyz(const GamBox& b, const Geo<R>& g, long c, R fI, R fIp, R fJ, R fJp, R fK,
-                                          R fKp, const Quot<R>& qV, R* B) {
+// gamCellBxyz (gridutils.F90:648-680) from the six face fluxes of cell c, with
+// the quotient by the cell volume qV. The metric is read through the read-only
+// path: the compiler may then move these loads above stores to the state and
+// work arrays.
+template <class R, class Q>
+__device__ __forceinline__ void cell_bxyz_q(const GamBox& b, const Geo<R>& g, long c, R fI, R fIp, R fJ, R fJp, R fK,
+                                            R fKp, const Q& qV, R* B) {
     const long fs = b.fs;
     if constexpr (std::is_same<R, float>::value) {
         // sum of flux x (face centroid - cell centroid): the same value as the
@@ -381,7 +427,8 @@ __device__ __forceinline__ void cell_bxyz(const GamBox& b, const Geo<R>& g, long
 #pragma unroll
         for (int x = 0; x < 3; x++) {
             const R* d = g.dxf + (long)x * fs + c;
-            R t = fIp * d[3 * fs] + fJp * d[9 * fs] + fKp * d[15 * fs] - fI * d[0] - fJ * d[6 * fs] - fK * d[12 * fs];
+            R t = fIp * __ldg(d + 3 * fs) + fJp * __ldg(d + 9 * fs) + fKp * __ldg(d + 15 * fs) - fI * __ldg(d) -
+                  fJ * __ldg(d + 6 * fs) - fK * __ldg(d + 12 * fs);
             B[x] = qV(t);
         }
         return;
@@ -389,20 +436,25 @@ __device__ __forceinline__ void cell_bxyz(const GamBox& b, const Geo<R>& g, long
     R Div = fIp - fI + fJp - fJ + fKp - fK;
 #pragma unroll
     for (int x = 0; x < 3; x++) {
-        R xfI = g.xfc[(x + 0) * fs + c];
-        R xfJ = g.xfc[(x + 3) * fs + c];
-        R xfK = g.xfc[(x + 6) * fs + c];
-        R xfIp = g.xfc[(x + 0) * fs + c + 1];
-        R xfJp = g.xfc[(x + 3) * fs + c + b.sx];
-        R xfKp = g.xfc[(x + 6) * fs + c + b.sk];
+        R xfI = __ldg(g.xfc + (x + 0) * fs + c);
+        R xfJ = __ldg(g.xfc + (x + 3) * fs + c);
+        R xfK = __ldg(g.xfc + (x + 6) * fs + c);
+        R xfIp = __ldg(g.xfc + (x + 0) * fs + c + 1);
+        R xfJp = __ldg(g.xfc + (x + 3) * fs + c + b.sx);
+        R xfKp = __ldg(g.xfc + (x + 6) * fs + c + b.sk);
         R t = qV(fIp * xfIp + fJp * xfJp + fKp * xfKp - fI * xfI - fJ * xfJ - fK * xfK);
-        B[x] = t - qV(Div * g.xyzcc[x * fs + c]);
+        B[x] = t - qV(Div * __ldg(g.xyzcc + x * fs + c));
     }
 }
 template <class R>
 __device__ __forceinline__ void cell_bxyz(const GamBox& b, const Geo<R>& g, long c, R fI, R fIp, R fJ, R fJp, R fK,
                                           R fKp, R* B) {
-    cell_bxyz(b, g, c, fI, fIp, fJ, fJp, fK, fKp, Quot<R>(g.vol[c]), B);
+    cell_bxyz_q(b, g, c, fI, fIp, fJ, fJp, fK, fKp, Quot<R>(g.vol[c]), B);
+}
+template <class R>
+__device__ __forceinline__ void cell_bxyz(const GamBox& b, const Geo<R>& g, long c, R fI, R fIp, R fJ, R fJp, R fK,
+                                          R fKp, const Quot<R>& qV, R* B) {
+    cell_bxyz_q(b, g, c, fI, fIp, fJ, fJp, fK, fKp, qV, B);
 }
 
 // ----------------------------------------------------------------- bounds checks
@@ -487,26 +539,19 @@ __global__ void k_step_begin(GamScalars* sc) {
     sc->odt = sc->time - sc->otime;
     sc->oodt = sc->otime - sc->ootime;  // Predictor (mhdgroup.F90:459-463), used with doAB3
     sc->pdt = 0.5 * sc->dt;
+    sc->rodt = 1.0 / sc->odt;
+    sc->rdt = 1.0 / sc->dt;
 }
 
-// Predictor over every face and cell of the ghosted box. Besides the half
-// state it stores the operands every later stencil uses, each computed once:
-// volume * primitive (the recon operand QdV of Cen8LRs/Up7LRs), the limiter
-// primitives, volume * momentum / density (Mom2Face), and per face
-// area * flux/max(area,TINY) and flux/max(area,TINY) (EdgeLRs), flux/area (Fluxes).
-template <class R, int MINB, bool AB3 = false>
-__global__ void __launch_bounds__(256, MINB) k_predict(GamBox b, DevParams<R> P, Geo<R> g, StateBuf<R> cur,
-                                                 StateBuf<R> old, Work<R> w, const GamScalars* sc,
-                                                 const R* __restrict__ oomf) {
-    if (sc->halted) return;
-    int ii, jj, kk;
-    Range r{0, b.Ni, 0, b.Nj, 0, b.Nk};
-    if (!thread_ijk(r, ii, jj, kk)) return;
+// The predictor's work at box position c (see k_predict): faces, then the cell.
+// Quotients by one density share its reciprocal; no branch between them in the
+// first try (192^3, strict: 862 -> 661 us; FMA form 713 -> 608).
+template <class R, bool AB3, bool EXACT>
+__device__ __forceinline__ void predict_at(const GamBox& b, const DevParams<R>& P, const Geo<R>& g,
+                                           const StateBuf<R>& cur, const StateBuf<R>& old, const Work<R>& w,
+                                           const R* __restrict__ oomf, int ii, int jj, int kk, long c, bool isCell, R pdt,
+                                           R odt, R rodt, R oodt, bool& ok) {
     const long fs = b.fs;
-    const long c = lidx(b, ii, jj, kk);
-    const R pdt = (R)sc->pdt, odt = (R)sc->odt;
-    const bool isCell = ii < b.Ni && jj < b.Nj && kk < b.Nk;
-    GAM_BOX_CHECK(c, isCell ? c + b.sk : c, 1);
     // The state and work pointers may alias as far as the compiler knows, so
     // every state load is issued before the first store.
     R fQ[3], foQ[3], fA[3], Q[5], oQ[5], uQ[3], uoQ[3];
@@ -537,58 +582,90 @@ __global__ void __launch_bounds__(256, MINB) k_predict(GamBox b, DevParams<R> P,
         }
     }
     R hm[3];
-    const Quot<R> qodt(odt);
-    [[maybe_unused]] R oodt = (R)0;
-    if constexpr (AB3) oodt = (R)sc->oodt;
+    const QuotTry<R, EXACT> qodt(odt, rodt);
     if (P.doMHD) {
+        if constexpr (AB3) {
+#pragma unroll
+            for (int d = 0; d < 3; d++) hm[d] = extrap_ab3(pdt, fQ[d], foQ[d], fooQ[d], odt, oodt);
+        } else {
+#pragma unroll
+            for (int d = 0; d < 3; d++) hm[d] = fQ[d] + pdt * qodt(fQ[d] - foQ[d], ok);  // ExtrapAB2
+        }
 #pragma unroll
         for (int d = 0; d < 3; d++) {
-            if constexpr (AB3) {
-                hm[d] = extrap_ab3(pdt, fQ[d], foQ[d], fooQ[d], odt, oodt);
-            } else {
-                R dQ = qodt(fQ[d] - foQ[d]);
-                hm[d] = fQ[d] + pdt * dQ;  // ExtrapAB2
-            }
             R A = fA[d];
             R Am = rmax(A, (R)TINY);
-            const Quot<R> qAm(Am);
-            R bh = qAm(hm[d]);
+            const QuotTry<R, EXACT> qAm(Am);
+            const R bh = qAm(hm[d], ok);
             w.abh[d * fs + c] = A * bh;
-            w.Bnf[d * fs + c] = qdiv(hm[d], A);
-            w.bn[d * fs + c] = P.doLFMLim ? qAm(fQ[d]) : bh;
+            // the area itself divides Bnf: the same quotient, but for areas below TINY
+            w.Bnf[d * fs + c] = Am == A ? bh : qdiv(hm[d], A);
+            w.bn[d * fs + c] = P.doLFMLim ? qAm(fQ[d], ok) : bh;
         }
     }
     if (!isCell) return;
-    R pQ[5];
-    if constexpr (AB3)
-        predict_cell_ab3(P, Q, oQ, pdt, odt, oodt, pQ);
-    else
-        predict_cell(P, Q, oQ, pdt, qodt, pQ);
-    R Wh[5], Wn[5];
-    block_c2p(P, pQ, Wh);
-    if (P.doLFMLim) block_c2p(P, Q, Wn);
-    const R vol = g.vol[c];
+    R pQ[5], Wn[5];
+    {
+        // CellC2P of State n and BlockCon2Prim's primitives of it divide by the
+        // same density unless the floor acts on it
+        R W[5], oW[5];
+        const R rho = Q[0], D = rmax(rho, P.dFloor);
+        const QuotTry<R, EXACT> qD(D), qo(oQ[0]);
+        Wn[0] = W[0] = D;
 #pragma unroll
-    for (int v = 0; v < 5; v++) {
-        w.QW[v * fs + c] = vol * Wh[v];
-        w.Wn[v * fs + c] = P.doLFMLim ? Wn[v] : Wh[v];
+        for (int x = 0; x < 3; x++) Wn[1 + x] = W[1 + x] = qD(Q[1 + x], ok);
+        Wn[4] = rmax(P.gm1 * (Q[4] - qD((R)0.5 * (Q[1] * Q[1] + Q[2] * Q[2] + Q[3] * Q[3]), ok)), P.pFloor);
+        if (D != rho) {
+#pragma unroll
+            for (int x = 0; x < 3; x++) W[1 + x] = Q[1 + x] / rho;
+        }
+        W[4] = rmax(P.gm1 * (Q[4] - (R)0.5 * rho * (W[1] * W[1] + W[2] * W[2] + W[3] * W[3])), P.pFloor);
+#pragma unroll
+        for (int x = 0; x < 3; x++) oW[1 + x] = qo(oQ[1 + x], ok);
+        oW[0] = rmax(oQ[0], P.dFloor);
+        oW[4] = rmax(P.gm1 * (oQ[4] - (R)0.5 * oQ[0] * (oW[1] * oW[1] + oW[2] * oW[2] + oW[3] * oW[3])), P.pFloor);
+        if constexpr (AB3) {
+            predict_prim_ab3(P, W, oW, pdt, odt, oodt, pQ);
+        } else {
+            R pW[5];
+#pragma unroll
+            for (int v = 0; v < 5; v++) pW[v] = W[v] + pdt * qodt(W[v] - oW[v], ok);
+            pW[0] = rmax(pW[0], P.dFloor);
+            pW[4] = rmax(pW[4], P.pFloor);
+            const R KinE = (R)0.5 * pW[0] * (pW[1] * pW[1] + pW[2] * pW[2] + pW[3] * pW[3]);  // CellP2C
+            pQ[0] = pW[0];
+#pragma unroll
+            for (int x = 0; x < 3; x++) pQ[1 + x] = pW[0] * pW[1 + x];
+            pQ[4] = QuotTry<R, EXACT>(P.gm1, P.rgm1)(pW[4], ok) + KinE;
+        }
     }
-    w.Dh[c] = Wh[0];
-    const R Dm = rmax(pQ[0], P.dFloor);
-    const Quot<R> qDm(Dm);
+    const R vol = __ldg(g.vol + c);
+    {
+        // BlockCon2Prim of the half state, and volume * momentum / density by the same density
+        R Wh[5];
+        Wh[0] = rmax(pQ[0], P.dFloor);
+        const QuotTry<R, EXACT> qh(Wh[0]);
 #pragma unroll
-    for (int x = 0; x < 3; x++) w.VdV[x * fs + c] = qDm(vol * pQ[1 + x]);
+        for (int x = 0; x < 3; x++) Wh[1 + x] = qh(pQ[1 + x], ok);
+        Wh[4] = rmax(P.gm1 * (pQ[4] - qh((R)0.5 * (pQ[1] * pQ[1] + pQ[2] * pQ[2] + pQ[3] * pQ[3]), ok)), P.pFloor);
+#pragma unroll
+        for (int v = 0; v < 5; v++) {
+            w.QW[v * fs + c] = vol * Wh[v];
+            w.Wn[v * fs + c] = P.doLFMLim ? Wn[v] : Wh[v];
+        }
+        w.Dh[c] = Wh[0];
+#pragma unroll
+        for (int x = 0; x < 3; x++) w.VdV[x * fs + c] = qh(vol * pQ[1 + x], ok);
+    }
     if (P.doMHD) {
         // upper faces of this cell, recomputed with the same ExtrapAB2
         R up[3];
+        if constexpr (AB3) {
 #pragma unroll
-        for (int d = 0; d < 3; d++) {
-            if constexpr (AB3) {
-                up[d] = extrap_ab3(pdt, uQ[d], uoQ[d], uooQ[d], odt, oodt);
-            } else {
-                R dQ = qodt(uQ[d] - uoQ[d]);
-                up[d] = uQ[d] + pdt * dQ;
-            }
+            for (int d = 0; d < 3; d++) up[d] = extrap_ab3(pdt, uQ[d], uoQ[d], uooQ[d], odt, oodt);
+        } else {
+#pragma unroll
+            for (int d = 0; d < 3; d++) up[d] = uQ[d] + pdt * qodt(uQ[d] - uoQ[d], ok);
         }
         R B[3];
         int jc = jj, kc = kk;
@@ -605,19 +682,54 @@ __global__ void __launch_bounds__(256, MINB) k_predict(GamBox b, DevParams<R> P,
                     lo[d] = extrap_ab3(pdt, cur.mf[f0], old.mf[f0], oomf[f0], odt, oodt);
                     hi[d] = extrap_ab3(pdt, cur.mf[f1], old.mf[f1], oomf[f1], odt, oodt);
                 } else {
-                    lo[d] = cur.mf[f0] + pdt * qodt(cur.mf[f0] - old.mf[f0]);
-                    hi[d] = cur.mf[f1] + pdt * qodt(cur.mf[f1] - old.mf[f1]);
+                    lo[d] = cur.mf[f0] + pdt * qodt(cur.mf[f0] - old.mf[f0], ok);
+                    hi[d] = cur.mf[f1] + pdt * qodt(cur.mf[f1] - old.mf[f1], ok);
                 }
             }
-            cell_bxyz(b, g, cc, lo[0], hi[0], lo[1], hi[1], lo[2], hi[2], B);
+            const QuotTry<R, EXACT> qv(__ldg(g.vol + cc));
+            cell_bxyz_q(b, g, cc, lo[0], hi[0], lo[1], hi[1], lo[2], hi[2], [&](R a) { return qv(a, ok); }, B);
         } else {
-            cell_bxyz(b, g, c, hm[0], up[0], hm[1], up[1], hm[2], up[2], B);
+            const QuotTry<R, EXACT> qv(vol);
+            cell_bxyz_q(b, g, c, hm[0], up[0], hm[1], up[1], hm[2], up[2], [&](R a) { return qv(a, ok); }, B);
         }
 #pragma unroll
         for (int x = 0; x < 3; x++) {
             w.QB[x * fs + c] = vol * B[x];
             if (!P.doLFMLim) w.Bl[x * fs + c] = B[x];
         }
+    }
+}
+
+// Predictor over every face and cell of the ghosted box. Besides the half
+// state it stores the operands every later stencil uses, each computed once:
+// volume * primitive (the recon operand QdV of Cen8LRs/Up7LRs), the limiter
+// primitives, volume * momentum / density (Mom2Face), and per face
+// area * flux/max(area,TINY) and flux/max(area,TINY) (EdgeLRs), flux/area (Fluxes).
+template <class R, int MINB, bool AB3 = false>
+__global__ void __launch_bounds__(256, MINB) k_predict(GamBox b, DevParams<R> P, Geo<R> g, StateBuf<R> cur,
+                                                 StateBuf<R> old, Work<R> w, const GamScalars* sc,
+                                                 const R* __restrict__ oomf) {
+    if (sc->halted) return;
+    int ii, jj, kk;
+    Range r{0, b.Ni, 0, b.Nj, 0, b.Nk};
+    if (!thread_ijk(r, ii, jj, kk)) return;
+    const long fs = b.fs;
+    const long c = lidx(b, ii, jj, kk);
+    const R pdt = (R)sc->pdt, odt = (R)sc->odt;
+    const bool isCell = ii < b.Ni && jj < b.Nj && kk < b.Nk;
+    GAM_BOX_CHECK(c, isCell ? c + b.sk : c, 1);
+    [[maybe_unused]] R oodt = (R)0;
+    if constexpr (AB3) oodt = (R)sc->oodt;
+#ifdef GAM_GEO_TABLES
+    const R rodt = (R)sc->rodt;
+#else
+    const R rodt = (R)1 / odt;
+#endif
+    bool ok = true;
+    predict_at<R, AB3, false>(b, P, g, cur, old, w, oomf, ii, jj, kk, c, isCell, pdt, odt, rodt, oodt, ok);
+    if constexpr (TwoTries<R>::v) {  // an operand out of the quick quotients' range: once more
+        if (!ok)
+            predict_at<R, AB3, true>(b, P, g, cur, old, w, oomf, ii, jj, kk, c, isCell, pdt, odt, rodt, oodt, ok);
     }
 }
 
@@ -831,7 +943,7 @@ __device__ __forceinline__ void mag_kin_flux(const DevParams<R>& P, R sgn, const
 template <class R>
 __device__ __forceinline__ void gas_kin_flux(const DevParams<R>& P, R sgn, const R* W, const R* T, R* gF, R* dW) {
     R D = W[0], Pr = W[4], Vx = W[1], Vy = W[2], Vz = W[3];
-    R E = (R)0.5 * D * (Vx * Vx + Vy * Vy + Vz * Vz) + Pr / P.gm1;
+    R E = (R)0.5 * D * (Vx * Vx + Vy * Vy + Vz * Vz) + gm1_quot(P)(Pr);
     R lambda = D / ((R)2 * Pr);
     R Vn = T[0] * Vx + T[1] * Vy + T[2] * Vz;
     R Vt1 = T[3] * Vx + T[4] * Vy + T[5] * Vz;
@@ -1119,12 +1231,14 @@ __device__ __forceinline__ double cell_dt(const DevParams<R>& P, const double* U
                                           double gamma, double gm1, double CFL) {
     double rho = U[0];
     const Quot<double> qr(rho);
-    double Vx = qr(U[1]), Vy = qr(U[2]), Vz = qr(U[3]);
+    double Vel[3];
+    qr.many<3>(U + 1, Vel);
+    double Vx = Vel[0], Vy = Vel[1], Vz = Vel[2];
     double MagV = sqrt(Vx * Vx + Vy * Vy + Vz * Vz);
     double ke = 0.5 * rho * (MagV * MagV);
     double e = U[4] - ke;
     double Pr = gm1 * e;
-    double Cs = sqrt(gamma * Pr / rho);
+    double Cs = sqrt(qr(gamma * Pr));
     double Valf = 0.0;
     if (P.doMHD) {
         double MagB = sqrt(Bt[0] * Bt[0] + Bt[1] * Bt[1] + Bt[2] * Bt[2]);
@@ -1184,8 +1298,92 @@ __device__ __forceinline__ void cell_boris(const DevParams<R>& P, R* U2, const R
     cell_p2c(P, W2, U2);
 }
 
-// Flux2Deltas + CellReynolds + bFlux2Fld + CellMaxwell for active cells,
-// copy + bFlux2Fld for ghost cells, then the CFL dt of cells in the dt range.
+// Flux2Deltas + CellReynolds + bFlux2Fld + CellMaxwell of an active cell, copy +
+// bFlux2Fld of a ghost cell: the new conserved state U and field Bc
+template <class R, bool BORIS, bool EXACT>
+__device__ __forceinline__ void update_cell(const GamBox& b, const DevParams<R>& P, const Geo<R>& g,
+                                            const StateBuf<R>& cur, const StateBuf<R>& nxt, const Work<R>& w, int ii,
+                                            int jj, int kk, long c, bool active, R dt, R* U, R* Bc, bool& ok) {
+    const long fs = b.fs;
+    // bFlux2Fld and Flux2Deltas divide by the same cell volume
+    const QuotTry<R, EXACT> qv(__ldg(g.vol + c));
+    auto qdV = [&](R a) { return qv(a, ok); };
+#pragma unroll
+    for (int x = 0; x < 3; x++) Bc[x] = (R)0;
+    if (P.doMHD) {
+        const long sj = b.sx, sk = b.sk;
+        int jc = jj, kc = kk;
+        // RingFlux2FieldFix: a cell across the pole takes its conjugate's
+        // field (the same volume, so the same quotient)
+        const long cb = (P.ring.on && ring_conj_cc(b, P.ring, jc, kc)) ? lidx(b, ii, jc, kc) : c;
+        cell_bxyz_q(b, g, cb, nxt.mf[cb], nxt.mf[cb + 1], nxt.mf[fs + cb], nxt.mf[fs + cb + sj], nxt.mf[2 * fs + cb],
+                  nxt.mf[2 * fs + cb + sk], qdV, Bc);
+    }
+    if (active) {
+        const long sj = b.sx, sk = b.sk;
+        R dGasH[5];
+#pragma unroll
+        for (int v = 0; v < 5; v++) {
+            const R* gI = w.gF + (v + 0) * fs;
+            const R* gJ = w.gF + (v + 5) * fs;
+            const R* gK = w.gF + (v + 10) * fs;
+            dGasH[v] = qdV(gI[c] - gI[c + 1] + gJ[c] - gJ[c + sj] + gK[c] - gK[c + sk]);
+            U[v] = cur.Gas[v * fs + c] + dt * dGasH[v];
+        }
+        if (P.doMHD) {
+            R dGasM[3];
+#pragma unroll
+            for (int x = 0; x < 3; x++) {
+                const R* mI = w.mF + (x + 0) * fs;
+                const R* mJ = w.mF + (x + 3) * fs;
+                const R* mK = w.mF + (x + 6) * fs;
+                dGasM[x] = qdV(mI[c] - mI[c + 1] + mJ[c] - mJ[c + sj] + mK[c] - mK[c + sk]);
+                if (P.doBackground) dGasM[x] = dGasM[x] + (R)g.dpB0[x * fs + c];
+            }
+            if constexpr (BORIS) {
+                R U0[5], B2[3], B0[3];
+#pragma unroll
+                for (int v = 0; v < 5; v++) U0[v] = cur.Gas[v * fs + c];
+#pragma unroll
+                for (int x = 0; x < 3; x++) {
+                    B2[x] = Bc[x];
+                    B0[x] = cur.B[x * fs + c];
+                    if (P.doBackground) {
+                        const R b0 = (R)g.B0[x * fs + c];
+                        B2[x] = B2[x] + b0;
+                        B0[x] = B0[x] + b0;
+                    }
+                }
+                cell_boris(P, U, U0, B2, B0, dGasH, dGasM, (R)P.Ca, dt);
+            } else {
+            // CellMaxwell (mhdgroup.F90:299-329)
+            R D = rmax(U[0], P.dFloor);
+            const QuotTry<R, EXACT> qd(D);
+            auto qD = [&](R a) { return qd(a, ok); };
+            R Mx = U[1], My = U[2], Mz = U[3], TotE = U[4];
+            R KinE = qD((R)0.5 * (Mx * Mx + My * My + Mz * Mz));
+            R Pr = rmax(P.gm1 * (TotE - KinE), P.pFloor);
+            Mx = Mx + dt * dGasM[0];
+            My = My + dt * dGasM[1];
+            Mz = Mz + dt * dGasM[2];
+            KinE = qD((R)0.5 * (Mx * Mx + My * My + Mz * Mz));
+            U[0] = D;
+            U[1] = Mx;
+            U[2] = My;
+            U[3] = Mz;
+            U[4] = KinE + QuotTry<R, EXACT>(P.gm1, P.rgm1)(Pr, ok);
+            }
+        }
+    } else {
+#pragma unroll
+        for (int v = 0; v < 5; v++) U[v] = cur.Gas[v * fs + c];
+    }
+}
+
+// update_cell for every cell, then the CFL dt of cells in the dt range. Bound by
+// the latency of its ~85 loads per cell: the strict form's branch at each
+// quotient kept the next loads waiting (192^3: 932 -> 732 us with quick
+// quotients and one check at the end; the FMA form, which has none, 625).
 template <class R, int MINB, bool BORIS = false>
 __global__ void __launch_bounds__(128, MINB) k_update_cells(GamBox b, DevParams<R> P, Geo<R> g, StateBuf<R> cur,
                                                       StateBuf<R> nxt, Work<R> w, GamScalars* sc, double gamma_d,
@@ -1204,76 +1402,11 @@ __global__ void __launch_bounds__(128, MINB) k_update_cells(GamBox b, DevParams<
         const int G = GAM_NG;
         const bool active = ii >= G && ii < G + b.Nip && jj >= G && jj < G + b.Njp && kk >= G && kk < G + b.Nkp;
         const R dt = (R)sc->dt;
-        R U[5];
-        R Bc[3] = {(R)0, (R)0, (R)0};
-        // bFlux2Fld and Flux2Deltas divide by the same cell volume
-        const Quot<R> qdV(g.vol[c]);
-        if (P.doMHD) {
-            const long sj = b.sx, sk = b.sk;
-            int jc = jj, kc = kk;
-            // RingFlux2FieldFix: a cell across the pole takes its conjugate's
-            // field (the same volume, so the same quotient)
-            const long cb = (P.ring.on && ring_conj_cc(b, P.ring, jc, kc)) ? lidx(b, ii, jc, kc) : c;
-            cell_bxyz(b, g, cb, nxt.mf[cb], nxt.mf[cb + 1], nxt.mf[fs + cb], nxt.mf[fs + cb + sj], nxt.mf[2 * fs + cb],
-                      nxt.mf[2 * fs + cb + sk], qdV, Bc);
-        }
-        if (active) {
-            const long sj = b.sx, sk = b.sk;
-            R dGasH[5];
-#pragma unroll
-            for (int v = 0; v < 5; v++) {
-                const R* gI = w.gF + (v + 0) * fs;
-                const R* gJ = w.gF + (v + 5) * fs;
-                const R* gK = w.gF + (v + 10) * fs;
-                dGasH[v] = qdV(gI[c] - gI[c + 1] + gJ[c] - gJ[c + sj] + gK[c] - gK[c + sk]);
-                U[v] = cur.Gas[v * fs + c] + dt * dGasH[v];
-            }
-            if (P.doMHD) {
-                R dGasM[3];
-#pragma unroll
-                for (int x = 0; x < 3; x++) {
-                    const R* mI = w.mF + (x + 0) * fs;
-                    const R* mJ = w.mF + (x + 3) * fs;
-                    const R* mK = w.mF + (x + 6) * fs;
-                    dGasM[x] = qdV(mI[c] - mI[c + 1] + mJ[c] - mJ[c + sj] + mK[c] - mK[c + sk]);
-                    if (P.doBackground) dGasM[x] = dGasM[x] + (R)g.dpB0[x * fs + c];
-                }
-                if constexpr (BORIS) {
-                    R U0[5], B2[3], B0[3];
-#pragma unroll
-                    for (int v = 0; v < 5; v++) U0[v] = cur.Gas[v * fs + c];
-#pragma unroll
-                    for (int x = 0; x < 3; x++) {
-                        B2[x] = Bc[x];
-                        B0[x] = cur.B[x * fs + c];
-                        if (P.doBackground) {
-                            const R b0 = (R)g.B0[x * fs + c];
-                            B2[x] = B2[x] + b0;
-                            B0[x] = B0[x] + b0;
-                        }
-                    }
-                    cell_boris(P, U, U0, B2, B0, dGasH, dGasM, (R)P.Ca, dt);
-                } else {
-                // CellMaxwell (mhdgroup.F90:299-329)
-                R D = rmax(U[0], P.dFloor);
-                const Quot<R> qD(D);
-                R Mx = U[1], My = U[2], Mz = U[3], TotE = U[4];
-                R KinE = qD((R)0.5 * (Mx * Mx + My * My + Mz * Mz));
-                R Pr = rmax(P.gm1 * (TotE - KinE), P.pFloor);
-                Mx = Mx + dt * dGasM[0];
-                My = My + dt * dGasM[1];
-                Mz = Mz + dt * dGasM[2];
-                KinE = qD((R)0.5 * (Mx * Mx + My * My + Mz * Mz));
-                U[0] = D;
-                U[1] = Mx;
-                U[2] = My;
-                U[3] = Mz;
-                U[4] = KinE + Pr / P.gm1;
-                }
-            }
-        } else {
-#pragma unroll
-            for (int v = 0; v < 5; v++) U[v] = cur.Gas[v * fs + c];
+        R U[5], Bc[3];
+        bool tok = true;
+        update_cell<R, BORIS, false>(b, P, g, cur, nxt, w, ii, jj, kk, c, active, dt, U, Bc, tok);
+        if constexpr (TwoTries<R>::v) {
+            if (!tok) update_cell<R, BORIS, true>(b, P, g, cur, nxt, w, ii, jj, kk, c, active, dt, U, Bc, tok);
         }
         // dt range isDT..ieDT = is-1..ie+1 (init.F90:511-530, single domain);
         // evaluated before the stores so that none of its loads waits on them
@@ -2648,11 +2781,8 @@ template <class R, class F> void for_each_kernel(const Ctx<R>& C, int cur, cudaS
         if (C.P.doAB3)
             k_predict<R, sizeof(R) == 8 ? 3 : 4, true><<<grid_for(all, pblk), pblk, 0, s>>>(b, C.P, C.g, S, O, C.w, C.sc,
                                                                                           C.oomf);
-        else if (C.kvar & 8)
-            k_predict<R, 1><<<grid_for(all, pblk), pblk, 0, s>>>(b, C.P, C.g, S, O, C.w, C.sc, nullptr);
-        else  // FP64: 3 blocks/SM (4 for the strict build, measured); FP32: 4
-            k_predict<R, (sizeof(R) == 8 && !GAM_STRICT_KERNELS) ? 3 : 4><<<grid_for(all, pblk), pblk, 0, s>>>(
-                b, C.P, C.g, S, O, C.w, C.sc, nullptr);
+        else  // 3 blocks/SM in FP64 (192^3, strict: 661 us; 4: 745, 2: 754), 4 in FP32
+            k_predict<R, sizeof(R) == 8 ? 3 : 4><<<grid_for(all, pblk), pblk, 0, s>>>(b, C.P, C.g, S, O, C.w, C.sc, nullptr);
     });
     if (C.P.doMHD) {
         const Range mf[3] = {{0, b.Ni - 1, G, G + b.Njp, 0, b.Nk - 1},
@@ -2735,10 +2865,8 @@ template <class R, class F> void for_each_kernel(const Ctx<R>& C, int cur, cudaS
         }
         if (C.P.doBoris)
             k_update_cells<R, sizeof(R) == 8 ? 6 : 8, true><<<grid_for(cells, blk), blk, 0, s>>>(b, C.P, C.g, S, O, C.w, C.sc, C.gamma, C.gm1);
-        else if (C.kvar & 4)
-            k_update_cells<R, 1><<<grid_for(cells, blk), blk, 0, s>>>(b, C.P, C.g, S, O, C.w, C.sc, C.gamma, C.gm1);
-        else
-            k_update_cells<R, 8><<<grid_for(cells, blk), blk, 0, s>>>(b, C.P, C.g, S, O, C.w, C.sc, C.gamma, C.gm1);
+        else  // strict: 6 blocks/SM (732 us at 192^3; 8: 792, 5: 784, 4: 819); the other forms 8
+            k_update_cells<R, GAM_STRICT_KERNELS ? 6 : 8><<<grid_for(cells, blk), blk, 0, s>>>(b, C.P, C.g, S, O, C.w, C.sc, C.gamma, C.gm1);
         if (C.P.ring.on) launch_ring_average(C, O, s);  // mhdgroup.F90:69-74
         if (C.P.ion.push) {  // HackStep (PerStep, earthcmi.F90:224-263): PushIon, before CalcDT
             const long np = (long)C.P.ion.nIonP * b.Njp * b.Nkp;

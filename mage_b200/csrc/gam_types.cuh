@@ -60,6 +60,7 @@ struct RingData {
 
 template <class R> struct DevParams {
     R gamma, gm1, CFL, pdmb, Vd0, cHogH, cHogM, dFloor, pFloor;
+    R rgm1;  // 1/gm1, rounded
     int doMHD, doLFMLim, do25D, doBackground, up7;
     int doBoris;  // Boris correction with the speed of light Ca (init.F90:417-423)
     double Ca;
