@@ -510,6 +510,108 @@ __global__ void __launch_bounds__(128, MINB) k_stress_box(GamBox b, DevParams<R>
     }
 }
 
+// EdgeLRs (fields.F90:288-362): flux of faces of direction a, stencil along b
+template <class R>
+__device__ __forceinline__ void edge_lrs(const GamBox& b, const DevParams<R>& P, const Geo<R>& g, const Work<R>& w,
+                                         long c, int a, int bd, R* area, R& bL, R& bR, R& fA) {
+    const long fs = b.fs;
+    const long s = dstride(b, bd);
+    R qdv[8], nmag[4];
+#pragma unroll
+    for (int n = 0; n < 8; n++) {
+        area[n] = g.face[a * fs + c + (n - 4) * s];
+        qdv[n] = w.abh[a * fs + c + (n - 4) * s];
+    }
+#pragma unroll
+    for (int m = 0; m < 4; m++) nmag[m] = w.bn[a * fs + c + (m - 2) * s];
+    const R Vi = central8(area);
+    if (P.up7)
+        lrs_from_qdv(P, qdv, nmag, Quot<R>(Vi), bL, bR);
+    else
+        lrs_from_qdv(P, qdv, nmag, Quot1<R>(Vi), bL, bR);
+    fA = Vi;  // dot_product(interpWgt, AreaB) again: the same value
+    bL = bL * fA;
+    bR = bR * fA;
+}
+
+// VxB edge loop for direction eD (fields.F90:184-228). SAVE (the
+// differentiation form's forward) also stores the corner values in w.esv.
+template <class R, int MINB = 1, bool SAVE = false>
+__global__ void __launch_bounds__(128, MINB) k_vxb_box(GamBox b, DevParams<R> P, Geo<R> g, Work<R> w, int eD, Range r,
+                                             const GamScalars* sc) {
+    if (sc->halted) return;
+    int ii, jj, kk;
+    if (!thread_ijk(r, ii, jj, kk)) return;
+    int dT1, dT2;
+    edge_dirs(eD, dT1, dT2);
+    const long fs = b.fs;
+    const long c = lidx(b, ii, jj, kk);
+    // GetCornerD (fields.F90:427-454): normal-plane unit offsets e1 < e2
+    const int e1 = eD == 0 ? 1 : 0, e2 = eD == 2 ? 1 : 2;
+    const long s1 = dstride(b, e1), s2 = dstride(b, e2);
+    {
+        const long sA = dstride(b, dT1), sB = dstride(b, dT2), sM = sA > sB ? sA : sB;
+        [[maybe_unused]] const long lo = c - s1 - s2 < c - 4 * sM ? c - s1 - s2 : c - 4 * sM;
+        GAM_BOX_CHECK(lo, c + 3 * sM, 3 + 2 * eD);
+    }
+    R Dc = (R)0.25 * (w.Dh[c] + w.Dh[c - s1] + w.Dh[c - s2] + w.Dh[c - s1 - s2]);
+    // GetCornerB: EdgeLRs for dT1 faces along dT2 and dT2 faces along dT1
+    R area1[8], area2[8];
+    R bT1L, bT1R, fA1, bT2L, bT2R, fA2;
+    edge_lrs(b, P, g, w, c, dT1, dT2, area1, bT1L, bT1R, fA1);
+    edge_lrs(b, P, g, w, c, dT2, dT1, area2, bT2L, bT2R, fA2);
+    // GetCornerV (fields.F90:457-517); its area stencil equals area1
+    R dA = rmax(fA1, (R)TINY);
+    const Quot<R> qdA(dA);
+    R VC[3];
+    const long s2v = dstride(b, dT2);
+#pragma unroll
+    for (int x = 0; x < 3; x++) {
+        R acc = (R)0;
+#pragma unroll
+        for (int n = 0; n < 8; n++) acc += Rc<R>(w8(n)) * w.AVf[(x + 3 * eD) * fs + c + (n - 4) * s2v];
+        VC[x] = qdA(acc);
+    }
+    const R* Te = g.Te;
+    R v1 = VC[0] * Te[(3 + 9 * eD) * fs + c] + VC[1] * Te[(4 + 9 * eD) * fs + c] + VC[2] * Te[(5 + 9 * eD) * fs + c];
+    R v2 = VC[0] * Te[(6 + 9 * eD) * fs + c] + VC[1] * Te[(7 + 9 * eD) * fs + c] + VC[2] * Te[(8 + 9 * eD) * fs + c];
+    R vDiff = Mth<R>::sqrt_(v1 * v1 + v2 * v2);
+    R xni = g.Teb[(0 + 4 * eD) * fs + c], yni = g.Teb[(1 + 4 * eD) * fs + c];
+    R xnj = g.Teb[(2 + 4 * eD) * fs + c], ynj = g.Teb[(3 + 4 * eD) * fs + c];
+    R detT = (R)1 / (xni * ynj - xnj * yni);
+    const Quot<R> qA1(fA1), qA2(fA2);
+    R bT1 = qA1((R)0.5 * (bT1L + bT1R));
+    R bT2 = qA2((R)0.5 * (bT2L + bT2R));
+    R db1 = qA1(bT1R - bT1L);
+    R db2 = qA2(bT2R - bT2L);
+    R Jd = db2 - db1;
+    R b1 = detT * (ynj * bT1 - yni * bT2);
+    R b2 = detT * (-(xnj * bT1) + xni * bT2);
+    if (P.doBackground) {
+        b1 = b1 + (R)g.edgB0[(0 + 2 * eD) * fs + c];
+        b2 = b2 + (R)g.edgB0[(1 + 2 * eD) * fs + c];
+    }
+    R vA = qdiv(Mth<R>::sqrt_(b1 * b1 + b2 * b2), Mth<R>::sqrt_(Dc));
+    if (P.doBoris) vA = boris_speed((R)P.Ca, vA);
+    vDiff = vDiff + vA;
+    const R edge = g.edge[eD * fs + c];
+    vDiff = rmin(vDiff, P.CFL * edge / (R)sc->dt);
+    R e = -(v1 * b2 - v2 * b1) + P.Vd0 * vDiff * Jd;
+    w.E[eD * fs + c] = e * edge;
+    if constexpr (SAVE) {
+        R* o = w.esv + (long)(GAM_ESV_NC * eD) * fs + c;
+        o[0] = Dc;
+        o[fs] = bT1L;
+        o[2 * fs] = bT1R;
+        o[3 * fs] = fA1;
+        o[4 * fs] = bT2L;
+        o[5 * fs] = bT2R;
+        o[6 * fs] = fA2;
+#pragma unroll
+        for (int x = 0; x < 3; x++) o[(7 + x) * fs] = VC[x];
+    }
+}
+
 // reverse of edge_lrs (EdgeLRs for faces of direction a along bd): adjoints of
 // bL*Vi, bR*Vi -> the abh (8) and bn (4) stencils
 template <class R, class A>
@@ -1686,9 +1788,9 @@ int efield_call(const gam_params* p, const void* Dh, const void* abh, const void
         // the adjoint of a whole step finds AVf as its forward left it
         if (!(dE && avf_saved)) k_mom2face<R><<<grid(mf[eD]), blk, 0, s>>>(b, P, g, w, eD, mf[eD], sc);
         if (!dE && estates) {
-            k_vxb<R, 1, true><<<grid(ed[eD]), blk, 0, s>>>(b, P, g, w, eD, ed[eD], sc);
+            k_vxb_box<R, 1, true><<<grid(ed[eD]), blk, 0, s>>>(b, P, g, w, eD, ed[eD], sc);
         } else if (!dE) {
-            k_vxb<R><<<grid(ed[eD]), blk, 0, s>>>(b, P, g, w, eD, ed[eD], sc);
+            k_vxb_box<R><<<grid(ed[eD]), blk, 0, s>>>(b, P, g, w, eD, ed[eD], sc);
         } else if (escratch) {
             // deterministic: the edges store their adjoints (14 components
             // from escratch + 14 eD fs), gathered per position after the third

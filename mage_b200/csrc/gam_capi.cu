@@ -43,8 +43,10 @@ void gam_geom_dxf(const GamBox& b, const double* xfc, const double* xyzcc, float
 void gam_geom_metric(const GamBox& b, const double* xyz, double* face, double* xfc, double* Tf, double* vol,
                      double* xyzcc, double* dijk, double* dl, double* edge, double* Te, double* Teb,
                      const GamRingGeo& ring, cudaStream_t s);
-void gam_geom_tables_d(const GamBox& b, const double* vol, double* vif, double* rvif, cudaStream_t s);
-void gam_geom_tables_f(const GamBox& b, const double* vol, float* vif, float* rvif, cudaStream_t s);
+void gam_geom_tables(const GamBox& b, const double* vol, const double* face, const double* Teb, const Geo<double>& g,
+                     cudaStream_t s);
+void gam_geom_tables(const GamBox& b, const double* vol, const double* face, const double* Teb, const Geo<float>& g,
+                     cudaStream_t s);
 void gam_geom_ic_ot(const GamBox& b, const double* xyzcc, const double* face, double* Gas, double* mf, double gamma,
                     cudaStream_t s);
 void gam_geom_ic_case(const GamBox& b, const double* xyz, const double* xyzcc, const double* vol, double* Gas,
@@ -191,21 +193,26 @@ template <class R> static void fill_dev_params(DevParams<R>& P, const gam_params
     P.dtIlo = P.dtIhi = P.dtJlo = P.dtJhi = 1;
 }
 
-// The tensor maps of the flux kernels' boxes (FluxTile): fields of nc
-// components over the box, components fs apart
+// The tensor maps of the flux and edge kernels' boxes (FluxTile, EdgeTile):
+// fields of nc components over the grid's box, components fs apart; bc of them
+// in one copy (0: all)
 template <class R>
-static bool encode_box(const GamBox& b, const R* base, int nc, int bx, int by, int bz, CUtensorMap* m) {
+static bool encode_box(const GamBox& b, const R* base, int nc, int bx, int by, int bz, CUtensorMap* m, int bc = 0) {
     typedef CUresult (*Encode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-        return false;
+    static void* const f = [] {  // the driver's entry point, the same for every handle
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
+                       q == cudaDriverEntryPointSuccess
+                   ? p
+                   : nullptr;
+    }();
+    if (!f) return false;
     const cuuint64_t dim[4] = {(cuuint64_t)b.sx, (cuuint64_t)(b.Nj + 1), (cuuint64_t)(b.Nk + 1), (cuuint64_t)nc};
     const cuuint64_t str[3] = {b.sx * sizeof(R), b.sk * sizeof(R), b.fs * sizeof(R)};
-    const cuuint32_t box[4] = {(cuuint32_t)bx, (cuuint32_t)by, (cuuint32_t)bz, (cuuint32_t)nc}, es[4] = {1, 1, 1, 1};
+    const cuuint32_t box[4] = {(cuuint32_t)bx, (cuuint32_t)by, (cuuint32_t)bz, (cuuint32_t)(bc ? bc : nc)}, es[4] = {1, 1, 1, 1};
     return ((Encode)f)(m, sizeof(R) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
                        (void*)base, dim, str, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                        CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
@@ -224,8 +231,19 @@ template <class R, int D> static bool flux_maps_of(gam_handle* h, Ctx<R>& C) {
     }
     return true;
 }
+template <class R, int E> static bool edge_maps_of(gam_handle* h, Ctx<R>& C) {
+    using T_ = EdgeTile<E>;
+    const R* base[6] = {C.w.abh, C.w.abh, C.w.AVf, C.w.bn, C.w.bn, C.w.Dh};
+    const int nc[6] = {3, 3, 9, 3, 3, 1}, bc[6] = {1, 1, 3, 1, 1, 1};
+    for (int q = 0; q < 6; q++)
+        if (T_::off(q) * sizeof(R) % 128 != 0 ||
+            !encode_box<R>(h->b, base[q], nc[q], T_::ext(q, 0), T_::ext(q, 1), T_::ext(q, 2), &h->fmaps.e[E].m[q], bc[q]))
+            return false;
+    return true;
+}
 template <class R> static bool make_flux_maps(gam_handle* h, Ctx<R>& C) {
-    return flux_maps_of<R, 0>(h, C) && flux_maps_of<R, 1>(h, C) && flux_maps_of<R, 2>(h, C);
+    return flux_maps_of<R, 0>(h, C) && flux_maps_of<R, 1>(h, C) && flux_maps_of<R, 2>(h, C) &&
+           edge_maps_of<R, 0>(h, C) && edge_maps_of<R, 1>(h, C) && edge_maps_of<R, 2>(h, C);
 }
 
 template <class R> static int alloc_bulk(gam_handle* h, Ctx<R>& C) {
@@ -268,13 +286,15 @@ template <class R> static int alloc_bulk(gam_handle* h, Ctx<R>& C) {
         C.g.edge = edge; C.g.Te = Te; C.g.Teb = Teb; C.g.dxf = dxf;
     }
     {
-        // the strict form divides by the interpolated volume, the others
-        // multiply by its reciprocal
-        R *vif = nullptr, *rvif;
-        if (h->p.strict) A(vif, 3);
-        A(rvif, 3);
-        C.g.vif = vif;
-        C.g.rvif = rvif;
+        // the strict form divides by the interpolated volumes and areas, the
+        // others multiply by their reciprocals
+        R *vif = nullptr, *fae = nullptr, *rvif, *rfae, *rdet;
+        if (h->p.strict) {
+            A(vif, 3);
+            A(fae, 6);
+        }
+        A(rvif, 3); A(rfae, 6); A(rdet, 3);
+        C.g.vif = vif; C.g.rvif = rvif; C.g.fae = fae; C.g.rfae = rfae; C.g.rdet = rdet;
     }
 #undef A
     if (!make_flux_maps(h, C)) return fail(h, GAM_ECUDA, "cuTensorMapEncodeTiled failed");
@@ -289,8 +309,7 @@ template <class R> static int alloc_bulk(gam_handle* h, Ctx<R>& C) {
     C.sc = h->sc;
     C.gamma = h->p.gamma;
     C.gm1 = h->p.gamma - 1;
-    const char* kv = getenv("GAM_KVAR");  // launch-configuration experiments
-    C.kvar = kv ? atoi(kv) : 0;
+    C.kvar = 0;
     return GAM_OK;
 }
 
@@ -472,8 +491,7 @@ template <class R> static int down_r(gam_handle* h, const R* src, double* dst, b
 // the compute form's copies and tables of a geometry just set
 static void sync_geo(gam_handle* h) {
     if (!h->f32) {
-        const Geo<double>& g = h->cd.g;
-        gam_geom_tables_d(h->b, h->gd.vol, (double*)g.vif, (double*)g.rvif, h->s);
+        gam_geom_tables(h->b, h->gd.vol, h->gd.face, h->gd.Teb, h->cd.g, h->s);
         return;
     }
     Geo<float>& g = h->cf.g;
@@ -488,7 +506,7 @@ static void sync_geo(gam_handle* h) {
     gam_geom_d2f(h->gd.Te, (float*)g.Te, 27 * fs, h->s);
     gam_geom_d2f(h->gd.Teb, (float*)g.Teb, 12 * fs, h->s);
     gam_geom_dxf(h->b, h->gd.xfc, h->gd.xyzcc, (float*)g.dxf, h->s);
-    gam_geom_tables_f(h->b, h->gd.vol, (float*)g.vif, (float*)g.rvif, h->s);
+    gam_geom_tables(h->b, h->gd.vol, h->gd.face, h->gd.Teb, h->cf.g, h->s);
 }
 
 static bool has_lfm(const gam_handle* h) { return h->p.bc[2] == GAM_BC_LFM || h->p.bc[3] == GAM_BC_LFM; }

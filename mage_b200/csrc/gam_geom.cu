@@ -343,6 +343,26 @@ __device__ __forceinline__ double cen8(const double* q, long s) {
     for (int n = 0; n < 8; n++) a += w[n] * q[(n - 4) * s];
     return a;
 }
+// on the active edges: the interpolant of the areas of dT1 faces along dT2 and
+// of dT2 faces along dT1, its reciprocal, and 1/(xi yj - xj yi) of the B map
+template <class T>
+__global__ void k_geo_edge_tables(GamBox b, const double* __restrict__ face, const double* __restrict__ Teb,
+                                  T* __restrict__ fae, T* __restrict__ rfae, T* __restrict__ rdet) {
+    int ii, jj, kk;
+    if (!tid3(b.Nip + 1, b.Njp + 1, b.Nkp + 1, ii, jj, kk)) return;
+    const long c = lidx(b, ii + GAM_NG, jj + GAM_NG, kk + GAM_NG), fs = b.fs;
+    const long st[3] = {1L, (long)b.sx, b.sk};
+    for (int eD = 0; eD < 3; eD++) {
+        const int d1 = (eD + 1) % 3, d2 = (eD + 2) % 3;
+        const double a[2] = {cen8(face + d1 * fs + c, st[d2]), cen8(face + d2 * fs + c, st[d1])};
+        for (int q = 0; q < 2; q++) {
+            if (fae) fae[(q + 2 * eD) * fs + c] = (T)a[q];
+            rfae[(q + 2 * eD) * fs + c] = (T)(1.0 / a[q]);
+        }
+        const double* t = Teb + 4 * eD * fs + c;
+        rdet[eD * fs + c] = (T)(1.0 / (t[0] * t[3 * fs] - t[2 * fs] * t[fs]));
+    }
+}
 template <class T>
 __global__ void k_geo_tables(GamBox b, const double* __restrict__ vol, T* __restrict__ vif, T* __restrict__ rvif) {
     int ii, jj, kk;
@@ -876,13 +896,21 @@ void gam_geom_metric(const GamBox& b, const double* xyz, double* face, double* x
     }
 }
 
-void gam_geom_tables_d(const GamBox& b, const double* vol, double* vif, double* rvif, cudaStream_t s) {
+template <class T>
+static void geom_tables(const GamBox& b, const double* vol, const double* face, const double* Teb, const Geo<T>& g,
+                        cudaStream_t s) {
     dim3 blk(32, 4, 1);
-    k_geo_tables<double><<<g3(b.Ni, b.Nj, b.Nk, blk), blk, 0, s>>>(b, vol, vif, rvif);
+    k_geo_tables<T><<<g3(b.Ni, b.Nj, b.Nk, blk), blk, 0, s>>>(b, vol, (T*)g.vif, (T*)g.rvif);
+    k_geo_edge_tables<T><<<g3(b.Nip + 1, b.Njp + 1, b.Nkp + 1, blk), blk, 0, s>>>(b, face, Teb, (T*)g.fae, (T*)g.rfae,
+                                                                                  (T*)g.rdet);
 }
-void gam_geom_tables_f(const GamBox& b, const double* vol, float* vif, float* rvif, cudaStream_t s) {
-    dim3 blk(32, 4, 1);
-    k_geo_tables<float><<<g3(b.Ni, b.Nj, b.Nk, blk), blk, 0, s>>>(b, vol, vif, rvif);
+void gam_geom_tables(const GamBox& b, const double* vol, const double* face, const double* Teb, const Geo<double>& g,
+                     cudaStream_t s) {
+    geom_tables(b, vol, face, Teb, g, s);
+}
+void gam_geom_tables(const GamBox& b, const double* vol, const double* face, const double* Teb, const Geo<float>& g,
+                     cudaStream_t s) {
+    geom_tables(b, vol, face, Teb, g, s);
 }
 void gam_geom_ic_ot(const GamBox& b, const double* xyzcc, const double* face, double* Gas, double* mf, double gamma,
                     cudaStream_t s) {

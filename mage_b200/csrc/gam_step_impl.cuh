@@ -733,147 +733,6 @@ __global__ void __launch_bounds__(256, MINB) k_predict(GamBox b, DevParams<R> P,
     }
 }
 
-// Edge geometry of the EMF in direction eD (fields.F90:84-170): face
-// direction dT1 (Mom2Face sweep), dT2 (corner sweep)
-__device__ __forceinline__ void edge_dirs(int eD, int& dT1, int& dT2) {
-    dT1 = (eD + 1) % 3;
-    dT2 = (eD + 2) % 3;
-}
-
-// Mom2Face for edge direction eD over the reference's loop range; stores
-// area(dT1) * Vf, the operand of GetCornerV's weighted interpolation.
-template <class R>
-__global__ void __launch_bounds__(256) k_mom2face(GamBox b, DevParams<R> P, Geo<R> g, Work<R> w, int eD, Range r,
-                                                  const GamScalars* sc) {
-    if (sc->halted) return;
-    int ii, jj, kk;
-    if (!thread_ijk(r, ii, jj, kk)) return;
-    int dT1, dT2;
-    edge_dirs(eD, dT1, dT2);
-    const long fs = b.fs;
-    const long c = lidx(b, ii, jj, kk);
-    const long s = dstride(b, dT1);
-    GAM_BOX_CHECK(c - 4 * s, c + 3 * s, 2 + 2 * eD);
-    R vol[8];
-#pragma unroll
-    for (int n = 0; n < 8; n++) vol[n] = g.vol[c + (n - 4) * s];
-    R dV = rmax(central8(vol), (R)TINY);
-    const Quot<R> qdV(dV);
-    const R A = g.face[dT1 * fs + c];
-    R out[3];
-#pragma unroll
-    for (int x = 0; x < 3; x++) {
-        R q[8];
-#pragma unroll
-        for (int n = 0; n < 8; n++) q[n] = w.VdV[x * fs + c + (n - 4) * s];
-        out[x] = A * qdV(central8(q));
-    }
-#pragma unroll
-    for (int x = 0; x < 3; x++) w.AVf[(x + 3 * eD) * fs + c] = out[x];
-}
-
-// EdgeLRs (fields.F90:288-362): flux of faces of direction a, stencil along b
-template <class R>
-__device__ __forceinline__ void edge_lrs(const GamBox& b, const DevParams<R>& P, const Geo<R>& g, const Work<R>& w,
-                                         long c, int a, int bd, R* area, R& bL, R& bR, R& fA) {
-    const long fs = b.fs;
-    const long s = dstride(b, bd);
-    R qdv[8], nmag[4];
-#pragma unroll
-    for (int n = 0; n < 8; n++) {
-        area[n] = g.face[a * fs + c + (n - 4) * s];
-        qdv[n] = w.abh[a * fs + c + (n - 4) * s];
-    }
-#pragma unroll
-    for (int m = 0; m < 4; m++) nmag[m] = w.bn[a * fs + c + (m - 2) * s];
-    const R Vi = central8(area);
-    if (P.up7)
-        lrs_from_qdv(P, qdv, nmag, Quot<R>(Vi), bL, bR);
-    else
-        lrs_from_qdv(P, qdv, nmag, Quot1<R>(Vi), bL, bR);
-    fA = Vi;  // dot_product(interpWgt, AreaB) again: the same value
-    bL = bL * fA;
-    bR = bR * fA;
-}
-
-// VxB edge loop for direction eD (fields.F90:184-228). SAVE (the
-// differentiation form's forward) also stores the corner values in w.esv.
-template <class R, int MINB = 1, bool SAVE = false>
-__global__ void __launch_bounds__(128, MINB) k_vxb(GamBox b, DevParams<R> P, Geo<R> g, Work<R> w, int eD, Range r,
-                                             const GamScalars* sc) {
-    if (sc->halted) return;
-    int ii, jj, kk;
-    if (!thread_ijk(r, ii, jj, kk)) return;
-    int dT1, dT2;
-    edge_dirs(eD, dT1, dT2);
-    const long fs = b.fs;
-    const long c = lidx(b, ii, jj, kk);
-    // GetCornerD (fields.F90:427-454): normal-plane unit offsets e1 < e2
-    const int e1 = eD == 0 ? 1 : 0, e2 = eD == 2 ? 1 : 2;
-    const long s1 = dstride(b, e1), s2 = dstride(b, e2);
-    {
-        const long sA = dstride(b, dT1), sB = dstride(b, dT2), sM = sA > sB ? sA : sB;
-        [[maybe_unused]] const long lo = c - s1 - s2 < c - 4 * sM ? c - s1 - s2 : c - 4 * sM;
-        GAM_BOX_CHECK(lo, c + 3 * sM, 3 + 2 * eD);
-    }
-    R Dc = (R)0.25 * (w.Dh[c] + w.Dh[c - s1] + w.Dh[c - s2] + w.Dh[c - s1 - s2]);
-    // GetCornerB: EdgeLRs for dT1 faces along dT2 and dT2 faces along dT1
-    R area1[8], area2[8];
-    R bT1L, bT1R, fA1, bT2L, bT2R, fA2;
-    edge_lrs(b, P, g, w, c, dT1, dT2, area1, bT1L, bT1R, fA1);
-    edge_lrs(b, P, g, w, c, dT2, dT1, area2, bT2L, bT2R, fA2);
-    // GetCornerV (fields.F90:457-517); its area stencil equals area1
-    R dA = rmax(fA1, (R)TINY);
-    const Quot<R> qdA(dA);
-    R VC[3];
-    const long s2v = dstride(b, dT2);
-#pragma unroll
-    for (int x = 0; x < 3; x++) {
-        R acc = (R)0;
-#pragma unroll
-        for (int n = 0; n < 8; n++) acc += Rc<R>(w8(n)) * w.AVf[(x + 3 * eD) * fs + c + (n - 4) * s2v];
-        VC[x] = qdA(acc);
-    }
-    const R* Te = g.Te;
-    R v1 = VC[0] * Te[(3 + 9 * eD) * fs + c] + VC[1] * Te[(4 + 9 * eD) * fs + c] + VC[2] * Te[(5 + 9 * eD) * fs + c];
-    R v2 = VC[0] * Te[(6 + 9 * eD) * fs + c] + VC[1] * Te[(7 + 9 * eD) * fs + c] + VC[2] * Te[(8 + 9 * eD) * fs + c];
-    R vDiff = Mth<R>::sqrt_(v1 * v1 + v2 * v2);
-    R xni = g.Teb[(0 + 4 * eD) * fs + c], yni = g.Teb[(1 + 4 * eD) * fs + c];
-    R xnj = g.Teb[(2 + 4 * eD) * fs + c], ynj = g.Teb[(3 + 4 * eD) * fs + c];
-    R detT = (R)1 / (xni * ynj - xnj * yni);
-    const Quot<R> qA1(fA1), qA2(fA2);
-    R bT1 = qA1((R)0.5 * (bT1L + bT1R));
-    R bT2 = qA2((R)0.5 * (bT2L + bT2R));
-    R db1 = qA1(bT1R - bT1L);
-    R db2 = qA2(bT2R - bT2L);
-    R Jd = db2 - db1;
-    R b1 = detT * (ynj * bT1 - yni * bT2);
-    R b2 = detT * (-(xnj * bT1) + xni * bT2);
-    if (P.doBackground) {
-        b1 = b1 + (R)g.edgB0[(0 + 2 * eD) * fs + c];
-        b2 = b2 + (R)g.edgB0[(1 + 2 * eD) * fs + c];
-    }
-    R vA = qdiv(Mth<R>::sqrt_(b1 * b1 + b2 * b2), Mth<R>::sqrt_(Dc));
-    if (P.doBoris) vA = boris_speed((R)P.Ca, vA);
-    vDiff = vDiff + vA;
-    const R edge = g.edge[eD * fs + c];
-    vDiff = rmin(vDiff, P.CFL * edge / (R)sc->dt);
-    R e = -(v1 * b2 - v2 * b1) + P.Vd0 * vDiff * Jd;
-    w.E[eD * fs + c] = e * edge;
-    if constexpr (SAVE) {
-        R* o = w.esv + (long)(GAM_ESV_NC * eD) * fs + c;
-        o[0] = Dc;
-        o[fs] = bT1L;
-        o[2 * fs] = bT1R;
-        o[3 * fs] = fA1;
-        o[4 * fs] = bT2L;
-        o[5 * fs] = bT2R;
-        o[6 * fs] = fA2;
-#pragma unroll
-        for (int x = 0; x < 3; x++) o[(7 + x) * fs] = VC[x];
-    }
-}
-
 // Quotient by the volume interpolated to the face c of direction D: from the
 // tables made with the geometry, else from the volumes (differentiation form)
 template <class R> __device__ __forceinline__ Quot<R> face_quot(const GamBox& b, const Geo<R>& g, long c, int D) {
@@ -891,6 +750,291 @@ template <class R> __device__ __forceinline__ Quot<R> face_quot(const GamBox& b,
     return Quot<R>(central8(vol));
 #endif
 }
+// the same with the volume floored at TINY (Mom2Face)
+template <class R> __device__ __forceinline__ Quot<R> face_quot_floor(const GamBox& b, const Geo<R>& g, long c, int D) {
+#ifdef GAM_GEO_TABLES
+    R v = (R)0, rv = g.rvif[D * b.fs + c];
+#ifndef GAM_FAST_RECIP
+    v = g.vif[D * b.fs + c];
+#endif
+    if (!(rv > (R)0 && rv < (R)(1.0 / TINY))) {
+        v = (R)TINY;
+        rv = (R)(1.0 / TINY);
+    }
+    return Quot<R>(v, rv);
+#else
+    const long s = dstride(b, D);
+    R vol[8];
+#pragma unroll
+    for (int n = 0; n < 8; n++) vol[n] = g.vol[c + (n - 4) * s];
+    return Quot<R>(rmax(central8(vol), (R)TINY));
+#endif
+}
+
+// Edge geometry of the EMF in direction eD (fields.F90:84-170): face
+// direction dT1 (Mom2Face sweep), dT2 (corner sweep)
+__device__ __forceinline__ void edge_dirs(int eD, int& dT1, int& dT2) {
+    dT1 = (eD + 1) % 3;
+    dT2 = (eD + 2) % 3;
+}
+
+// Mom2Face for edge direction eD over the reference's loop range (192^3, the
+// three directions with the interpolated volume from its table: strict 503 ->
+// 375 us, FMA form 470 -> 325, FP32 276 -> 234); stores
+// area(dT1) * Vf, the operand of GetCornerV's weighted interpolation.
+template <class R>
+__global__ void __launch_bounds__(256) k_mom2face(GamBox b, DevParams<R> P, Geo<R> g, Work<R> w, int eD, Range r,
+                                                  const GamScalars* sc) {
+    if (sc->halted) return;
+    int ii, jj, kk;
+    if (!thread_ijk(r, ii, jj, kk)) return;
+    int dT1, dT2;
+    edge_dirs(eD, dT1, dT2);
+    const long fs = b.fs;
+    const long c = lidx(b, ii, jj, kk);
+    const long s = dstride(b, dT1);
+    GAM_BOX_CHECK(c - 4 * s, c + 3 * s, 2 + 2 * eD);
+    const Quot<R> qdV = face_quot_floor<R>(b, g, c, dT1);
+    const R A = g.face[dT1 * fs + c];
+    R num[3], quo[3];
+#pragma unroll
+    for (int x = 0; x < 3; x++) {
+        R q[8];
+#pragma unroll
+        for (int n = 0; n < 8; n++) q[n] = w.VdV[x * fs + c + (n - 4) * s];
+        num[x] = central8(q);
+    }
+    qdV.template many<3>(num, quo);
+#pragma unroll
+    for (int x = 0; x < 3; x++) w.AVf[(x + 3 * eD) * fs + c] = A * quo[x];
+}
+
+// EdgeLRs (fields.F90:288-362), the weighted sums of its reconstruction from
+// the operand p (the edge's own face) with stride s: one sum in 8CENT, in sR too
+template <class R> __device__ __forceinline__ void edge_sums(bool up7, const R* p, int s, R& sL, R& sR) {
+    R q[8];
+#pragma unroll
+    for (int n = 0; n < 8; n++) q[n] = p[(n - 4) * s];
+    if (!up7) {
+        sL = sR = central8(q);
+    } else {
+        sL = q[0] * Rc<R>(up7c(0));
+        sR = q[7] * Rc<R>(up7c(0));
+#pragma unroll
+        for (int n = 1; n < 7; n++) {
+            sL = sL + q[n] * Rc<R>(up7c(n));
+            sR = sR + q[7 - n] * Rc<R>(up7c(n));
+        }
+    }
+}
+
+// The metric of an edge that edge_emf takes
+template <class R> struct EdgeMetric {
+    R t1[3], t2[3];              // tangents
+    R xni, yni, xnj, ynj, detT;  // B map
+    R fA1, fA2, rA1;             // interpolated areas (not in the forms that multiply by 1/area), 1/fA1
+    R edge;
+};
+// The EMF of edge c (VxB edge loop, fields.F90:184-228) from its block's boxes in
+// shared memory (EdgeTile) and its metric. SAVE: also the corner values into
+// w.esv, where that is not null (see flux_face).
+template <class R, int E, bool SAVE>
+__device__ __forceinline__ void edge_emf(const GamBox& b, const DevParams<R>& P, const Geo<R>& g, const Work<R>& w,
+                                         long c, const R* sm, int tx, int ty, int tz, const EdgeMetric<R>& m,
+                                         const Quot<R>& qA1, const Quot<R>& qA2, const Quot<R>& qdt) {
+    using T_ = EdgeTile<E>;
+    constexpr int eD = E, dT1 = T_::d1, dT2 = T_::d2;
+    const long fs = b.fs;
+    const R* pD = sm + T_::at(5, tx, ty, tz);
+    // GetCornerD (fields.F90:427-454): normal-plane unit offsets e1 < e2
+    constexpr int e1 = E == 0 ? 1 : 0, e2 = E == 2 ? 1 : 2;
+    constexpr int h1 = T_::str(5, e1), h2 = T_::str(5, e2);
+    R Dc = (R)0.25 * (pD[0] + pD[-h1] + pD[-h2] + pD[-h1 - h2]);
+    // GetCornerB: EdgeLRs for dT1 faces along dT2 and dT2 faces along dT1, and
+    // GetCornerV (fields.F90:457-517), whose area stencil is the first one's:
+    // all sums, then their quotients by the two interpolated areas
+    R num[5], quo[5], n2[2], q2[2];
+    edge_sums(P.up7, sm + T_::at(0, tx, ty, tz), T_::str(0, dT2), num[0], num[1]);
+    edge_sums(P.up7, sm + T_::at(1, tx, ty, tz), T_::str(1, dT1), n2[0], n2[1]);
+#pragma unroll
+    for (int x = 0; x < 3; x++) {
+        const R* p = sm + T_::at(2, tx, ty, tz) + x * T_::size(2);
+        R q[8];
+#pragma unroll
+        for (int n = 0; n < 8; n++) q[n] = p[(n - 4) * T_::str(2, dT2)];
+        num[2 + x] = central8(q);
+    }
+    qA1.template many<5>(num, quo);
+    qA2.template many<2>(n2, q2);
+    R VC[3] = {quo[2], quo[3], quo[4]};
+#ifdef GAM_FAST_RECIP
+    const bool small = !(m.rA1 > (R)0 && m.rA1 <= (R)(1.0 / TINY));
+#else
+    const bool small = m.fA1 < (R)TINY;
+#endif
+    if (small) {  // GetCornerV divides by an area of TINY at least
+#pragma unroll
+        for (int x = 0; x < 3; x++) VC[x] = num[2 + x] / (R)TINY;
+    }
+    R bT1L, bT1R, bT2L, bT2R;
+    {
+        const R* p = sm + T_::at(3, tx, ty, tz);
+        constexpr int s = T_::str(3, dT2);
+        pdm_both(P.pdmb, p[-2 * s], p[-s], p[0], p[s], quo[0], quo[1], bT1L, bT1R);
+    }
+    {
+        const R* p = sm + T_::at(4, tx, ty, tz);
+        constexpr int s = T_::str(4, dT1);
+        pdm_both(P.pdmb, p[-2 * s], p[-s], p[0], p[s], q2[0], q2[1], bT2L, bT2R);
+    }
+    R v1 = VC[0] * m.t1[0] + VC[1] * m.t1[1] + VC[2] * m.t1[2];
+    R v2 = VC[0] * m.t2[0] + VC[1] * m.t2[1] + VC[2] * m.t2[2];
+    R vDiff = Mth<R>::sqrt_(v1 * v1 + v2 * v2);
+#ifdef GAM_FAST_RECIP
+    // the reference multiplies by the area and divides by it again
+    R bT1 = (R)0.5 * (bT1L + bT1R), bT2 = (R)0.5 * (bT2L + bT2R);
+    R db1 = bT1R - bT1L, db2 = bT2R - bT2L;
+#else
+    bT1L = bT1L * m.fA1;
+    bT1R = bT1R * m.fA1;
+    bT2L = bT2L * m.fA2;
+    bT2R = bT2R * m.fA2;
+    const R m1[2] = {(R)0.5 * (bT1L + bT1R), bT1R - bT1L}, m2[2] = {(R)0.5 * (bT2L + bT2R), bT2R - bT2L};
+    R o1[2], o2[2];
+    qA1.template many<2>(m1, o1);
+    qA2.template many<2>(m2, o2);
+    R bT1 = o1[0], bT2 = o2[0];
+    R db1 = o1[1], db2 = o2[1];
+#endif
+    R Jd = db2 - db1;
+    R b1 = m.detT * (m.ynj * bT1 - m.yni * bT2);
+    R b2 = m.detT * (-(m.xnj * bT1) + m.xni * bT2);
+    if (P.doBackground) {
+        b1 = b1 + (R)g.edgB0[(0 + 2 * eD) * fs + c];
+        b2 = b2 + (R)g.edgB0[(1 + 2 * eD) * fs + c];
+    }
+    R vA = qdiv(Mth<R>::sqrt_(b1 * b1 + b2 * b2), Mth<R>::sqrt_(Dc));
+    if (P.doBoris) vA = boris_speed((R)P.Ca, vA);
+    vDiff = vDiff + vA;
+    vDiff = rmin(vDiff, qdt(P.CFL * m.edge));
+    R e = -(v1 * b2 - v2 * b1) + P.Vd0 * vDiff * Jd;
+    w.E[eD * fs + c] = e * m.edge;
+    if (SAVE && w.esv) {
+        R* o = w.esv + (long)(GAM_ESV_NC * eD) * fs + c;
+        o[0] = Dc;
+        o[fs] = bT1L;
+        o[2 * fs] = bT1R;
+        o[3 * fs] = m.fA1;
+        o[4 * fs] = bT2L;
+        o[5 * fs] = bT2R;
+        o[6 * fs] = m.fA2;
+#pragma unroll
+        for (int x = 0; x < 3; x++) o[(7 + x) * fs] = VC[x];
+    }
+}
+
+#ifdef GAM_GEO_TABLES
+// ----------------------------------------------------------------- TMA
+// Box copies of a (i, j, k, component) field into shared memory and the
+// mbarrier that counts their bytes.
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void tma_bar_init(uint64_t* bar) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+__device__ __forceinline__ void tma_expect(uint64_t* bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void tma_load(void* dst, const CUtensorMap* map, int i, int j, int k, int comp,
+                                         uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
+        "[%6];" ::"r"(smem_u32(dst)), "l"(map), "r"(i), "r"(j), "r"(k), "r"(comp), "r"(smem_u32(bar))
+        : "memory");
+}
+// Wait for the first phase; false when it does not complete within the limit
+// (each try waits in hardware for a while)
+__device__ __forceinline__ bool tma_wait(uint64_t* bar) {
+    for (int n = 0; n < (1 << 20); n++) {
+        uint32_t done;
+        asm volatile(
+            "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0; selp.b32 %0, 1, 0, p; }"
+            : "=r"(done)
+            : "r"(smem_u32(bar))
+            : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+
+// VxB edge loop for direction E (fields.F90:184-228), one edge per thread. The
+// stencils (the two EdgeLRs with their limiters, GetCornerV's, GetCornerD's)
+// are read from shared memory, where one thread has the block's boxes copied
+// by TMA; the metric's loads are issued meanwhile, and what the geometry alone
+// gives (interpolated areas, the B map's determinant) comes from tables (see
+// k_stress). 192^3, the three directions: strict 366/404/416 -> 289/299/299 us,
+// FMA form 328/372/376 -> 246/248/242, FP32 211/224/225 -> 148/137/140.
+template <class R, int E, int MINB>
+__global__ void __launch_bounds__(EdgeTile<E>::NT, MINB)
+    k_vxb(GamBox b, DevParams<R> P, Geo<R> g, Work<R> w, Range r, GamScalars* sc,
+          const __grid_constant__ GamEdgeMaps maps) {
+    using T_ = EdgeTile<E>;
+    constexpr int eD = E, dT1 = T_::d1, dT2 = T_::d2;
+    extern __shared__ __align__(128) unsigned char flux_smem[];
+    __shared__ __align__(8) uint64_t bar;
+    if (sc->halted) return;
+    R* sm = (R*)flux_smem;
+    const int tx = threadIdx.x % T_::T0, ty = threadIdx.x / T_::T0 % T_::T1, tz = threadIdx.x / (T_::T0 * T_::T1);
+    const int i0 = r.i0 + blockIdx.x * T_::T0, j0 = r.j0 + blockIdx.y * T_::T1, k0 = r.k0 + blockIdx.z * T_::T2;
+    if (threadIdx.x == 0) {
+        tma_bar_init(&bar);
+        tma_expect(&bar, T_::all() * sizeof(R));
+#pragma unroll
+        for (int q = 0; q < 6; q++)
+            tma_load(sm + T_::off(q), &maps.m[q], i0 - T_::org(q, 0), j0 - T_::org(q, 1), k0 - T_::org(q, 2),
+                     q == 2 ? 3 * E : (q == 0 || q == 3) ? dT1 : (q == 1 || q == 4) ? dT2 : 0, &bar);
+    }
+    const int ii = i0 + tx, jj = j0 + ty, kk = k0 + tz;
+    const bool in = ii <= r.i1 && jj <= r.j1 && kk <= r.k1;
+    const long fs = b.fs;
+    const long c = lidx(b, min(ii, r.i1), min(jj, r.j1), min(kk, r.k1));
+    const R* Te = g.Te + c;
+    EdgeMetric<R> m;
+#pragma unroll
+    for (int x = 0; x < 3; x++) {
+        m.t1[x] = Te[(3 + x + 9 * eD) * fs];
+        m.t2[x] = Te[(6 + x + 9 * eD) * fs];
+    }
+    m.xni = g.Teb[(0 + 4 * eD) * fs + c];
+    m.yni = g.Teb[(1 + 4 * eD) * fs + c];
+    m.xnj = g.Teb[(2 + 4 * eD) * fs + c];
+    m.ynj = g.Teb[(3 + 4 * eD) * fs + c];
+    m.rA1 = g.rfae[(2 * eD) * fs + c];
+#ifdef GAM_FAST_RECIP
+    m.fA1 = m.fA2 = (R)0;  // not used
+#else
+    m.fA1 = g.fae[(2 * eD) * fs + c];
+    m.fA2 = g.fae[(2 * eD + 1) * fs + c];
+#endif
+    const Quot<R> qA1(m.fA1, m.rA1), qA2(m.fA2, g.rfae[(2 * eD + 1) * fs + c]), qdt((R)sc->dt, (R)sc->rdt);
+    m.detT = g.rdet[eD * fs + c];
+    m.edge = g.edge[eD * fs + c];
+    __syncthreads();  // the barrier's initialisation
+    if (!tma_wait(&bar)) {  // never in a sound step: stop it
+        sc->status = 5;
+        sc->halted = 1;
+        return;
+    }
+    if (!in) return;
+    {
+        [[maybe_unused]] const long sA = dstride(b, dT1), sB = dstride(b, dT2), sM = sA > sB ? sA : sB;
+        [[maybe_unused]] const long lo = c - sA - sB < c - 4 * sM ? c - sA - sB : c - 4 * sM;
+        GAM_BOX_CHECK(lo, c + 3 * sM, 3 + 2 * eD);
+    }
+    edge_emf<R, E, false>(b, P, g, w, c, sm, tx, ty, tz, m, qA1, qA2, qdt);
+}
+
+#endif  // GAM_GEO_TABLES
 
 // One-sided Gaussian-moment fluxes for one side q (sgn = -1 LEFT, +1 RIGHT).
 // MagKinFlux (stress.F90:513-599).
@@ -974,38 +1118,7 @@ __device__ __forceinline__ void gas_kin_flux(const DevParams<R>& P, R sgn, const
     dW[4] = dW[4] + sgn * E;
 }
 
-// ----------------------------------------------------------------- TMA
-// Box copies of a (i, j, k, component) field into shared memory and the
-// mbarrier that counts their bytes.
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void tma_bar_init(uint64_t* bar) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void tma_expect(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void tma_load(void* dst, const CUtensorMap* map, int i, int j, int k, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
-        "[%6];" ::"r"(smem_u32(dst)), "l"(map), "r"(i), "r"(j), "r"(k), "r"(0), "r"(smem_u32(bar))
-        : "memory");
-}
-// Wait for the first phase; false when it does not complete within the limit
-// (each try waits in hardware for a while)
-__device__ __forceinline__ bool tma_wait(uint64_t* bar) {
-    for (int n = 0; n < (1 << 20); n++) {
-        uint32_t done;
-        asm volatile(
-            "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0; selp.b32 %0, 1, 0, p; }"
-            : "=r"(done)
-            : "r"(smem_u32(bar))
-            : "memory");
-        if (done) return true;
-    }
-    return false;
-}
-
+#ifdef GAM_GEO_TABLES
 // Face fluxes of direction D (Fluxes, stress.F90:204-429), one face per
 // thread. The stencil operands are the per-cell products volume*primitive and
 // volume*B of the half state (QdV of Cen8LRs) and the limiter values of 16
@@ -1036,11 +1149,11 @@ __global__ void __launch_bounds__(FluxTile<R, D>::NT, MINB)
         tma_expect(&bar, P.doMHD ? T_::BYTES : T_::BYTES_GAS);
         const int qi = D == 0 ? i0 - 4 : i0, qj = D == 1 ? j0 - 4 : j0, qk = D == 2 ? k0 - 4 : k0;
         const int lj = D == 1 ? j0 - 2 : j0, lk = D == 2 ? k0 - 2 : k0;
-        tma_load(sQ, &maps.QW, qi, qj, qk, &bar);
-        tma_load(sL, &maps.Wn, qi, lj, lk, &bar);
+        tma_load(sQ, &maps.QW, qi, qj, qk, 0, &bar);
+        tma_load(sL, &maps.Wn, qi, lj, lk, 0, &bar);
         if (P.doMHD) {
-            tma_load(sQ + 5 * T_::QN * T_::QX, &maps.QB, qi, qj, qk, &bar);
-            tma_load(sL + 5 * T_::LN * T_::QX, &maps.Bl, qi, lj, lk, &bar);
+            tma_load(sQ + 5 * T_::QN * T_::QX, &maps.QB, qi, qj, qk, 0, &bar);
+            tma_load(sL + 5 * T_::LN * T_::QX, &maps.Bl, qi, lj, lk, 0, &bar);
         }
     }
     const int ii = i0 + tx, jj = D == 2 ? j0 : j0 + tn, kk = D == 2 ? k0 + tn : k0;
@@ -1183,6 +1296,8 @@ __global__ void __launch_bounds__(FluxTile<R, D>::NT, MINB)
 #pragma unroll
     for (int v = 0; v < 5; v++) w.gF[(v + 5 * D) * fs + c] = fa * gv[v];
 }
+
+#endif  // GAM_GEO_TABLES
 
 // E2Flux into the new buffer; faces outside its range are copied. With
 // doAB3 the buffer's old content (oState, n-1) first moves to ooState
@@ -2722,10 +2837,22 @@ __global__ void __launch_bounds__(128) k_bfield_all(GamBox b, Geo<R> g, StateBuf
     for (int x = 0; x < 3; x++) s.B[x * fs + c] = B[x];
 }
 
+#ifdef GAM_GEO_TABLES  // the builds that hold the step
 // ----------------------------------------------------------------- launches
 static inline dim3 grid_for(const Range& r, dim3 blk) {
     return dim3((unsigned)((r.i1 - r.i0 + 1 + blk.x - 1) / blk.x), (unsigned)((r.j1 - r.j0 + 1 + blk.y - 1) / blk.y),
                 (unsigned)((r.k1 - r.k0 + 1 + blk.z - 1) / blk.z));
+}
+
+template <class R, int E> void launch_vxb(const Ctx<R>& C, const Range& r, cudaStream_t s) {
+    using T_ = EdgeTile<E>;
+    const dim3 gr((unsigned)((r.i1 - r.i0 + T_::T0) / T_::T0), (unsigned)((r.j1 - r.j0 + T_::T1) / T_::T1),
+                  (unsigned)((r.k1 - r.k0 + T_::T2) / T_::T2));
+    const unsigned sm = T_::all() * sizeof(R);
+    // blocks of 256 per SM: 3 in FP64 (strict 289/299/299 us for the three
+    // directions at 192^3; 2: 372/376/377, 4: 305/313/325), 5 in FP32
+    // (148/137/140; 4: 156/152/154)
+    k_vxb<R, E, sizeof(R) == 4 ? 5 : 3><<<gr, T_::NT, sm, s>>>(C.b, C.P, C.g, C.w, r, C.sc, C.fmaps->e[E]);
 }
 
 // RingAverage (ringav.F90:26-75) on the updated state: smoothing EMFs of both
@@ -2792,19 +2919,11 @@ template <class R, class F> void for_each_kernel(const Ctx<R>& C, int cur, cudaS
                              {G, G + b.Nip, G, G + b.Njp - 1, G, G + b.Nkp},
                              {G, G + b.Nip, G, G + b.Njp, G, G + b.Nkp - 1}};
         for (int eD = 0; eD < 3; eD++) {
-            // edge directions whose stencils run along k (Mom2Face of eD = 1, VxB of eD = 0, 1)
-            const dim3 mb = (eD == 1 && (C.kvar & 1024)) ? dim3(32, 1, 4) : blk;
-            const dim3 vb = (eD < 2 && (C.kvar & 512)) ? dim3(32, 1, 4) : blk;
-            f(2 + 2 * eD, [&] { k_mom2face<R><<<grid_for(mf[eD], mb), mb, 0, s>>>(b, C.P, C.g, C.w, eD, mf[eD], C.sc); });
+            f(2 + 2 * eD, [&] { k_mom2face<R><<<grid_for(mf[eD], blk), blk, 0, s>>>(b, C.P, C.g, C.w, eD, mf[eD], C.sc); });
             f(3 + 2 * eD, [&] {
-                if (C.kvar & 16)
-                    k_vxb<R, 10><<<grid_for(ed[eD], vb), vb, 0, s>>>(b, C.P, C.g, C.w, eD, ed[eD], C.sc);
-                else if ((C.kvar & 32) || sizeof(R) == 4)  // FP32: 12 blocks/SM (40 registers) measured best
-                    k_vxb<R, 12><<<grid_for(ed[eD], vb), vb, 0, s>>>(b, C.P, C.g, C.w, eD, ed[eD], C.sc);
-                else if (C.kvar & 128)
-                    k_vxb<R><<<grid_for(ed[eD], vb), vb, 0, s>>>(b, C.P, C.g, C.w, eD, ed[eD], C.sc);
-                else  // FP64: 8 blocks/SM (64 registers)
-                    k_vxb<R, 8><<<grid_for(ed[eD], vb), vb, 0, s>>>(b, C.P, C.g, C.w, eD, ed[eD], C.sc);
+                if (eD == 0) launch_vxb<R, 0>(C, ed[0], s);
+                else if (eD == 1) launch_vxb<R, 1>(C, ed[1], s);
+                else launch_vxb<R, 2>(C, ed[2], s);
             });
         }
     }
@@ -3119,5 +3238,7 @@ template <class R> void launch_halo(const Ctx<R>& C, int cur, cudaStream_t s, in
         k_halo_bxyz<R><<<(unsigned)((m + 255) / 256), 256, 0, s>>>(b, C.g, S, d, side, C.sc, C.P.ring);
     }
 }
+
+#endif  // GAM_GEO_TABLES
 
 }  // namespace GAM_NS

@@ -98,6 +98,11 @@ template <class R> struct Geo {  // Grid_T arrays on the device (gamtypes.F90:16
     // forms that multiply by the reciprocal keep only that one.
     const R* vif;    // face, 3
     const R* rvif;   // face, 3
+    // the same of the areas at the edges (dT1 faces along dT2, then dT2 faces
+    // along dT1, per edge direction), and 1/(determinant of the edge's B map)
+    const R* fae;    // edge, 6: q + 2*eD
+    const R* rfae;   // edge, 6
+    const R* rdet;   // edge, 3
     const double* fcB0;    // face, 9  (background; FP64 in both forms)
     const double* bFlux0;  // face, 3
     const double* edgB0;   // edge, 6: c + 2*d
@@ -163,8 +168,47 @@ template <class R, int D> struct FluxTile {
 struct GamFluxMaps {
     CUtensorMap QW, QB, Wn, Bl;
 };
+// The tile of one block of the edge-EMF kernel of direction E (dT1 = E+1, dT2 =
+// E+2) and its boxes in shared memory, one after the other: 0, 1 the EdgeLRs
+// operands of dT1 faces along dT2 and of dT2 faces along dT1 (cells -4..3), 2
+// the three components of GetCornerV's operand (along dT2), 3, 4 the limiter
+// values of 0, 1 (-2..1), 5 the density (-1..0 along both). A box that extends
+// along i starts 4 below the tile (16-byte boundary, see FluxTile).
+template <int E> struct EdgeTile {
+    static constexpr int d1 = (E + 1) % 3, d2 = (E + 2) % 3;
+    static constexpr int T0 = E == 0 ? 16 : 32, T1 = E == 0 ? 4 : (E == 1 ? 1 : 8), T2 = E == 0 ? 4 : (E == 1 ? 8 : 1);
+    static constexpr int NT = T0 * T1 * T2;
+    __host__ __device__ static constexpr int T(int d) { return d == 0 ? T0 : d == 1 ? T1 : T2; }
+    __host__ __device__ static constexpr bool along(int q, int d) {
+        return (q == 0 || q == 2 || q == 3) ? d == d2 : (q == 1 || q == 4) ? d == d1 : d != E;
+    }
+    __host__ __device__ static constexpr int org(int q, int d) {
+        return !along(q, d) ? 0 : d == 0 ? 4 : q < 3 ? 4 : q < 5 ? 2 : 1;
+    }
+    __host__ __device__ static constexpr int ext(int q, int d) {
+        return T(d) + (!along(q, d) ? 0 : d == 0 ? 8 : q < 3 ? 7 : q < 5 ? 3 : 1);
+    }
+    __host__ __device__ static constexpr int size(int q) { return ext(q, 0) * ext(q, 1) * ext(q, 2); }
+    __host__ __device__ static constexpr int off(int q) {
+        int o = 0;
+        for (int p = 0; p < q; p++) o += size(p) * (p == 2 ? 3 : 1);
+        return o;
+    }
+    __host__ __device__ static constexpr int str(int q, int d) {
+        return d == 0 ? 1 : d == 1 ? ext(q, 0) : ext(q, 0) * ext(q, 1);
+    }
+    // position of the tile's point (x, y, z) in box q
+    __host__ __device__ static constexpr int at(int q, int x, int y, int z) {
+        return off(q) + ((z + org(q, 2)) * ext(q, 1) + y + org(q, 1)) * ext(q, 0) + x + org(q, 0);
+    }
+    __host__ __device__ static constexpr int all() { return off(6); }
+};
+struct GamEdgeMaps {
+    CUtensorMap m[6];
+};
 struct GamFluxMapSet {
     GamFluxMaps m[2][3];  // [State buffer][direction]
+    GamEdgeMaps e[3];     // [edge direction]
 };
 
 // Everything one step launch needs.
@@ -178,9 +222,9 @@ template <class R> struct Ctx {
     GamScalars* sc;
     const GamFluxMapSet* fmaps;  // host memory, with the handle
     double gamma, gm1;
-    int kvar;  // launch-configuration variant for tuning runs (GAM_KVAR); 0 = the tuned default
     // side streams and fork/join events of the step graph (independent
     // kernels of a step run as parallel branches); null: one stream
+    int kvar;  // launch-configuration variant for tuning runs (GAM_KVAR); 0 = the tuned default
     cudaStream_t aux[5];
     cudaEvent_t ev[8];
 };
