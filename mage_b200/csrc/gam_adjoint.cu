@@ -419,95 +419,80 @@ __global__ void __launch_bounds__(256) k_stress_adj_gather3(GamBox b, Range r0, 
 }
 
 
-// Face fluxes of direction D (Fluxes, stress.F90:204-429), one face per
-// thread. The stencil operands are the per-cell products volume*primitive and
-// volume*B of the half state (QdV of Cen8LRs) and the limiter values, read
-// along D through L1 (the callers' unpadded boxes have rows that a TMA copy
-// cannot start on). SAVE (the whole step's forward) also stores the face
-// states in w.fsv.
-template <class R, int D, int MINB, bool SAVE = false>
-__global__ void __launch_bounds__(128, MINB) k_stress_box(GamBox b, DevParams<R> P, Geo<R> g, const R* __restrict__ Blim,
-                                                      Work<R> w, Range r, const GamScalars* sc) {
+// Asynchronous copies of single values into shared memory: rows of the callers'
+// unpadded boxes start anywhere, which a TMA copy cannot
+__device__ __forceinline__ void cp_async(double* dst, const double* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async(float* dst, const float* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+// Face fluxes of direction D (Fluxes, stress.F90:204-429) on the callers'
+// arrays, one face per thread; the stencil boxes come into shared memory by
+// asynchronous copies of all threads (see k_stress).
+template <class R, int D, int MINB>
+__global__ void __launch_bounds__(FluxTile<R, D>::NT, MINB)
+    k_stress_box(GamBox b, DevParams<R> P, Geo<R> g, const R* __restrict__ Blim, Work<R> w, Range r, const GamScalars* sc) {
+    using T_ = FluxTile<R, D>;
+    extern __shared__ __align__(128) unsigned char flux_smem[];
     if (sc->halted) return;
-    int ii, jj, kk;
-    if (!thread_ijk(r, ii, jj, kk)) return;
+    R* sQ = (R*)flux_smem;
+    R* sL = (R*)(flux_smem + T_::LOFF);
+    const int tx = threadIdx.x % T_::TX, tn = threadIdx.x / T_::TX;
+    const int i0 = r.i0 + blockIdx.x * T_::TX;
+    const int j0 = r.j0 + blockIdx.y * (D == 2 ? 1 : T_::TN);
+    const int k0 = r.k0 + blockIdx.z * (D == 2 ? T_::TN : 1);
     const long fs = b.fs;
-    const long c = lidx(b, ii, jj, kk);
-    const long s = D == 0 ? 1L : (D == 1 ? (long)b.sx : b.sk);
-    GAM_BOX_CHECK(c - 4 * s, c + 3 * s, 8 + D);
+    const long s = D == 0 ? 1L : (D == 1 ? (long)b.sx : b.sk), sn = D == 2 ? b.sk : (long)b.sx;
+    const int nvar = P.doMHD ? 8 : 5;
+    {
+        // box position (x, n) of field v, n along j or k; a position past the box
+        // (of a tile past the range) takes its last value
+        const long q0 = lidx(b, i0, j0, k0) - 4 * s, l0 = lidx(b, i0, j0, k0) - (D == 0 ? 4 : 2) * s;
+        for (int x = tx; x < T_::QX; x += T_::TX)
+            for (int n = tn; n < T_::QN; n += T_::TN) {
+                const long cq = min(q0 + x + n * sn, b.nbox - 1), cl = min(l0 + x + n * sn, b.nbox - 1);
+#pragma unroll
+                for (int v = 0; v < 8; v++) {
+                    if (v >= nvar) break;
+                    cp_async(sQ + (v * T_::QN + n) * T_::QX + x, (v < 5 ? w.QW + v * fs : w.QB + (v - 5) * fs) + cq);
+                    if (n < T_::LN)
+                        cp_async(sL + (v * T_::LN + n) * T_::QX + x, (v < 5 ? w.Wn + v * fs : Blim + (v - 5) * fs) + cl);
+                }
+            }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    const int ii = i0 + tx, jj = D == 2 ? j0 : j0 + tn, kk = D == 2 ? k0 + tn : k0;
+    const bool in = ii <= r.i1 && jj <= r.j1 && kk <= r.k1;
+    const long c = lidx(b, min(ii, r.i1), min(jj, r.j1), min(kk, r.k1));
     R T[9];
 #pragma unroll
     for (int n = 0; n < 9; n++) T[n] = g.Tf[(n + 9 * D) * fs + c];
     const R fa = g.face[D * fs + c];
-    R vol[8];
-#pragma unroll
-    for (int n = 0; n < 8; n++) vol[n] = g.vol[c + (n - 4) * s];
-    const Quot<R> Vi(central8(vol));
-    R MagL[3] = {(R)0, (R)0, (R)0}, MagR[3] = {(R)0, (R)0, (R)0};
+    const Quot<R> Vi = face_quot<R>(b, g, c, D);
     R Bn = (R)0;
     double B0[3] = {0.0, 0.0, 0.0}, B0n = 0.0;
     if (P.doMHD) {
         Bn = w.Bnf[D * fs + c];
-#pragma unroll
-        for (int x = 0; x < 3; x++) {
-            R q[8], nq[4];
-            const R* qp = w.QB + x * fs + c - 4 * s;
-            const R* lp = Blim + x * fs + c - 2 * s;
-#pragma unroll
-            for (int n = 0; n < 8; n++) q[n] = qp[n * s];
-#pragma unroll
-            for (int m = 0; m < 4; m++) nq[m] = lp[m * s];
-            lrs_from_qdv(P, q, nq, Vi, MagL[x], MagR[x]);
-        }
         if (P.doBackground) {
 #pragma unroll
             for (int x = 0; x < 3; x++) B0[x] = g.fcB0[(x + 3 * D) * fs + c];
             B0n = qdiv(g.bFlux0[D * fs + c], (double)fa);
         }
     }
-    R WL[5], WR[5];
-#pragma unroll
-    for (int v = 0; v < 5; v++) {
-        R q[8], nq[4];
-        const R* qp = w.QW + v * fs + c - 4 * s;
-        const R* lp = w.Wn + v * fs + c - 2 * s;
-#pragma unroll
-        for (int n = 0; n < 8; n++) q[n] = qp[n * s];
-#pragma unroll
-        for (int m = 0; m < 4; m++) nq[m] = lp[m * s];
-        lrs_from_qdv(P, q, nq, Vi, WL[v], WR[v]);
-    }
-    R VaD = (R)0, bbD = (R)0;
-    if (P.doMHD) {
-        R mF[3] = {(R)0, (R)0, (R)0};
-        mag_kin_flux<R>(P, (R)-1, WL, MagL, Bn, T, B0, B0n, mF, bbD, VaD);
-        mag_kin_flux<R>(P, (R)1, WR, MagR, Bn, T, B0, B0n, mF, bbD, VaD);
-#pragma unroll
-        for (int x = 0; x < 3; x++) w.mF[(x + 3 * D) * fs + c] = fa * mF[x];
-    }
-    R gF[5] = {(R)0, (R)0, (R)0, (R)0, (R)0}, dW[5] = {(R)0, (R)0, (R)0, (R)0, (R)0};
-    gas_kin_flux(P, (R)-1, WL, T, gF, dW);
-    gas_kin_flux(P, (R)1, WR, T, gF, dW);
-    R gv[5];
-#pragma unroll
-    for (int v = 0; v < 5; v++) gv[v] = gF[v] - (R)1 * P.cHogH * VaD * dW[v];
-#pragma unroll
-    for (int v = 0; v < 5; v++) w.gF[(v + 5 * D) * fs + c] = fa * gv[v];
-    if constexpr (SAVE) {
-        R* o = w.fsv + (long)(GAM_FSV_NC * D) * fs + c;
-#pragma unroll
-        for (int v = 0; v < 5; v++) {
-            o[v * fs] = WL[v];
-            o[(5 + v) * fs] = WR[v];
-            o[(17 + v) * fs] = dW[v];
-        }
-#pragma unroll
-        for (int x = 0; x < 3; x++) {
-            o[(10 + x) * fs] = MagL[x];
-            o[(13 + x) * fs] = MagR[x];
-        }
-        o[16 * fs] = VaD;
-    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    if (!in) return;
+    flux_face<R, D, false, true>(b, P, w, sc, nullptr, nullptr, c, sQ, sL, tx, tn, Vi, T, fa, Bn, B0, B0n);
+}
+template <class R, int D>
+void launch_stress_box(const GamBox& b, const DevParams<R>& P, const Geo<R>& g, const R* Bl, const Work<R>& w,
+                       const Range& r, const GamScalars* sc, cudaStream_t s) {
+    using T_ = FluxTile<R, D>;
+    const dim3 sg((unsigned)((r.i1 - r.i0 + T_::TX) / T_::TX),
+                  (unsigned)(D == 2 ? r.j1 - r.j0 + 1 : (r.j1 - r.j0 + T_::TN) / T_::TN),
+                  (unsigned)(D == 2 ? (r.k1 - r.k0 + T_::TN) / T_::TN : r.k1 - r.k0 + 1));
+    k_stress_box<R, D, sizeof(R) == 8 ? 4 : (D == 0 ? 7 : 4)><<<sg, T_::NT, T_::SMEM, s>>>(b, P, g, Bl, w, r, sc);
 }
 
 // EdgeLRs (fields.F90:288-362): flux of faces of direction a, stencil along b
@@ -534,82 +519,74 @@ __device__ __forceinline__ void edge_lrs(const GamBox& b, const DevParams<R>& P,
     bR = bR * fA;
 }
 
-// VxB edge loop for direction eD (fields.F90:184-228). SAVE (the
-// differentiation form's forward) also stores the corner values in w.esv.
-template <class R, int MINB = 1, bool SAVE = false>
-__global__ void __launch_bounds__(128, MINB) k_vxb_box(GamBox b, DevParams<R> P, Geo<R> g, Work<R> w, int eD, Range r,
-                                             const GamScalars* sc) {
+// the area interpolated to edge c from the faces of direction a along b
+template <class R> __device__ __forceinline__ R edge_area(const GamBox& b, const Geo<R>& g, long c, int a, int bd) {
+    const long s = dstride(b, bd);
+    R area[8];
+#pragma unroll
+    for (int n = 0; n < 8; n++) area[n] = g.face[a * b.fs + c + (n - 4) * s];
+    return central8(area);
+}
+// VxB edge loop for direction E (fields.F90:184-228) on the callers' arrays, one
+// edge per thread; the stencil boxes come into shared memory by asynchronous
+// copies of all threads (see k_vxb).
+template <class R, int E, int MINB>
+__global__ void __launch_bounds__(EdgeTile<E>::NT, MINB)
+    k_vxb_box(GamBox b, DevParams<R> P, Geo<R> g, Work<R> w, Range r, const GamScalars* sc) {
+    using T_ = EdgeTile<E>;
+    constexpr int dT1 = T_::d1, dT2 = T_::d2;
+    extern __shared__ __align__(128) unsigned char flux_smem[];
     if (sc->halted) return;
-    int ii, jj, kk;
-    if (!thread_ijk(r, ii, jj, kk)) return;
-    int dT1, dT2;
-    edge_dirs(eD, dT1, dT2);
+    R* sm = (R*)flux_smem;
+    const int tid = threadIdx.x, tx = tid % T_::T0, ty = tid / T_::T0 % T_::T1, tz = tid / (T_::T0 * T_::T1);
+    const int i0 = r.i0 + blockIdx.x * T_::T0, j0 = r.j0 + blockIdx.y * T_::T1, k0 = r.k0 + blockIdx.z * T_::T2;
     const long fs = b.fs;
-    const long c = lidx(b, ii, jj, kk);
-    // GetCornerD (fields.F90:427-454): normal-plane unit offsets e1 < e2
-    const int e1 = eD == 0 ? 1 : 0, e2 = eD == 2 ? 1 : 2;
-    const long s1 = dstride(b, e1), s2 = dstride(b, e2);
-    {
-        const long sA = dstride(b, dT1), sB = dstride(b, dT2), sM = sA > sB ? sA : sB;
-        [[maybe_unused]] const long lo = c - s1 - s2 < c - 4 * sM ? c - s1 - s2 : c - 4 * sM;
-        GAM_BOX_CHECK(lo, c + 3 * sM, 3 + 2 * eD);
+#pragma unroll
+    for (int q = 0; q < 6; q++) {
+        const R* f = q < 2 ? w.abh + (q == 0 ? dT1 : dT2) * fs
+                           : q == 2 ? w.AVf + 3 * E * fs : q < 5 ? w.bn + (q == 3 ? dT1 : dT2) * fs : w.Dh;
+        const long c0 = lidx(b, i0 - T_::org(q, 0), j0 - T_::org(q, 1), k0 - T_::org(q, 2));
+        for (int e = tid; e < T_::size(q); e += T_::NT) {
+            const int x = e % T_::ext(q, 0), y = e / T_::ext(q, 0) % T_::ext(q, 1), z = e / (T_::ext(q, 0) * T_::ext(q, 1));
+            const long cq = min(c0 + x + (long)y * b.sx + z * b.sk, b.nbox - 1);
+#pragma unroll
+            for (int v = 0; v < (q == 2 ? 3 : 1); v++) cp_async(sm + T_::off(q) + v * T_::size(q) + e, f + v * fs + cq);
+        }
     }
-    R Dc = (R)0.25 * (w.Dh[c] + w.Dh[c - s1] + w.Dh[c - s2] + w.Dh[c - s1 - s2]);
-    // GetCornerB: EdgeLRs for dT1 faces along dT2 and dT2 faces along dT1
-    R area1[8], area2[8];
-    R bT1L, bT1R, fA1, bT2L, bT2R, fA2;
-    edge_lrs(b, P, g, w, c, dT1, dT2, area1, bT1L, bT1R, fA1);
-    edge_lrs(b, P, g, w, c, dT2, dT1, area2, bT2L, bT2R, fA2);
-    // GetCornerV (fields.F90:457-517); its area stencil equals area1
-    R dA = rmax(fA1, (R)TINY);
-    const Quot<R> qdA(dA);
-    R VC[3];
-    const long s2v = dstride(b, dT2);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const int ii = i0 + tx, jj = j0 + ty, kk = k0 + tz;
+    const bool in = ii <= r.i1 && jj <= r.j1 && kk <= r.k1;
+    const long c = lidx(b, min(ii, r.i1), min(jj, r.j1), min(kk, r.k1));
+    EdgeMetric<R> m;
+    const R* Te = g.Te + c;
 #pragma unroll
     for (int x = 0; x < 3; x++) {
-        R acc = (R)0;
-#pragma unroll
-        for (int n = 0; n < 8; n++) acc += Rc<R>(w8(n)) * w.AVf[(x + 3 * eD) * fs + c + (n - 4) * s2v];
-        VC[x] = qdA(acc);
+        m.t1[x] = Te[(3 + x + 9 * E) * fs];
+        m.t2[x] = Te[(6 + x + 9 * E) * fs];
     }
-    const R* Te = g.Te;
-    R v1 = VC[0] * Te[(3 + 9 * eD) * fs + c] + VC[1] * Te[(4 + 9 * eD) * fs + c] + VC[2] * Te[(5 + 9 * eD) * fs + c];
-    R v2 = VC[0] * Te[(6 + 9 * eD) * fs + c] + VC[1] * Te[(7 + 9 * eD) * fs + c] + VC[2] * Te[(8 + 9 * eD) * fs + c];
-    R vDiff = Mth<R>::sqrt_(v1 * v1 + v2 * v2);
-    R xni = g.Teb[(0 + 4 * eD) * fs + c], yni = g.Teb[(1 + 4 * eD) * fs + c];
-    R xnj = g.Teb[(2 + 4 * eD) * fs + c], ynj = g.Teb[(3 + 4 * eD) * fs + c];
-    R detT = (R)1 / (xni * ynj - xnj * yni);
-    const Quot<R> qA1(fA1), qA2(fA2);
-    R bT1 = qA1((R)0.5 * (bT1L + bT1R));
-    R bT2 = qA2((R)0.5 * (bT2L + bT2R));
-    R db1 = qA1(bT1R - bT1L);
-    R db2 = qA2(bT2R - bT2L);
-    R Jd = db2 - db1;
-    R b1 = detT * (ynj * bT1 - yni * bT2);
-    R b2 = detT * (-(xnj * bT1) + xni * bT2);
-    if (P.doBackground) {
-        b1 = b1 + (R)g.edgB0[(0 + 2 * eD) * fs + c];
-        b2 = b2 + (R)g.edgB0[(1 + 2 * eD) * fs + c];
-    }
-    R vA = qdiv(Mth<R>::sqrt_(b1 * b1 + b2 * b2), Mth<R>::sqrt_(Dc));
-    if (P.doBoris) vA = boris_speed((R)P.Ca, vA);
-    vDiff = vDiff + vA;
-    const R edge = g.edge[eD * fs + c];
-    vDiff = rmin(vDiff, P.CFL * edge / (R)sc->dt);
-    R e = -(v1 * b2 - v2 * b1) + P.Vd0 * vDiff * Jd;
-    w.E[eD * fs + c] = e * edge;
-    if constexpr (SAVE) {
-        R* o = w.esv + (long)(GAM_ESV_NC * eD) * fs + c;
-        o[0] = Dc;
-        o[fs] = bT1L;
-        o[2 * fs] = bT1R;
-        o[3 * fs] = fA1;
-        o[4 * fs] = bT2L;
-        o[5 * fs] = bT2R;
-        o[6 * fs] = fA2;
-#pragma unroll
-        for (int x = 0; x < 3; x++) o[(7 + x) * fs] = VC[x];
-    }
+    m.xni = g.Teb[(0 + 4 * E) * fs + c];
+    m.yni = g.Teb[(1 + 4 * E) * fs + c];
+    m.xnj = g.Teb[(2 + 4 * E) * fs + c];
+    m.ynj = g.Teb[(3 + 4 * E) * fs + c];
+    m.edge = g.edge[E * fs + c];
+    m.fA1 = edge_area(b, g, c, dT1, dT2);
+    m.fA2 = edge_area(b, g, c, dT2, dT1);
+    m.detT = (R)1 / (m.xni * m.ynj - m.xnj * m.yni);
+    const Quot<R> qA1(m.fA1), qA2(m.fA2), qdt((R)sc->dt);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    if (!in) return;
+    edge_emf<R, E, true>(b, P, g, w, c, sm, tx, ty, tz, m, qA1, qA2, qdt);
+}
+template <class R, int E>
+void launch_vxb_box(const GamBox& b, const DevParams<R>& P, const Geo<R>& g, const Work<R>& w, const Range& r,
+                    const GamScalars* sc, cudaStream_t s) {
+    using T_ = EdgeTile<E>;
+    const dim3 gr((unsigned)((r.i1 - r.i0 + T_::T0) / T_::T0), (unsigned)((r.j1 - r.j0 + T_::T1) / T_::T1),
+                  (unsigned)((r.k1 - r.k0 + T_::T2) / T_::T2));
+    const unsigned sm = T_::all() * sizeof(R);
+    constexpr int MB = sizeof(R) == 8 ? 2 : 4;
+    k_vxb_box<R, E, MB><<<gr, T_::NT, sm, s>>>(b, P, g, w, r, sc);
 }
 
 // reverse of edge_lrs (EdgeLRs for faces of direction a along bd): adjoints of
@@ -1657,14 +1634,10 @@ int flux_call(const gam_params* p, const void* QW, const void* Wn, const void* Q
                     (unsigned)((r.k1 - r.k0 + 1 + blk.z - 1) / blk.z));
     };
     const R* Bl = (const R*)Blim;
-    if (!dgF && fstates) {
-        k_stress_box<R, 0, 1, true><<<grid(fr[0]), blk, 0, s>>>(b, P, g, Bl, w, fr[0], sc);
-        k_stress_box<R, 1, 1, true><<<grid(fr[1]), blk, 0, s>>>(b, P, g, Bl, w, fr[1], sc);
-        k_stress_box<R, 2, 1, true><<<grid(fr[2]), blk, 0, s>>>(b, P, g, Bl, w, fr[2], sc);
-    } else if (!dgF) {
-        k_stress_box<R, 0, 1><<<grid(fr[0]), blk, 0, s>>>(b, P, g, Bl, w, fr[0], sc);
-        k_stress_box<R, 1, 1><<<grid(fr[1]), blk, 0, s>>>(b, P, g, Bl, w, fr[1], sc);
-        k_stress_box<R, 2, 1><<<grid(fr[2]), blk, 0, s>>>(b, P, g, Bl, w, fr[2], sc);
+    if (!dgF) {
+        launch_stress_box<R, 0>(b, P, g, Bl, w, fr[0], sc, s);
+        launch_stress_box<R, 1>(b, P, g, Bl, w, fr[1], sc, s);
+        launch_stress_box<R, 2>(b, P, g, Bl, w, fr[2], sc, s);
     } else if (fstates) {
         R* rs = (R*)rscratch;
         const long fs40 = 40L * b.fs;
@@ -1787,10 +1760,10 @@ int efield_call(const gam_params* p, const void* Dh, const void* abh, const void
     for (int eD = 0; eD < 3; eD++) {
         // the adjoint of a whole step finds AVf as its forward left it
         if (!(dE && avf_saved)) k_mom2face<R><<<grid(mf[eD]), blk, 0, s>>>(b, P, g, w, eD, mf[eD], sc);
-        if (!dE && estates) {
-            k_vxb_box<R, 1, true><<<grid(ed[eD]), blk, 0, s>>>(b, P, g, w, eD, ed[eD], sc);
-        } else if (!dE) {
-            k_vxb_box<R><<<grid(ed[eD]), blk, 0, s>>>(b, P, g, w, eD, ed[eD], sc);
+        if (!dE) {
+            if (eD == 0) launch_vxb_box<R, 0>(b, P, g, w, ed[0], sc, s);
+            else if (eD == 1) launch_vxb_box<R, 1>(b, P, g, w, ed[1], sc, s);
+            else launch_vxb_box<R, 2>(b, P, g, w, ed[2], sc, s);
         } else if (escratch) {
             // deterministic: the edges store their adjoints (14 components
             // from escratch + 14 eD fs), gathered per position after the third

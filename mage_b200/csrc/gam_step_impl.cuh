@@ -1118,80 +1118,25 @@ __device__ __forceinline__ void gas_kin_flux(const DevParams<R>& P, R sgn, const
     dW[4] = dW[4] + sgn * E;
 }
 
-#ifdef GAM_GEO_TABLES
-// Face fluxes of direction D (Fluxes, stress.F90:204-429), one face per
-// thread. The stencil operands are the per-cell products volume*primitive and
-// volume*B of the half state (QdV of Cen8LRs) and the limiter values of 16
-// fields. One thread has the block's tile of all of them copied to shared
-// memory by TMA (four box copies, one mbarrier); the metric's loads are issued
-// meanwhile. What bounds the kernel is the FP64 pipe's issue and the latency of
-// the formulas' chains: with plain loads through L1 (about half of them
-// missing) every variable exposed a memory latency, a third of all stalls.
-// 192^3, I/J/K sweeps, plain loads -> tiles: strict 934/920/957 -> 816/739/808
-// us, FMA form 746/751/811 -> 598/560/563, FP32 386/415/424 -> 295/263/264.
-// MINB bounds the registers for occupancy.
-template <class R, int D, int MINB, bool BORIS = false>
-__global__ void __launch_bounds__(FluxTile<R, D>::NT, MINB)
-    k_stress(GamBox b, DevParams<R> P, Geo<R> g, Work<R> w, Range r, GamScalars* sc, const R* __restrict__ gasN,
-             const R* __restrict__ gasO, const __grid_constant__ GamFluxMaps maps) {
+// The fluxes of face c (Fluxes, stress.F90:204-429) from its block's stencil
+// boxes in shared memory (FluxTile) and its metric. SAVE (the differentiation
+// form): also the face states into w.fsv, where that is not null (a run-time
+// choice, so that both ways are one code with one rounding).
+template <class R, int D, bool BORIS, bool SAVE>
+__device__ __forceinline__ void flux_face(const GamBox& b, const DevParams<R>& P, const Work<R>& w, const GamScalars* sc,
+                                          const R* __restrict__ gasN, const R* __restrict__ gasO, long c, const R* sQ,
+                                          const R* sL, int tx, int tn, const Quot<R>& Vi, const R* T, R fa, R Bn,
+                                          const double* B0, double B0n) {
     using T_ = FluxTile<R, D>;
-    extern __shared__ __align__(128) unsigned char flux_smem[];
-    __shared__ __align__(8) uint64_t bar;
-    if (sc->halted) return;
-    R* sQ = (R*)flux_smem;                // [8][QN][QX]: QW (5), QB (3)
-    R* sL = (R*)(flux_smem + T_::LOFF);   // [8][LN][QX]: Wn (5), limiter B (3)
-    const int tx = threadIdx.x % T_::TX, tn = threadIdx.x / T_::TX;
-    const int i0 = r.i0 + blockIdx.x * T_::TX;
-    const int j0 = r.j0 + blockIdx.y * (D == 2 ? 1 : T_::TN);
-    const int k0 = r.k0 + blockIdx.z * (D == 2 ? T_::TN : 1);
-    if (threadIdx.x == 0) {
-        tma_bar_init(&bar);
-        tma_expect(&bar, P.doMHD ? T_::BYTES : T_::BYTES_GAS);
-        const int qi = D == 0 ? i0 - 4 : i0, qj = D == 1 ? j0 - 4 : j0, qk = D == 2 ? k0 - 4 : k0;
-        const int lj = D == 1 ? j0 - 2 : j0, lk = D == 2 ? k0 - 2 : k0;
-        tma_load(sQ, &maps.QW, qi, qj, qk, 0, &bar);
-        tma_load(sL, &maps.Wn, qi, lj, lk, 0, &bar);
-        if (P.doMHD) {
-            tma_load(sQ + 5 * T_::QN * T_::QX, &maps.QB, qi, qj, qk, 0, &bar);
-            tma_load(sL + 5 * T_::LN * T_::QX, &maps.Bl, qi, lj, lk, 0, &bar);
-        }
-    }
-    const int ii = i0 + tx, jj = D == 2 ? j0 : j0 + tn, kk = D == 2 ? k0 + tn : k0;
     const long fs = b.fs;
-    const long s = D == 0 ? 1L : (D == 1 ? (long)b.sx : b.sk);
-    // threads past the range take the range's last face (and store nothing)
-    const bool in = ii <= r.i1 && jj <= r.j1 && kk <= r.k1;
-    const long c = lidx(b, min(ii, r.i1), min(jj, r.j1), min(kk, r.k1));
-    R T[9];
-#pragma unroll
-    for (int n = 0; n < 9; n++) T[n] = g.Tf[(n + 9 * D) * fs + c];
-    const R fa = g.face[D * fs + c];
-    const Quot<R> Vi = face_quot<R>(b, g, c, D);
+    [[maybe_unused]] const long s = D == 0 ? 1L : (D == 1 ? (long)b.sx : b.sk);
     R MagL[3] = {(R)0, (R)0, (R)0}, MagR[3] = {(R)0, (R)0, (R)0};
-    R Bn = (R)0;
-    double B0[3] = {0.0, 0.0, 0.0}, B0n = 0.0;
-    if (P.doMHD) {
-        Bn = w.Bnf[D * fs + c];
-        if (P.doBackground) {
-#pragma unroll
-            for (int x = 0; x < 3; x++) B0[x] = g.fcB0[(x + 3 * D) * fs + c];
-            B0n = qdiv(g.bFlux0[D * fs + c], (double)fa);
-        }
-    }
-    __syncthreads();  // the barrier's initialisation
-    if (!tma_wait(&bar)) {  // never in a sound step: stop it
-        sc->status = 5;
-        sc->halted = 1;
-        return;
-    }
-    if (!in) return;
-    GAM_BOX_CHECK(c - 4 * s, c + 3 * s, 8 + D);
     R WL[5], WR[5];
     // reconstruction, GRP variables at a time: their interpolants, one range
     // check for the quotients, the limiter
     constexpr int GRP = 4;
-    const R* pQ = sQ + (D == 0 ? tn * T_::QX + tx : tn * T_::TX + tx);
-    const R* pL = sL + (D == 0 ? tn * T_::QX + tx + 2 : tn * T_::TX + tx);
+    const R* pQ = sQ + tn * T_::QX + tx;
+    const R* pL = sL + tn * T_::QX + tx + (D == 0 ? 2 : 0);
     constexpr int st = D == 0 ? 1 : T_::TX;
     const int nvar = P.doMHD ? 8 : 5;
 #pragma unroll
@@ -1295,8 +1240,90 @@ __global__ void __launch_bounds__(FluxTile<R, D>::NT, MINB)
     }
 #pragma unroll
     for (int v = 0; v < 5; v++) w.gF[(v + 5 * D) * fs + c] = fa * gv[v];
+    if (SAVE && w.fsv) {
+        R* o = w.fsv + (long)(GAM_FSV_NC * D) * fs + c;
+#pragma unroll
+        for (int v = 0; v < 5; v++) {
+            o[v * fs] = WL[v];
+            o[(5 + v) * fs] = WR[v];
+            o[(17 + v) * fs] = dW[v];
+        }
+#pragma unroll
+        for (int x = 0; x < 3; x++) {
+            o[(10 + x) * fs] = MagL[x];
+            o[(13 + x) * fs] = MagR[x];
+        }
+        o[16 * fs] = VaD;
+    }
 }
 
+#ifdef GAM_GEO_TABLES
+// Face fluxes of direction D (Fluxes, stress.F90:204-429), one face per
+// thread. The stencil operands are the per-cell products volume*primitive and
+// volume*B of the half state (QdV of Cen8LRs) and the limiter values of 16
+// fields. One thread has the block's tile of all of them copied to shared
+// memory by TMA (four box copies, one mbarrier); the metric's loads are issued
+// meanwhile. What bounds the kernel is the FP64 pipe's issue and the latency of
+// the formulas' chains: with plain loads through L1 (about half of them
+// missing) every variable exposed a memory latency, a third of all stalls.
+// MINB bounds the registers for occupancy.
+template <class R, int D, int MINB, bool BORIS = false>
+__global__ void __launch_bounds__(FluxTile<R, D>::NT, MINB)
+    k_stress(GamBox b, DevParams<R> P, Geo<R> g, Work<R> w, Range r, GamScalars* sc, const R* __restrict__ gasN,
+             const R* __restrict__ gasO, const __grid_constant__ GamFluxMaps maps) {
+    using T_ = FluxTile<R, D>;
+    extern __shared__ __align__(128) unsigned char flux_smem[];
+    __shared__ __align__(8) uint64_t bar;
+    if (sc->halted) return;
+    R* sQ = (R*)flux_smem;                // [8][QN][QX]: QW (5), QB (3)
+    R* sL = (R*)(flux_smem + T_::LOFF);   // [8][LN][QX]: Wn (5), limiter B (3)
+    const int tx = threadIdx.x % T_::TX, tn = threadIdx.x / T_::TX;
+    const int i0 = r.i0 + blockIdx.x * T_::TX;
+    const int j0 = r.j0 + blockIdx.y * (D == 2 ? 1 : T_::TN);
+    const int k0 = r.k0 + blockIdx.z * (D == 2 ? T_::TN : 1);
+    if (threadIdx.x == 0) {
+        tma_bar_init(&bar);
+        tma_expect(&bar, P.doMHD ? T_::BYTES : T_::BYTES_GAS);
+        const int qi = D == 0 ? i0 - 4 : i0, qj = D == 1 ? j0 - 4 : j0, qk = D == 2 ? k0 - 4 : k0;
+        const int lj = D == 1 ? j0 - 2 : j0, lk = D == 2 ? k0 - 2 : k0;
+        tma_load(sQ, &maps.QW, qi, qj, qk, 0, &bar);
+        tma_load(sL, &maps.Wn, qi, lj, lk, 0, &bar);
+        if (P.doMHD) {
+            tma_load(sQ + 5 * T_::QN * T_::QX, &maps.QB, qi, qj, qk, 0, &bar);
+            tma_load(sL + 5 * T_::LN * T_::QX, &maps.Bl, qi, lj, lk, 0, &bar);
+        }
+    }
+    const int ii = i0 + tx, jj = D == 2 ? j0 : j0 + tn, kk = D == 2 ? k0 + tn : k0;
+    const long fs = b.fs;
+    const long s = D == 0 ? 1L : (D == 1 ? (long)b.sx : b.sk);
+    // threads past the range take the range's last face (and store nothing)
+    const bool in = ii <= r.i1 && jj <= r.j1 && kk <= r.k1;
+    const long c = lidx(b, min(ii, r.i1), min(jj, r.j1), min(kk, r.k1));
+    R T[9];
+#pragma unroll
+    for (int n = 0; n < 9; n++) T[n] = g.Tf[(n + 9 * D) * fs + c];
+    const R fa = g.face[D * fs + c];
+    const Quot<R> Vi = face_quot<R>(b, g, c, D);
+    R Bn = (R)0;
+    double B0[3] = {0.0, 0.0, 0.0}, B0n = 0.0;
+    if (P.doMHD) {
+        Bn = w.Bnf[D * fs + c];
+        if (P.doBackground) {
+#pragma unroll
+            for (int x = 0; x < 3; x++) B0[x] = g.fcB0[(x + 3 * D) * fs + c];
+            B0n = qdiv(g.bFlux0[D * fs + c], (double)fa);
+        }
+    }
+    __syncthreads();  // the barrier's initialisation
+    if (!tma_wait(&bar)) {  // never in a sound step: stop it
+        sc->status = 5;
+        sc->halted = 1;
+        return;
+    }
+    if (!in) return;
+    GAM_BOX_CHECK(c - 4 * s, c + 3 * s, 8 + D);
+    flux_face<R, D, BORIS, false>(b, P, w, sc, gasN, gasO, c, sQ, sL, tx, tn, Vi, T, fa, Bn, B0, B0n);
+}
 #endif  // GAM_GEO_TABLES
 
 // E2Flux into the new buffer; faces outside its range are copied. With
