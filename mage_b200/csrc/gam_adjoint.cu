@@ -1898,7 +1898,7 @@ int update_call(const gam_params* p, const void* const* in, const void* const* g
         StateBuf<R> nxt{(R*)out[0], (R*)out[1], (R*)out[2]};
         k_update_faces<R><<<grid3(all, blk), blk, 0, s>>>(b, P, cur, nxt, w, sc, nullptr);
         const double gamma = p->gamma, gm1 = p->gamma - 1;
-        k_update_cells<R, sizeof(R) == 8 ? 6 : 8><<<grid3(cells, blk), blk, 0, s>>>(b, P, g, cur, nxt, w, sc, gamma, gm1);
+        k_update_cells<R, sizeof(R) == 8 ? 6 : 8><<<grid3(cells, blk), blk, 0, s>>>(b, P, g, cur, nxt, w, sc, gamma, gm1, 0);
     } else {
         k_update_adj_cells<R><<<grid3(cells, blk), blk, 0, s>>>(b, P, g, cur, w, dt, (const R*)din[0], (R*)dst[0],
                                                                  (R*)sU, (R*)sM);

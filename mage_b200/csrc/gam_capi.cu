@@ -309,7 +309,6 @@ template <class R> static int alloc_bulk(gam_handle* h, Ctx<R>& C) {
     C.sc = h->sc;
     C.gamma = h->p.gamma;
     C.gm1 = h->p.gamma - 1;
-    C.kvar = 0;
     return GAM_OK;
 }
 
@@ -817,6 +816,17 @@ extern "C" int gam_download_state(gam_handle* h, double* Gas, double* magFlux, d
     return GAM_OK;
 }
 
+void gam_strict_begin_f64(const Ctx<double>& C, cudaStream_t s);
+void gam_fast_begin_f64(const Ctx<double>& C, cudaStream_t s);
+void gam_fast_begin_f32(const Ctx<float>& C, cudaStream_t s);
+static void launch_begin(gam_handle* h) {
+    if (h->f32)
+        gam_fast_begin_f32(h->cf, h->s);
+    else if (h->p.strict)
+        gam_strict_begin_f64(h->cd, h->s);
+    else
+        gam_fast_begin_f64(h->cd, h->s);
+}
 static void launch_one(gam_handle* h, int cur) {
     if (h->f32)
         gam_fast_step_f32(h->cf, cur, h->s);
@@ -900,6 +910,7 @@ extern "C" int gam_step(gam_handle* h, int32_t nsteps, double* dt, double* t) {
     // host-side range with the reference's priority clock label (gamapp.F90:96-99)
     nvtxRangePushA("Gamera");
     CK(h, cudaEventRecord(h->ev0, h->s));
+    launch_begin(h);
     for (int n = 0; n < nsteps; n++) CK(h, cudaGraphLaunch(h->graph[(cur0 + n) & 1], h->s));
     CK(h, cudaEventRecord(h->ev1, h->s));
     nvtxRangePop();

@@ -1366,6 +1366,76 @@ __global__ void __launch_bounds__(256) k_update_faces(GamBox b, DevParams<R> P, 
 }
 
 __device__ __forceinline__ unsigned long long dbits(double x) { return (unsigned long long)__double_as_longlong(x); }
+// Scalars of the coming step from the current ones: AdvanceMHD's time trap and
+// the AB2 spacing (mhdgroup.F90:25-31, 457), Predictor (:459-463)
+__device__ __forceinline__ void step_scalars(GamScalars* sc) {
+    const double ot = fabs(sc->otime - sc->time) < TINY ? sc->time - sc->dt : sc->otime;
+    sc->odt = sc->time - ot;
+    sc->oodt = ot - sc->ootime;  // used with doAB3
+    sc->pdt = 0.5 * sc->dt;
+    sc->rodt = 1.0 / sc->odt;
+    sc->rdt = 1.0 / sc->dt;
+}
+// The end of a step: time bookkeeping and CalcDT's checks (gamapp.F90:110-111,
+// step.F90:58-168), by one thread; then the scalars of the next step
+__device__ __forceinline__ void finalize_dt(GamScalars* sc) {
+    if (fabs(sc->otime - sc->time) < TINY) sc->otime = sc->time - sc->dt;  // the time trap of this step
+    sc->ootime = sc->otime;        // CopyState(oState, ooState) (mhdgroup.F90:100-102)
+    sc->otime = sc->time;          // CopyState (mhdgroup.F90:255)
+    sc->time = sc->time + sc->dt;  // mhdgroup.F90:106
+    sc->ts = sc->ts + 1;
+    sc->t = sc->t + sc->dt;
+    if (sc->fixedTimestep) {
+        step_scalars(sc);
+        return;
+    }
+    const double dtOld = sc->dt;
+    double dtMin = __longlong_as_double((long long)sc->dtmin_bits);
+    sc->dtmin_bits = dbits(HUGE_DT);
+    bool isDisaster = (dtMin == HUGE_DT) || sc->nbad > 0;
+    bool isBad = false;
+    if (sc->ts > 0) {
+        if (dtOld / dtMin >= 10.0) isBad = true;
+        if (sc->dt0 > TINY && dtMin / sc->dt0 <= sc->limDT0) isBad = true;
+        if (dtMin <= TINY) isDisaster = true;
+    }
+    double dt = dtMin;
+    if (sc->t + dt > sc->tFin) dt = fmax(sc->tFin - sc->t, TINY);
+    if (sc->dt0 > TINY && dt > 10.0 * sc->dt0) dt = 10.0 * sc->dt0;
+    sc->dt = dt;
+    if (isDisaster) { sc->status = 5; sc->halted = 1; }
+    else if (isBad) { sc->status = 4; sc->halted = 1; }
+    else step_scalars(sc);
+}
+// The block's smallest dt candidate into the step's minimum, and whether one of
+// its cells has none. The minimum only falls, so a block that is not below the
+// value it reads leaves the atomic out: tens of thousands of them on one address
+// (69 us of a 96 x 96 x 128 CalcDT pass, one per warp) queue up behind each other.
+// last > 0: the last of that many blocks ends the step (finalize_dt).
+__device__ __forceinline__ void block_min_dt(double mydt, bool bad, double* smin, GamScalars* sc, unsigned last = 0) {
+    for (int o = 16; o > 0; o >>= 1) mydt = fmin(mydt, __shfl_xor_sync(0xffffffffu, mydt, o));
+    const int t = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
+    const int lane = t & 31, wid = t >> 5, nw = (blockDim.x * blockDim.y * blockDim.z + 31) >> 5;
+    if (lane == 0) smin[wid] = mydt;
+    const int anybad = __syncthreads_or(bad ? 1 : 0);
+    if (wid == 0) {
+        double v = lane < nw ? smin[lane] : HUGE_DT;
+        for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
+        if (lane == 0) {
+            if (v < HUGE_DT && dbits(v) < *(volatile unsigned long long*)&sc->dtmin_bits)
+                atomicMin(&sc->dtmin_bits, dbits(v));
+            if (anybad) atomicAdd(&sc->nbad, 1);
+            if (last) {
+                __threadfence();
+                if (atomicAdd(&sc->done, 1u) == last - 1) {
+                    sc->done = 0;
+                    __threadfence();
+                    finalize_dt(sc);
+                }
+            }
+        }
+    }
+}
 
 // CellDT (gridutils.F90:49-106), evaluated in FP64
 template <class R, bool BORIS>
@@ -1529,7 +1599,7 @@ __device__ __forceinline__ void update_cell(const GamBox& b, const DevParams<R>&
 template <class R, int MINB, bool BORIS = false>
 __global__ void __launch_bounds__(128, MINB) k_update_cells(GamBox b, DevParams<R> P, Geo<R> g, StateBuf<R> cur,
                                                       StateBuf<R> nxt, Work<R> w, GamScalars* sc, double gamma_d,
-                                                      double gm1_d) {
+                                                      double gm1_d, int fin) {
     __shared__ double smin[32];
     if (sc->halted) return;
     int ii, jj, kk;
@@ -1578,21 +1648,7 @@ __global__ void __launch_bounds__(128, MINB) k_update_cells(GamBox b, DevParams<
             for (int x = 0; x < 3; x++) nxt.B[x * fs + c] = Bc[x];
         }
     }
-    // block min
-    for (int o = 16; o > 0; o >>= 1) mydt = fmin(mydt, __shfl_xor_sync(0xffffffffu, mydt, o));
-    const int lane = (threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z)) & 31;
-    const int wid = (threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z)) >> 5;
-    const int nw = (blockDim.x * blockDim.y * blockDim.z + 31) >> 5;
-    if (lane == 0) smin[wid] = mydt;
-    unsigned anybad = __syncthreads_or(bad ? 1 : 0);
-    if (wid == 0) {
-        double v = lane < nw ? smin[lane] : HUGE_DT;
-        for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-        if (lane == 0) {
-            if (v < HUGE_DT) atomicMin(&sc->dtmin_bits, dbits(v));
-            if (anybad) atomicAdd(&sc->nbad, 1);
-        }
-    }
+    block_min_dt(mydt, bad, smin, sc, fin ? gridDim.x * gridDim.y * gridDim.z : 0u);
 }
 
 // ---- model hooks of the ionospheric boundary (bc[0] = 7; earthcmi.F90)
@@ -1682,18 +1738,7 @@ __global__ void __launch_bounds__(128) k_ion_push(GamBox b, DevParams<R> P, Geo<
             else bad = true;
         }
     }
-    for (int o = 16; o > 0; o >>= 1) mydt = fmin(mydt, __shfl_xor_sync(0xffffffffu, mydt, o));
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-    if (lane == 0) smin[wid] = mydt;
-    unsigned anybad = __syncthreads_or(bad ? 1 : 0);
-    if (wid == 0) {
-        double v = lane < nw ? smin[lane] : HUGE_DT;
-        for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-        if (lane == 0) {
-            if (v < HUGE_DT) atomicMin(&sc->dtmin_bits, dbits(v));
-            if (anybad) atomicAdd(&sc->nbad, 1);
-        }
-    }
+    block_min_dt(mydt, bad, smin, sc);
 }
 
 // HackE, wind part: WindEFix (apps/wind.F90:489-566), the EMFs of shells
@@ -1799,18 +1844,7 @@ __global__ void __launch_bounds__(128) k_nudge_sw(GamBox b, DevParams<R> P, Geo<
             else bad = true;
         }
     }
-    for (int o = 16; o > 0; o >>= 1) mydt = fmin(mydt, __shfl_xor_sync(0xffffffffu, mydt, o));
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-    if (lane == 0) smin[wid] = mydt;
-    unsigned anybad = __syncthreads_or(bad ? 1 : 0);
-    if (wid == 0) {
-        double v = lane < nw ? smin[lane] : HUGE_DT;
-        for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-        if (lane == 0) {
-            if (v < HUGE_DT) atomicMin(&sc->dtmin_bits, dbits(v));
-            if (anybad) atomicAdd(&sc->nbad, 1);
-        }
-    }
+    block_min_dt(mydt, bad, smin, sc);
 }
 
 
@@ -2007,14 +2041,18 @@ template <class R> __device__ __forceinline__ void ring_chunk_ghosts(R* chW, int
     }
 }
 
-// CalcSmoothE (ringav.F90:212-344) for one ring, one warp per ring: the J
+// CalcSmoothE (ringav.F90:212-344) for one ring, one block per ring: the J
 // fluxes through the ring (then the I fluxes) cleaned of Fourier modes
 // 0..nft, chunk-averaged, reconstructed, dirtied again; the change of each
 // face's flux accumulated along its chunk into the I (J) EMFs of the
 // smoothing field. Every sum keeps the sequential order of the CPU code
-// (one lane per sum); the lanes split the independent cells and chunks.
+// (one lane per sum); the lanes split the independent cells and chunks. A ring's
+// chain of dependent steps bounds both smoothing kernels, so a block of RING_NT
+// threads takes a ring's cells at once (one warp per ring took four rounds of
+// loads and divisions on a ring of 128).
+constexpr int RING_NT = 128;
 template <class R>
-__global__ void __launch_bounds__(32) k_ring_smooth_e(GamBox b, RingData Rg, StateBuf<R> S, const GamScalars* sc) {
+__global__ void __launch_bounds__(RING_NT) k_ring_smooth_e(GamBox b, RingData Rg, StateBuf<R> S, const GamScalars* sc) {
     if (sc->halted) return;
     const int G = GAM_NG, Np = Rg.Np, nsl = b.Nip + 1, lane = threadIdx.x;
     const long t = blockIdx.x;
@@ -2039,8 +2077,8 @@ __global__ void __launch_bounds__(32) k_ring_smooth_e(GamBox b, RingData Rg, Sta
         const int je = pole == 1 ? G + b.Njp - nR : (eD == 0 ? G + nR : G + nR - 1);
         const R* mf = S.mf + fD * fs;
         if (!GAM_BOX_OK(lidx(b, nS, jf, G), lidx(b, nS, jf, G + Np - 1), 15)) return;
-        for (int n = lane; n < Np; n += 32) bF[n] = mf[lidx(b, nS, jf, G + n)];
-        __syncwarp();
+        for (int n = lane; n < Np; n += RING_NT) bF[n] = mf[lidx(b, nS, jf, G + n)];
+        __syncthreads();
         // CleanRing's coefficients: one lane per sum, sequential over the ring
         if (lane < 2 * (Rg.nft + 1)) {
             const int m = lane >> 1;
@@ -2049,24 +2087,24 @@ __global__ void __launch_bounds__(32) k_ring_smooth_e(GamBox b, RingData Rg, Sta
             for (int n = 0; n < Np; n++) acc = acc + bF[n] * (R)tab[n];
             cf[lane] = (m == 0 ? (R)0.5 * (R)Rg.aScl : (R)1 * (R)Rg.aScl) * acc;
         }
-        __syncwarp();
-        for (int n = lane; n < Np; n += 32) {
+        __syncthreads();
+        for (int n = lane; n < Np; n += RING_NT) {
             R Q = bF[n];
             for (int m = 0; m <= Rg.nft; m++)
                 Q = Q - cf[2 * m] * (R)cs[(2 * m) * Np + n] - cf[2 * m + 1] * (R)cs[(2 * m + 1) * Np + n];
             cl[n] = Q;
         }
-        __syncwarp();
-        for (int c = lane; c < NumCh; c += 32) {
+        __syncthreads();
+        for (int c = lane; c < NumCh; c += RING_NT) {
             R sum = (R)0;
             for (int l = c * dC; l < (c + 1) * dC; l++) sum = sum + cl[l];
             chW[c + 2] = sum / (R)dC;
         }
-        __syncwarp();
+        __syncthreads();
         if (lane == 0) ring_chunk_ghosts(chW, NumCh);
-        __syncwarp();
+        __syncthreads();
         // reconstruct and dirty each cell, then its flux change
-        for (int n = lane; n < Np; n += 32) {
+        for (int n = lane; n < Np; n += RING_NT) {
             const int c = n / dC, m = n - c * dC + 1;
             R a, bq, cq;
             ring_parabola(Rg.recon, chW, c + 1, a, bq, cq);
@@ -2075,9 +2113,9 @@ __global__ void __launch_bounds__(32) k_ring_smooth_e(GamBox b, RingData Rg, Sta
                 ra = ra + cf[2 * mm] * (R)cs[(2 * mm) * Np + n] + cf[2 * mm + 1] * (R)cs[(2 * mm + 1) * Np + n];
             cl[n] = ra - bF[n];
         }
-        __syncwarp();
+        __syncthreads();
         // the changes accumulated along each chunk into the EMFs
-        for (int c = lane; c < NumCh; c += 32) {
+        for (int c = lane; c < NumCh; c += RING_NT) {
             R cum = (R)0;
             for (int m = 0; m < dC; m++) {
                 const int n = c * dC + m;
@@ -2091,10 +2129,10 @@ __global__ void __launch_bounds__(32) k_ring_smooth_e(GamBox b, RingData Rg, Sta
                 }
             }
         }
-        __syncwarp();
+        __syncthreads();
         // replicate k = ks at ke+1 (chunk 0 is lane 0's)
         if (lane == 0) E[eD * fs + lidx(b, nS, je, G + Np)] = E[eD * fs + lidx(b, nS, je, G)];
-        __syncwarp();
+        __syncthreads();
     }
 }
 
@@ -2172,12 +2210,12 @@ template <class R> __global__ void __launch_bounds__(128) k_ring_bfield(GamBox b
     for (int x = 0; x < 3; x++) S.B[x * fs + c] = B[x];
 }
 
-// SmoothGas (ringav.F90:78-210) for one ring, one warp per ring: the ring
+// SmoothGas (ringav.F90:78-210) for one ring, one block per ring: the ring
 // variables (rho, momentum, internal energy; Gas2Ring, ringutils.F90:
 // 804-830) chunk-averaged, reconstructed per chunk and written back as gas
 // (Ring2Gas :832-856); each chunk sum sequential on one lane
 template <class R>
-__global__ void __launch_bounds__(32) k_ring_smooth_gas(GamBox b, DevParams<R> P, StateBuf<R> S, const GamScalars* sc) {
+__global__ void __launch_bounds__(RING_NT) k_ring_smooth_gas(GamBox b, DevParams<R> P, StateBuf<R> S, const GamScalars* sc) {
     if (sc->halted) return;
     const RingData& Rg = P.ring;
     const int G = GAM_NG, Np = Rg.Np, nsl = b.Nip, lane = threadIdx.x;
@@ -2195,7 +2233,7 @@ __global__ void __launch_bounds__(32) k_ring_smooth_gas(GamBox b, DevParams<R> P
     R* chW = rW + 5 * Np;   // 5 x (NumCh + 4) chunk values
     const long fs = b.fs;
     if (!GAM_BOX_OK(lidx(b, nS, jr, G), lidx(b, nS, jr, G + Np - 1), 15)) return;
-    for (int n = lane; n < Np; n += 32) {
+    for (int n = lane; n < Np; n += RING_NT) {
         const long c = lidx(b, nS, jr, G + n);
         R W[5];
 #pragma unroll
@@ -2208,17 +2246,17 @@ __global__ void __launch_bounds__(32) k_ring_smooth_gas(GamBox b, DevParams<R> P
 #pragma unroll
         for (int v = 0; v < 5; v++) rW[v * Np + n] = W[v];
     }
-    __syncwarp();
-    for (int q = lane; q < 5 * NumCh; q += 32) {
+    __syncthreads();
+    for (int q = lane; q < 5 * NumCh; q += RING_NT) {
         const int v = q / NumCh, c = q % NumCh;
         R sum = (R)0;
         for (int l = c * dC; l < (c + 1) * dC; l++) sum = sum + rW[v * Np + l];
         chW[v * cst + c + 2] = sum / (R)dC;
     }
-    __syncwarp();
+    __syncthreads();
     if (lane < 5) ring_chunk_ghosts(chW + lane * cst, NumCh);
-    __syncwarp();
-    for (int n = lane; n < Np; n += 32) {
+    __syncthreads();
+    for (int n = lane; n < Np; n += RING_NT) {
         const int c = n / dC, m = n - c * dC + 1;
         R W[5];
 #pragma unroll
@@ -2282,28 +2320,7 @@ __global__ void __launch_bounds__(128) k_ring_nudge_axis(GamBox b, DevParams<R> 
 // mhdgroup.F90:106, step.F90:58-168). A failure halts the remaining kernels.
 __global__ void k_dt_finalize(GamScalars* sc) {
     if (sc->halted) return;
-    sc->ootime = sc->otime;        // CopyState(oState, ooState) (mhdgroup.F90:100-102)
-    sc->otime = sc->time;          // CopyState (mhdgroup.F90:255)
-    sc->time = sc->time + sc->dt;  // mhdgroup.F90:106
-    sc->ts = sc->ts + 1;
-    sc->t = sc->t + sc->dt;
-    if (sc->fixedTimestep) return;
-    const double dtOld = sc->dt;
-    double dtMin = __longlong_as_double((long long)sc->dtmin_bits);
-    sc->dtmin_bits = dbits(HUGE_DT);
-    bool isDisaster = (dtMin == HUGE_DT) || sc->nbad > 0;
-    bool isBad = false;
-    if (sc->ts > 0) {
-        if (dtOld / dtMin >= 10.0) isBad = true;
-        if (sc->dt0 > TINY && dtMin / sc->dt0 <= sc->limDT0) isBad = true;
-        if (dtMin <= TINY) isDisaster = true;
-    }
-    double dt = dtMin;
-    if (sc->t + dt > sc->tFin) dt = fmax(sc->tFin - sc->t, TINY);
-    if (sc->dt0 > TINY && dt > 10.0 * sc->dt0) dt = 10.0 * sc->dt0;
-    sc->dt = dt;
-    if (isDisaster) { sc->status = 5; sc->halted = 1; }
-    else if (isBad) { sc->status = 4; sc->halted = 1; }
+    finalize_dt(sc);
 }
 
 // Boundary kinds: 0 periodic, 1 none, 2 zero-gradient, 3 inner sphere,
@@ -2682,31 +2699,37 @@ static inline Shell make_shell(const GamBox& b) {
     return sh;
 }
 __device__ __forceinline__ int outer_coord(int o, int a, int bnd) { return (bnd >= a && o >= a) ? o - a + bnd + 1 : o; }
-__device__ __forceinline__ bool shell_ijk(const Shell& sh, long t, int& ii, int& jj, int& kk) {
-    if (t < sh.nA) {
-        ii = (int)(t % sh.nx);
-        long q = t / sh.nx;
-        jj = (int)(q % sh.ny);
-        kk = outer_coord((int)(q / sh.ny), sh.a[2], sh.bnd[2]);
+// 32-bit index arithmetic: a box whose fields fit the device holds far fewer
+// than 2^32 positions, and the 64-bit divisions were most of the work of a
+// thread with nothing to copy
+__device__ __forceinline__ bool shell_ijk(const Shell& sh, unsigned t, int& ii, int& jj, int& kk) {
+    const unsigned nx = sh.nx, ny = sh.ny;
+    if (t < (unsigned)sh.nA) {
+        const unsigned q = t / nx;
+        ii = t - q * nx;
+        const unsigned z = q / ny;
+        jj = q - z * ny;
+        kk = outer_coord((int)z, sh.a[2], sh.bnd[2]);
         return true;
     }
-    t -= sh.nA;
-    if (t < sh.nB) {
-        ii = (int)(t % sh.nx);
-        long q = t / sh.nx;
-        const int nout1 = sh.ny - (sh.bnd[1] >= sh.a[1] ? sh.bnd[1] - sh.a[1] + 1 : 0);
-        jj = outer_coord((int)(q % nout1), sh.a[1], sh.bnd[1]);
-        kk = sh.a[2] + (int)(q / nout1);
+    t -= (unsigned)sh.nA;
+    const int nin1 = sh.bnd[1] >= sh.a[1] ? sh.bnd[1] - sh.a[1] + 1 : 0;
+    if (t < (unsigned)sh.nB) {
+        const unsigned q = t / nx, nout1 = ny - nin1;
+        ii = t - q * nx;
+        const unsigned z = q / nout1;
+        jj = outer_coord((int)(q - z * nout1), sh.a[1], sh.bnd[1]);
+        kk = sh.a[2] + (int)z;
         return true;
     }
-    t -= sh.nB;
-    if (t < sh.nC) {
-        const int nout0 = sh.nx - (sh.bnd[0] >= sh.a[0] ? sh.bnd[0] - sh.a[0] + 1 : 0);
-        ii = outer_coord((int)(t % nout0), sh.a[0], sh.bnd[0]);
-        long q = t / nout0;
-        const int nin1 = sh.bnd[1] - sh.a[1] + 1;
-        jj = sh.a[1] + (int)(q % nin1);
-        kk = sh.a[2] + (int)(q / nin1);
+    t -= (unsigned)sh.nB;
+    if (t < (unsigned)sh.nC) {
+        const unsigned nout0 = nx - (sh.bnd[0] >= sh.a[0] ? sh.bnd[0] - sh.a[0] + 1 : 0);
+        const unsigned q = t / nout0;
+        ii = outer_coord((int)(t - q * nout0), sh.a[0], sh.bnd[0]);
+        const unsigned z = q / (unsigned)nin1;
+        jj = sh.a[1] + (int)(q - z * nin1);
+        kk = sh.a[2] + (int)z;
         return true;
     }
     return false;
@@ -2717,8 +2740,7 @@ __global__ void __launch_bounds__(256) k_bc(GamBox b, DevParams<R> P, Geo<R> g, 
                                             int copyB, Shell sh) {
     if (sc->halted) return;
     int ii, jj, kk;
-    const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (!shell_ijk(sh, t, ii, jj, kk)) return;
+    if (!shell_ijk(sh, blockIdx.x * blockDim.x + threadIdx.x, ii, jj, kk)) return;
     const long fs = b.fs;
     const long c = lidx(b, ii, jj, kk);
     GAM_BOX_CHECK(c, c, 14);
@@ -2816,11 +2838,13 @@ template <class R> void launch_bcs(const Ctx<R>& C, const StateBuf<R>& S, cudaSt
 template <class R>
 __global__ void __launch_bounds__(128) k_dt_only(GamBox b, DevParams<R> P, Geo<R> g, StateBuf<R> s,
                                                  GamScalars* sc, double gamma_d, double gm1_d, int countBad) {
+    __shared__ double smin[32];
     int ii, jj, kk;
     const int G = GAM_NG;
     Range r{G - P.dtIlo, G + b.Nip - 1 + P.dtIhi, G - P.dtJlo, G + b.Njp - 1 + P.dtJhi, G - P.dtKlo,
             G + b.Nkp - 1 + P.dtKhi};
     double mydt = HUGE_DT;
+    bool bad = false;
     if (thread_ijk(r, ii, jj, kk) && GAM_BOX_OK(lidx(b, ii, jj, kk), lidx(b, ii, jj, kk), 13)) {
         const long fs = b.fs;
         const long c = lidx(b, ii, jj, kk);
@@ -2837,11 +2861,10 @@ __global__ void __launch_bounds__(128) k_dt_only(GamBox b, DevParams<R> P, Geo<R
         double dtc = P.doBoris ? cell_dt<R, true>(P, Ud, Bt, (double)g.dl[c], gamma_d, gm1_d, sc->CFL)
                                 : cell_dt<R, false>(P, Ud, Bt, (double)g.dl[c], gamma_d, gm1_d, sc->CFL);
         if (dtc > 0.0 && dtc < 1.0e300) mydt = dtc;
-        else if (countBad && !sc->fixedTimestep) atomicAdd(&sc->nbad, 1);
+        else bad = countBad != 0;
     }
     if (sc->fixedTimestep && countBad) return;
-    for (int o = 16; o > 0; o >>= 1) mydt = fmin(mydt, __shfl_xor_sync(0xffffffffu, mydt, o));
-    if ((threadIdx.x & 31) == 0 && mydt < HUGE_DT) atomicMin(&sc->dtmin_bits, dbits(mydt));
+    block_min_dt(mydt, bad, smin, sc);
 }
 
 
@@ -2894,7 +2917,7 @@ template <class R> void launch_ring_average(const Ctx<R>& C, const StateBuf<R>& 
         k_ring_zero_e<R><<<(unsigned)((nz + 255) / 256), 256, 0, s>>>(b, Rg, C.sc);
         const long ne = 2L * (b.Nip + 1) * Rg.NumR;
         const size_t smE = (size_t)(2 * Rg.Np + Rg.chunkStride / 5) * sizeof(R);
-        k_ring_smooth_e<R><<<(unsigned)ne, 32, smE, s>>>(b, Rg, O, C.sc);
+        k_ring_smooth_e<R><<<(unsigned)ne, RING_NT, smE, s>>>(b, Rg, O, C.sc);
         R* E = (R*)Rg.smoothE;
         const int ni = b.Nip + 1;
         k_ring_pole_e<R><<<(unsigned)(2 * ni), 32, Rg.Np * sizeof(R), s>>>(b, Rg, E, G, G + b.Nip, C.sc);
@@ -2913,7 +2936,7 @@ template <class R> void launch_ring_average(const Ctx<R>& C, const StateBuf<R>& 
     }
     const long ng = 2L * b.Nip * Rg.NumR;
     const size_t smG = (size_t)(5 * Rg.Np + Rg.chunkStride) * sizeof(R);
-    k_ring_smooth_gas<R><<<(unsigned)ng, 32, smG, s>>>(b, C.P, O, C.sc);
+    k_ring_smooth_gas<R><<<(unsigned)ng, RING_NT, smG, s>>>(b, C.P, O, C.sc);
 }
 
 // The kernels of one stepGamera in order, each handed to f(id, launch) with
@@ -2921,7 +2944,7 @@ template <class R> void launch_ring_average(const Ctx<R>& C, const StateBuf<R>& 
 // I/J/K, 11 update_faces, 12 update_cells, 13 dt_finalize, 14 bc.
 // st[cur] is State (n); st[1-cur] holds oState (n-1) on entry and State
 // (n+1) on exit.
-template <class R, class F> void for_each_kernel(const Ctx<R>& C, int cur, cudaStream_t& s, F&& f) {
+template <class R, class F> void for_each_kernel(const Ctx<R>& C, int cur, cudaStream_t& s, F&& f, int fold = 0) {
     const GamBox& b = C.b;
     const int G = GAM_NG;
     const StateBuf<R> S = C.st[cur], O = C.st[1 - cur];
@@ -3010,9 +3033,9 @@ template <class R, class F> void for_each_kernel(const Ctx<R>& C, int cur, cudaS
                 k_ion_flux<R><<<16, 32, C.P.ring.Np * sizeof(R), s>>>(b, C.P, C.w, C.sc);
         }
         if (C.P.doBoris)
-            k_update_cells<R, sizeof(R) == 8 ? 6 : 8, true><<<grid_for(cells, blk), blk, 0, s>>>(b, C.P, C.g, S, O, C.w, C.sc, C.gamma, C.gm1);
+            k_update_cells<R, sizeof(R) == 8 ? 6 : 8, true><<<grid_for(cells, blk), blk, 0, s>>>(b, C.P, C.g, S, O, C.w, C.sc, C.gamma, C.gm1, fold);
         else  // strict: 6 blocks/SM (732 us at 192^3; 8: 792, 5: 784, 4: 819); the other forms 8
-            k_update_cells<R, GAM_STRICT_KERNELS ? 6 : 8><<<grid_for(cells, blk), blk, 0, s>>>(b, C.P, C.g, S, O, C.w, C.sc, C.gamma, C.gm1);
+            k_update_cells<R, GAM_STRICT_KERNELS ? 6 : 8><<<grid_for(cells, blk), blk, 0, s>>>(b, C.P, C.g, S, O, C.w, C.sc, C.gamma, C.gm1, fold);
         if (C.P.ring.on) launch_ring_average(C, O, s);  // mhdgroup.F90:69-74
         if (C.P.ion.push) {  // HackStep (PerStep, earthcmi.F90:224-263): PushIon, before CalcDT
             const long np = (long)C.P.ion.nIonP * b.Njp * b.Nkp;
@@ -3037,7 +3060,7 @@ template <class R, class F> void for_each_kernel(const Ctx<R>& C, int cur, cudaS
             k_dt_only<R><<<grid_for(r, blk2), blk2, 0, s>>>(b, C.P, C.g, O, C.sc, C.gamma, C.gm1, 1);
         }
     });
-    f(13, [&] { k_dt_finalize<<<1, 1, 0, s>>>(C.sc); });
+    if (!fold) f(13, [&] { k_dt_finalize<<<1, 1, 0, s>>>(C.sc); });
     f(14, [&] { launch_bcs(C, O, s, 0); });
 }
 
@@ -3046,22 +3069,26 @@ template <class R, class F> void for_each_kernel(const Ctx<R>& C, int cur, cudaS
 // (then the face update) beside the three flux directions; the cell update
 // joins them. Every branch writes its own arrays, so the result is the same
 // bits as the sequential order.
+//
+// A grid of a few cells is bound by the chain of its launches: the step's
+// scalars are ready from the step before (finalize_dt; launch_begin before the
+// first), and the last block of the cell update ends the step where no later
+// kernel adds to CalcDT (rings, the ionospheric hooks).
 template <class R> void launch_step(const Ctx<R>& C, int cur, cudaStream_t s) {
     cudaStream_t cs = s;
-    if (!C.aux[0] || (C.kvar & 64)) {
-        for_each_kernel(C, cur, cs, [](int, auto&& L) { L(); });
+    const int fold = !C.P.ring.on && !C.P.ion.push && !C.P.ion.wind;
+    if (!C.aux[0]) {
+        for_each_kernel(C, cur, cs, [](int id, auto&& L) { if (id) L(); }, fold);
         return;
     }
     for_each_kernel(C, cur, cs, [&](int id, auto&& L) {
         switch (id) {
-            case 0:
+            case 0: return;
             case 1:
                 cs = s;
                 L();
-                if (id == 1) {
-                    cudaEventRecord(C.ev[0], s);
-                    for (int q = 0; q < 5; q++) cudaStreamWaitEvent(C.aux[q], C.ev[0], 0);
-                }
+                cudaEventRecord(C.ev[0], s);
+                for (int q = 0; q < 5; q++) cudaStreamWaitEvent(C.aux[q], C.ev[0], 0);
                 return;
             case 2: case 3: cs = C.aux[0]; break;
             case 4: case 5: cs = C.aux[1]; break;
@@ -3088,8 +3115,10 @@ template <class R> void launch_step(const Ctx<R>& C, int cur, cudaStream_t s) {
             default: cs = s; break;
         }
         L();
-    });
+    }, fold);
 }
+// the scalars of the first step after the host may have set some
+template <class R> void launch_begin(const Ctx<R>& C, cudaStream_t s) { k_step_begin<<<1, 1, 0, s>>>(C.sc); }
 
 // Device time of each kernel of a step (ms, average of reps back-to-back
 // launches; ms[15]). The kernels after k_step_begin read their inputs and

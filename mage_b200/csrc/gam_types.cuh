@@ -224,7 +224,6 @@ template <class R> struct Ctx {
     double gamma, gm1;
     // side streams and fork/join events of the step graph (independent
     // kernels of a step run as parallel branches); null: one stream
-    int kvar;  // launch-configuration variant for tuning runs (GAM_KVAR); 0 = the tuned default
     cudaStream_t aux[5];
     cudaEvent_t ev[8];
 };
