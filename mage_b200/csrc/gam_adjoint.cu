@@ -36,12 +36,12 @@ template <class A> __device__ __forceinline__ A sgnz(A x) { return x > (A)0 ? (A
 // reverse of lrs_from_qdv (8CENT) for one variable: scatter the adjoints of
 // Ql, Qr to the 8-point operand stencil and the 4-point limiter stencil
 template <class R, class A>
-__device__ void lrs_adj(R pdmb, const R* qdv, const R* v, R Vi, A rVi, A aL, A aR, A* aq,
+__device__ void lrs_adj(R pdmb, const R* qdv, const R* v, const Quot<R>& Vi, A rVi, A aL, A aR, A* aq,
                         A* av, A* a_scale = nullptr) {
     R s = (R)0;
 #pragma unroll
     for (int n = 0; n < 8; n++) s += Rc<R>(w8(n)) * qdv[n];
-    const R Qi = s / Vi;
+    const R Qi = Vi(s);
     const R v0 = v[0], v1 = v[1], v2 = v[2], v3 = v[3];
     const R maxV = rmax(v1, v2), minV = rmin(v1, v2);
     const R t = rmin(Qi, maxV);
@@ -75,6 +75,40 @@ __device__ void lrs_adj(R pdmb, const R* qdv, const R* v, R Vi, A rVi, A aL, A a
 #pragma unroll
     for (int n = 0; n < 8; n++) aq[n] = (A)w8(n) * a_s;
     av[0] = a0; av[1] = a1; av[2] = a2; av[3] = a3;
+}
+
+// Asynchronous copies of single values into shared memory: rows of the callers'
+// unpadded boxes start anywhere, which a TMA copy cannot
+__device__ __forceinline__ void cp_async(double* dst, const double* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async(float* dst, const float* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+// The stencil boxes of a block's tile (FluxTile) from the callers' arrays by all
+// of its threads: box position (x, n) of field v, n along j or k; a position past
+// the box (of a tile past the range) takes its last value.
+template <class R, int D>
+__device__ __forceinline__ void load_flux_tile(const GamBox& b, const DevParams<R>& P, const Work<R>& w,
+                                               const R* __restrict__ Blim, int i0, int j0, int k0, R* sQ, R* sL) {
+    using T_ = FluxTile<R, D>;
+    const int tx = threadIdx.x % T_::TX, tn = threadIdx.x / T_::TX;
+    const long fs = b.fs;
+    const long s = D == 0 ? 1L : (D == 1 ? (long)b.sx : b.sk), sn = D == 2 ? b.sk : (long)b.sx;
+    const int nvar = P.doMHD ? 8 : 5;
+    const long q0 = lidx(b, i0, j0, k0) - 4 * s, l0 = lidx(b, i0, j0, k0) - (D == 0 ? 4 : 2) * s;
+    for (int x = tx; x < T_::QX; x += T_::TX)
+        for (int n = tn; n < T_::QN; n += T_::TN) {
+            const long cq = min(q0 + x + n * sn, b.nbox - 1), cl = min(l0 + x + n * sn, b.nbox - 1);
+#pragma unroll
+            for (int v = 0; v < 8; v++) {
+                if (v >= nvar) break;
+                cp_async(sQ + (v * T_::QN + n) * T_::QX + x, (v < 5 ? w.QW + v * fs : w.QB + (v - 5) * fs) + cq);
+                if (n < T_::LN)
+                    cp_async(sL + (v * T_::LN + n) * T_::QX + x, (v < 5 ? w.Wn + v * fs : Blim + (v - 5) * fs) + cl);
+            }
+        }
+    asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
 // reverse of mag_kin_flux for one side: adjoints aM (of the mF sums) and aVaD
@@ -219,17 +253,32 @@ __device__ void gas_adj(const DevParams<R>& P, A sgn, const R* W, const R* T, co
 // recomputing kernel took 214-240 registers (2 blocks); bounded it spills
 // (local memory, L1-resident) but hides more load latency (measured on
 // 128^3: 3 -> 4 FP64 blocks took the adjoint step from 5.9 to 5.7 ms; with
-// the saved states, 5 -> 6 FP32 blocks about 1 %).
+// the saved states, 5 -> 6 FP32 blocks about 1 %). The stencils come to shared
+// memory while the first loads are under way: with loads by each thread, kept
+// twice because registers were short, the three sweeps took 537/545/575 us at
+// 128^3 in FP64, now 496/480/515 (3.6 to 4.0 TB/s).
 template <class R, int D, bool SAVED = false>
-__global__ void __launch_bounds__(128, (sizeof(R) == 8 ? 4 : 6)) k_stress_adj(GamBox b, DevParams<R> P, Geo<R> g, const R* __restrict__ Blim,
+__global__ void __launch_bounds__(FluxTile<R, D>::NT, sizeof(R) == 8 ? 4 : (D == 0 ? 6 : 3)) k_stress_adj(GamBox b, DevParams<R> P, Geo<R> g, const R* __restrict__ Blim,
                                                     Work<R> w, Range r, const R* __restrict__ dgF,
                                                     const R* __restrict__ dmF, R* dQW, R* dWn, R* dQB, R* dBlim,
                                                     R* dBnf, R* __restrict__ rs) {
-    int ii, jj, kk;
-    if (!thread_ijk(r, ii, jj, kk)) return;
+    using T_ = FluxTile<R, D>;
+    extern __shared__ __align__(128) unsigned char flux_smem[];
+    R* sQ = (R*)flux_smem;
+    R* sL = (R*)(flux_smem + T_::LOFF);
+    const int tx = threadIdx.x % T_::TX, tn = threadIdx.x / T_::TX;
+    const int i0 = r.i0 + blockIdx.x * T_::TX;
+    const int j0 = r.j0 + blockIdx.y * (D == 2 ? 1 : T_::TN);
+    const int k0 = r.k0 + blockIdx.z * (D == 2 ? T_::TN : 1);
+    load_flux_tile<R, D>(b, P, w, Blim, i0, j0, k0, sQ, sL);
+    const int ii = i0 + tx, jj = D == 2 ? j0 : j0 + tn, kk = D == 2 ? k0 + tn : k0;
+    const bool in = ii <= r.i1 && jj <= r.j1 && kk <= r.k1;
     const long fs = b.fs;
-    const long c = lidx(b, ii, jj, kk);
+    const long c = lidx(b, min(ii, r.i1), min(jj, r.j1), min(kk, r.k1));
     const long s = D == 0 ? 1L : (D == 1 ? (long)b.sx : b.sk);
+    const R* pQ = sQ + tn * T_::QX + tx;
+    const R* pL = sL + tn * T_::QX + tx + (D == 0 ? 2 : 0);
+    constexpr int st = D == 0 ? 1 : T_::TX;
     R T[9];
     for (int n = 0; n < 9; n++) T[n] = g.Tf[(n + 9 * D) * fs + c];
     const R fa = g.face[D * fs + c];
@@ -260,20 +309,21 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 8 ? 4 : 6)) k_stress_adj(Ga
         }
         VaD = o[16 * fs];
     } else {
-        // forward states; the stencils are loaded again for the reverse of
-        // the reconstruction rather than kept live (fewer registers, more warps)
+        // forward states
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
         const Quot<R> qVi(Vi);  // the 8 reconstructions share the divisor
         for (int v = 0; v < 5; v++) {
             R qW[8], nW[4];
-            for (int n = 0; n < 8; n++) qW[n] = w.QW[v * fs + c + (n - 4) * s];
-            for (int m = 0; m < 4; m++) nW[m] = w.Wn[v * fs + c + (m - 2) * s];
+            for (int n = 0; n < 8; n++) qW[n] = pQ[v * T_::QN * T_::QX + n * st];
+            for (int m = 0; m < 4; m++) nW[m] = pL[v * T_::LN * T_::QX + m * st];
             lrs_from_qdv(P, qW, nW, qVi, WL[v], WR[v]);
         }
         if (P.doMHD) {
             for (int x = 0; x < 3; x++) {
                 R qB[8], nB[4];
-                for (int n = 0; n < 8; n++) qB[n] = w.QB[x * fs + c + (n - 4) * s];
-                for (int m = 0; m < 4; m++) nB[m] = Blim[x * fs + c + (m - 2) * s];
+                for (int n = 0; n < 8; n++) qB[n] = pQ[(5 + x) * T_::QN * T_::QX + n * st];
+                for (int m = 0; m < 4; m++) nB[m] = pL[(5 + x) * T_::LN * T_::QX + m * st];
                 lrs_from_qdv(P, qB, nB, qVi, MagL[x], MagR[x]);
             }
             R mFs[3] = {(R)0, (R)0, (R)0}, bbD = (R)0;
@@ -301,17 +351,23 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 8 ? 4 : 6)) k_stress_adj(Ga
         for (int x = 0; x < 3; x++) aM[x] = (A)fa * dmF[(x + 3 * D) * fs + c];
         mag_adj(P, (A)-1, WL, MagL, Bn, T, B0, B0n, aM, aVaD, aWL, aBL, aBn);
         mag_adj(P, (A)1, WR, MagR, Bn, T, B0, B0n, aM, aVaD, aWR, aBR, aBn);
-        dBnf[D * fs + c] += (R)aBn;
+        if (in) dBnf[D * fs + c] += (R)aBn;
     }
     // reverse of the reconstruction: scatter to the stencils
+    if constexpr (SAVED) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+    }
+    if (!in) return;
     A aq[8], av[4];
+    const Quot<R> qVi(Vi);
     const A rVi = (A)1 / (A)Vi;
     for (int v = 0; v < 5; v++) {
         R qW[8], nW[4];
-        for (int n = 0; n < 8; n++) qW[n] = w.QW[v * fs + c + (n - 4) * s];
-        for (int m = 0; m < 4; m++) nW[m] = w.Wn[v * fs + c + (m - 2) * s];
+        for (int n = 0; n < 8; n++) qW[n] = pQ[v * T_::QN * T_::QX + n * st];
+        for (int m = 0; m < 4; m++) nW[m] = pL[v * T_::LN * T_::QX + m * st];
         A as;
-        lrs_adj(P.pdmb, qW, nW, Vi, rVi, aWL[v], aWR[v], aq, av, &as);
+        lrs_adj(P.pdmb, qW, nW, qVi, rVi, aWL[v], aWR[v], aq, av, &as);
         if (rs) {  // per face: the stencil weight scale and the 4 limiter adjoints
             rs[(5 * v) * fs + c] = (R)as;
             for (int m = 0; m < 4; m++) rs[(5 * v + 1 + m) * fs + c] = (R)av[m];
@@ -323,10 +379,10 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 8 ? 4 : 6)) k_stress_adj(Ga
     if (P.doMHD)
         for (int x = 0; x < 3; x++) {
             R qB[8], nB[4];
-            for (int n = 0; n < 8; n++) qB[n] = w.QB[x * fs + c + (n - 4) * s];
-            for (int m = 0; m < 4; m++) nB[m] = Blim[x * fs + c + (m - 2) * s];
+            for (int n = 0; n < 8; n++) qB[n] = pQ[(5 + x) * T_::QN * T_::QX + n * st];
+            for (int m = 0; m < 4; m++) nB[m] = pL[(5 + x) * T_::LN * T_::QX + m * st];
             A as;
-            lrs_adj(P.pdmb, qB, nB, Vi, rVi, aBL[x], aBR[x], aq, av, &as);
+            lrs_adj(P.pdmb, qB, nB, qVi, rVi, aBL[x], aBR[x], aq, av, &as);
             if (rs) {
                 rs[(5 * (5 + x)) * fs + c] = (R)as;
                 for (int m = 0; m < 4; m++) rs[(5 * (5 + x) + 1 + m) * fs + c] = (R)av[m];
@@ -419,14 +475,6 @@ __global__ void __launch_bounds__(256) k_stress_adj_gather3(GamBox b, Range r0, 
 }
 
 
-// Asynchronous copies of single values into shared memory: rows of the callers'
-// unpadded boxes start anywhere, which a TMA copy cannot
-__device__ __forceinline__ void cp_async(double* dst, const double* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async(float* dst, const float* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
 // Face fluxes of direction D (Fluxes, stress.F90:204-429) on the callers'
 // arrays, one face per thread; the stencil boxes come into shared memory by
 // asynchronous copies of all threads (see k_stress).
@@ -443,25 +491,7 @@ __global__ void __launch_bounds__(FluxTile<R, D>::NT, MINB)
     const int j0 = r.j0 + blockIdx.y * (D == 2 ? 1 : T_::TN);
     const int k0 = r.k0 + blockIdx.z * (D == 2 ? T_::TN : 1);
     const long fs = b.fs;
-    const long s = D == 0 ? 1L : (D == 1 ? (long)b.sx : b.sk), sn = D == 2 ? b.sk : (long)b.sx;
-    const int nvar = P.doMHD ? 8 : 5;
-    {
-        // box position (x, n) of field v, n along j or k; a position past the box
-        // (of a tile past the range) takes its last value
-        const long q0 = lidx(b, i0, j0, k0) - 4 * s, l0 = lidx(b, i0, j0, k0) - (D == 0 ? 4 : 2) * s;
-        for (int x = tx; x < T_::QX; x += T_::TX)
-            for (int n = tn; n < T_::QN; n += T_::TN) {
-                const long cq = min(q0 + x + n * sn, b.nbox - 1), cl = min(l0 + x + n * sn, b.nbox - 1);
-#pragma unroll
-                for (int v = 0; v < 8; v++) {
-                    if (v >= nvar) break;
-                    cp_async(sQ + (v * T_::QN + n) * T_::QX + x, (v < 5 ? w.QW + v * fs : w.QB + (v - 5) * fs) + cq);
-                    if (n < T_::LN)
-                        cp_async(sL + (v * T_::LN + n) * T_::QX + x, (v < 5 ? w.Wn + v * fs : Blim + (v - 5) * fs) + cl);
-                }
-            }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    }
+    load_flux_tile<R, D>(b, P, w, Blim, i0, j0, k0, sQ, sL);
     const int ii = i0 + tx, jj = D == 2 ? j0 : j0 + tn, kk = D == 2 ? k0 + tn : k0;
     const bool in = ii <= r.i1 && jj <= r.j1 && kk <= r.k1;
     const long c = lidx(b, min(ii, r.i1), min(jj, r.j1), min(kk, r.k1));
@@ -485,13 +515,18 @@ __global__ void __launch_bounds__(FluxTile<R, D>::NT, MINB)
     if (!in) return;
     flux_face<R, D, false, true>(b, P, w, sc, nullptr, nullptr, c, sQ, sL, tx, tn, Vi, T, fa, Bn, B0, B0n);
 }
+// the grid of FluxTile's blocks over the faces r of direction D
+template <class R, int D> dim3 flux_grid(const Range& r) {
+    using T_ = FluxTile<R, D>;
+    return dim3((unsigned)((r.i1 - r.i0 + T_::TX) / T_::TX),
+                (unsigned)(D == 2 ? r.j1 - r.j0 + 1 : (r.j1 - r.j0 + T_::TN) / T_::TN),
+                (unsigned)(D == 2 ? (r.k1 - r.k0 + T_::TN) / T_::TN : r.k1 - r.k0 + 1));
+}
 template <class R, int D>
 void launch_stress_box(const GamBox& b, const DevParams<R>& P, const Geo<R>& g, const R* Bl, const Work<R>& w,
                        const Range& r, const GamScalars* sc, cudaStream_t s) {
     using T_ = FluxTile<R, D>;
-    const dim3 sg((unsigned)((r.i1 - r.i0 + T_::TX) / T_::TX),
-                  (unsigned)(D == 2 ? r.j1 - r.j0 + 1 : (r.j1 - r.j0 + T_::TN) / T_::TN),
-                  (unsigned)(D == 2 ? (r.k1 - r.k0 + T_::TN) / T_::TN : r.k1 - r.k0 + 1));
+    const dim3 sg = flux_grid<R, D>(r);
     k_stress_box<R, D, sizeof(R) == 8 ? 4 : (D == 0 ? 7 : 4)><<<sg, T_::NT, T_::SMEM, s>>>(b, P, g, Bl, w, r, sc);
 }
 
@@ -604,7 +639,7 @@ __device__ void edge_lrs_adj(const GamBox& b, const DevParams<R>& P, const Geo<R
     for (int m = 0; m < 4; m++) nmag[m] = w.bn[a * fs + c + (m - 2) * s];
     const R Vi = central8(area);
     A aq[8], av[4], as;
-    lrs_adj<R, A>(P.pdmb, qdv, nmag, Vi, (A)1.0 / (A)Vi, aBL * (A)Vi, aBR * (A)Vi, aq, av, &as);
+    lrs_adj<R, A>(P.pdmb, qdv, nmag, Quot<R>(Vi), (A)1.0 / (A)Vi, aBL * (A)Vi, aBR * (A)Vi, aq, av, &as);
     if (es) {  // per edge: the stencil weight scale and the 4 limiter adjoints (es[0..4 fs])
         es[c] = (R)as;
         for (int m = 0; m < 4; m++) es[(1 + m) * fs + c] = (R)av[m];
@@ -824,30 +859,35 @@ __global__ void __launch_bounds__(256) k_vxb_adj_gather3(GamBox b, Geo<R> g, Ran
         const Range rm = mf.r[eD];
         const bool inm = ii >= rm.i0 && ii <= rm.i1 && jj >= rm.j0 && jj <= rm.j1 && kk >= rm.k0 && kk <= rm.k1;
         const long s2 = dstride(b, dT2);
-        double AdV = 0.0;
+        A v[3] = {(A)0, (A)0, (A)0};
+        if (inm && full) {
+            R y[3][8];
+#pragma unroll
+            for (int x = 0; x < 3; x++)
+#pragma unroll
+                for (int n = 0; n < 8; n++) y[x][n] = e[(10 + x) * fs + (4 - n) * s2];
+#pragma unroll
+            for (int x = 0; x < 3; x++)
+#pragma unroll
+                for (int n = 0; n < 8; n++) v[x] += (A)w8(n) * (A)y[x][n];
+        } else if (inm) {
+#pragma unroll
+            for (int x = 0; x < 3; x++)
+#pragma unroll
+                for (int n = 0; n < 8; n++)
+                    if (in_r(dT2, 4 - n)) v[x] += (A)w8(n) * (A)e[(10 + x) * fs + (4 - n) * s2];
+        }
+        double AdV = 0.0;  // after the stencil's loads: its division has a branch
         if (inm) {
             const long s1 = dstride(b, dT1);
             R vol[8];
-            for (int n = 0; n < 8; n++) vol[n] = g.vol[c + (n - 4) * s1];
+#pragma unroll
+            for (int n = 0; n < 8; n++) vol[n] = __ldg(g.vol + c + (n - 4) * s1);
             const R dV = rmax(central8(vol), (R)TINY);
-            AdV = (double)g.face[dT1 * fs + c] / (double)dV;
+            AdV = (double)__ldg(g.face + dT1 * fs + c) / (double)dV;
         }
 #pragma unroll
-        for (int x = 0; x < 3; x++) {
-            A v = (A)0;
-            if (inm && full) {
-                R y[8];
-#pragma unroll
-                for (int n = 0; n < 8; n++) y[n] = e[(10 + x) * fs + (4 - n) * s2];
-#pragma unroll
-                for (int n = 0; n < 8; n++) v += (A)w8(n) * (A)y[n];
-            } else if (inm) {
-#pragma unroll
-                for (int n = 0; n < 8; n++)
-                    if (in_r(dT2, 4 - n)) v += (A)w8(n) * (A)e[(10 + x) * fs + (4 - n) * s2];
-            }
-            aS[(3 * eD + x) * fs + c] = inm ? (R)((double)(R)v * AdV) : (R)0;
-        }
+        for (int x = 0; x < 3; x++) aS[(3 * eD + x) * fs + c] = inm ? (R)((double)(R)v[x] * AdV) : (R)0;
         // the 4 corners of GetCornerD: edges c, c + s1, c + s2, c + s1 + s2
         const int e1 = eD == 0 ? 1 : 0, e2 = eD == 2 ? 1 : 2;
         const long t1 = dstride(b, e1), t2 = dstride(b, e2);
@@ -1028,7 +1068,20 @@ __global__ void __launch_bounds__(128) k_predict_adj_cells(GamBox b, DevParams<R
     const long fs = b.fs, c = lidx(b, ii, jj, kk);
     const A dF = P.dFloor, pF = P.pFloor, gm1 = P.gm1;
     A Q[5], oQ[5], W[5], oW[5], pW[5], pWf[5], pQ[5];
+    // every load before the first division (its branches keep later loads
+    // waiting: 128^3 FP64 took 350 us for 1 GB; now 157)
+    A dQW[5], dWn[5], dV[3], dB[3] = {0, 0, 0}, gQ[5], goQ[5];
     for (int v = 0; v < 5; v++) { Q[v] = cur.Gas[v * fs + c]; oQ[v] = old.Gas[v * fs + c]; }
+    for (int v = 0; v < 5; v++) {
+        dQW[v] = dw.QW[v * fs + c];
+        dWn[v] = dw.Wn[v * fs + c];
+        gQ[v] = dGas[v * fs + c];
+        goQ[v] = doGas[v * fs + c];
+    }
+    for (int x = 0; x < 3; x++) dV[x] = dw.VdV[x * fs + c];
+    if (P.doMHD)
+        for (int x = 0; x < 3; x++) dB[x] = dw.QB[x * fs + c];
+    const A dD = dw.Dh[c], vol = g.vol[c];
     auto c2p = [&](const A* U, A* Wo) {
         const A rho = U[0], rr = (A)1.0 / rho;
         const A Vx = U[1] * rr, Vy = U[2] * rr, Vz = U[3] * rr;
@@ -1050,14 +1103,13 @@ __global__ void __launch_bounds__(128) k_predict_adj_cells(GamBox b, DevParams<R
         const A KinE = (A)0.5 * rho * (pWf[1] * pWf[1] + pWf[2] * pWf[2] + pWf[3] * pWf[3]);
         pQ[0] = rho; pQ[1] = rho * pWf[1]; pQ[2] = rho * pWf[2]; pQ[3] = rho * pWf[3]; pQ[4] = IntE + KinE;
     }
-    const A vol = g.vol[c];
     A aWh[5], apQ[5] = {0, 0, 0, 0, 0};
-    for (int v = 0; v < 5; v++) aWh[v] = vol * (A)dw.QW[v * fs + c];
-    aWh[0] += dw.Dh[c];
+    for (int v = 0; v < 5; v++) aWh[v] = vol * dQW[v];
+    aWh[0] += dD;
     const A Dm = pQ[0] < dF ? dF : pQ[0], rDm = (A)1.0 / Dm;
     A aDm = (A)0.0;
     for (int x = 0; x < 3; x++) {
-        const A a = dw.VdV[x * fs + c];
+        const A a = dV[x];
         apQ[1 + x] += vol * a * rDm;
         aDm += -vol * pQ[1 + x] * a * rDm * rDm;
     }
@@ -1078,14 +1130,14 @@ __global__ void __launch_bounds__(128) k_predict_adj_cells(GamBox b, DevParams<R
     c2p_adj(dF, pF, gm1, Q, aW, aQ);
     c2p_adj(dF, pF, gm1, oQ, aoW, aoQ);
     A aWn[5];
-    for (int v = 0; v < 5; v++) aWn[v] = dw.Wn[v * fs + c];
+    for (int v = 0; v < 5; v++) aWn[v] = dWn[v];
     bc2p_adj(dF, pF, gm1, Q, aWn, aQ);
     for (int v = 0; v < 5; v++) {
-        dGas[v * fs + c] += (R)aQ[v];
-        doGas[v * fs + c] += (R)aoQ[v];
+        dGas[v * fs + c] = (R)gQ[v] + (R)aQ[v];
+        doGas[v * fs + c] = (R)goQ[v] + (R)aoQ[v];
     }
     if (P.doMHD)
-        for (int x = 0; x < 3; x++) aB[x * fs + c] = (R)(vol * (A)dw.QB[x * fs + c]);
+        for (int x = 0; x < 3; x++) aB[x * fs + c] = (R)(vol * dB[x]);
 }
 
 // predictor adjoint, faces: dabh, dBnf, dbn and the Bxyz adjoints of the two
@@ -1101,28 +1153,61 @@ __global__ void __launch_bounds__(256) k_predict_adj_faces(GamBox b, DevParams<R
     if (!P.doMHD) return;
     const int ijk[3] = {ii, jj, kk}, n[3] = {b.Ni, b.Nj, b.Nk};
     const A pr = pdt / odt;
-    A rv = (A)0.0;
-    if (ii < b.Ni && jj < b.Nj && kk < b.Nk) rv = (A)1.0 / (A)g.vol[c];
+    // loads first (see k_predict_adj_cells): this cell's, then per direction the
+    // face's and those of the cell whose upper face it is (128^3 FP64: 269 -> 222 us)
+    const bool inLo = ii < b.Ni && jj < b.Nj && kk < b.Nk;
+    A aLo[3] = {0, 0, 0}, Af[3], ah[3], bf[3], bl[3], gm[3], gom[3], rvol[4] = {1, 1, 1, 1}, aUp[3][3];
+    R wLo[3][3], wUp[3][3];
+    bool inUp[3];
+    if (inLo) {
+        rvol[3] = (A)g.vol[c];
+#pragma unroll
+        for (int x = 0; x < 3; x++) aLo[x] = (A)aB[x * fs + c];
+    }
+#pragma unroll
     for (int d = 0; d < 3; d++) {
-        const A Af = g.face[d * fs + c];
-        const A Am = Af < (A)TINY ? (A)TINY : Af, rAm = (A)1.0 / Am;
-        A ahm = (A)dw.abh[d * fs + c] * Af * rAm + (A)dw.Bnf[d * fs + c] / Af;
-        // cells c (this is its lower face d) and c - s_d (its upper face)
-        bool inLo = true, inUp = true;
-        for (int e = 0; e < 3; e++) {
-            const int lo = ijk[e] - (e == d ? 1 : 0);
-            if (ijk[e] >= n[e]) inLo = false;
-            if (lo < 0 || lo >= n[e]) inUp = false;
+        Af[d] = g.face[d * fs + c];
+        ah[d] = dw.abh[d * fs + c];
+        bf[d] = dw.Bnf[d * fs + c];
+        bl[d] = dw.bn[d * fs + c];
+        gm[d] = dmf[d * fs + c];
+        gom[d] = domf[d * fs + c];
+        inUp[d] = ijk[d] >= 1;
+#pragma unroll
+        for (int e = 0; e < 3; e++)
+            if (ijk[e] - (e == d ? 1 : 0) >= n[e]) inUp[d] = false;
+#pragma unroll
+        for (int x = 0; x < 3; x++) {
+            wLo[d][x] = wUp[d][x] = (R)0;
+            aUp[d][x] = (A)0;
         }
-        if (inLo)
-            for (int x = 0; x < 3; x++) ahm += (A)aB[x * fs + c] * rv * dbdf(b, g, c, 2 * d, x);
-        if (inUp) {
+        if (inLo) {
+#pragma unroll
+            for (int x = 0; x < 3; x++) wLo[d][x] = dbdf(b, g, c, 2 * d, x);
+        }
+        if (inUp[d]) {
             const long cu = c - dstride(b, d);
-            const A rvu = (A)1.0 / (A)g.vol[cu];
-            for (int x = 0; x < 3; x++) ahm += (A)aB[x * fs + cu] * rvu * dbdf(b, g, cu, 2 * d + 1, x);
+            rvol[d] = (A)g.vol[cu];
+#pragma unroll
+            for (int x = 0; x < 3; x++) {
+                aUp[d][x] = (A)aB[x * fs + cu];
+                wUp[d][x] = dbdf(b, g, cu, 2 * d + 1, x);
+            }
         }
-        dmf[d * fs + c] += (R)(ahm + ahm * pr + (A)dw.bn[d * fs + c] * rAm);
-        domf[d * fs + c] += (R)(-ahm * pr);
+    }
+    const A rv = (A)1.0 / rvol[3];
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        const A Am = Af[d] < (A)TINY ? (A)TINY : Af[d], rAm = (A)1.0 / Am;
+        A ahm = ah[d] * Af[d] * rAm + bf[d] / Af[d];
+        // cells c (this is its lower face d) and c - s_d (its upper face)
+#pragma unroll
+        for (int x = 0; x < 3; x++) ahm += aLo[x] * rv * wLo[d][x];
+        const A rvu = (A)1.0 / rvol[d];
+#pragma unroll
+        for (int x = 0; x < 3; x++) ahm += aUp[d][x] * rvu * wUp[d][x];
+        dmf[d * fs + c] = (R)gm[d] + (R)(ahm + ahm * pr + bl[d] * rAm);
+        domf[d * fs + c] = (R)gom[d] + (R)(-ahm * pr);
     }
 }
 
@@ -1643,11 +1728,11 @@ int flux_call(const gam_params* p, const void* QW, const void* Wn, const void* Q
         const long fs40 = 40L * b.fs;
         const R* a = (const R*)dgF;
         const R* m = (const R*)dmF;
-        k_stress_adj<R, 0, true><<<grid(fr[0]), blk, 0, s>>>(b, P, g, Bl, w, fr[0], a, m, (R*)dQW, (R*)dWn, (R*)dQB,
+        k_stress_adj<R, 0, true><<<flux_grid<R, 0>(fr[0]), FluxTile<R, 0>::NT, FluxTile<R, 0>::SMEM, s>>>(b, P, g, Bl, w, fr[0], a, m, (R*)dQW, (R*)dWn, (R*)dQB,
                                                               (R*)dBlim, (R*)dBnf, rs);
-        k_stress_adj<R, 1, true><<<grid(fr[1]), blk, 0, s>>>(b, P, g, Bl, w, fr[1], a, m, (R*)dQW, (R*)dWn, (R*)dQB,
+        k_stress_adj<R, 1, true><<<flux_grid<R, 1>(fr[1]), FluxTile<R, 1>::NT, FluxTile<R, 1>::SMEM, s>>>(b, P, g, Bl, w, fr[1], a, m, (R*)dQW, (R*)dWn, (R*)dQB,
                                                               (R*)dBlim, (R*)dBnf, rs ? rs + fs40 : nullptr);
-        k_stress_adj<R, 2, true><<<grid(fr[2]), blk, 0, s>>>(b, P, g, Bl, w, fr[2], a, m, (R*)dQW, (R*)dWn, (R*)dQB,
+        k_stress_adj<R, 2, true><<<flux_grid<R, 2>(fr[2]), FluxTile<R, 2>::NT, FluxTile<R, 2>::SMEM, s>>>(b, P, g, Bl, w, fr[2], a, m, (R*)dQW, (R*)dWn, (R*)dQB,
                                                               (R*)dBlim, (R*)dBnf, rs ? rs + 2 * fs40 : nullptr);
         if (rs) {
             const dim3 gblk(32, 8, 1);
@@ -1664,11 +1749,11 @@ int flux_call(const gam_params* p, const void* QW, const void* Wn, const void* Q
         // dQW, dWn, dQB and dBlim
         R* rs = (R*)rscratch;
         const long fs40 = 40L * b.fs;
-        k_stress_adj<R, 0><<<grid(fr[0]), blk, 0, s>>>(b, P, g, Bl, w, fr[0], a, m, (R*)dQW, (R*)dWn, (R*)dQB,
+        k_stress_adj<R, 0><<<flux_grid<R, 0>(fr[0]), FluxTile<R, 0>::NT, FluxTile<R, 0>::SMEM, s>>>(b, P, g, Bl, w, fr[0], a, m, (R*)dQW, (R*)dWn, (R*)dQB,
                                                         (R*)dBlim, (R*)dBnf, rs);
-        k_stress_adj<R, 1><<<grid(fr[1]), blk, 0, s>>>(b, P, g, Bl, w, fr[1], a, m, (R*)dQW, (R*)dWn, (R*)dQB,
+        k_stress_adj<R, 1><<<flux_grid<R, 1>(fr[1]), FluxTile<R, 1>::NT, FluxTile<R, 1>::SMEM, s>>>(b, P, g, Bl, w, fr[1], a, m, (R*)dQW, (R*)dWn, (R*)dQB,
                                                         (R*)dBlim, (R*)dBnf, rs ? rs + fs40 : nullptr);
-        k_stress_adj<R, 2><<<grid(fr[2]), blk, 0, s>>>(b, P, g, Bl, w, fr[2], a, m, (R*)dQW, (R*)dWn, (R*)dQB,
+        k_stress_adj<R, 2><<<flux_grid<R, 2>(fr[2]), FluxTile<R, 2>::NT, FluxTile<R, 2>::SMEM, s>>>(b, P, g, Bl, w, fr[2], a, m, (R*)dQW, (R*)dWn, (R*)dQB,
                                                         (R*)dBlim, (R*)dBnf, rs ? rs + 2 * fs40 : nullptr);
         if (rs) {
             const dim3 gblk(32, 8, 1);

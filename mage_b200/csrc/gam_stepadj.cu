@@ -167,28 +167,50 @@ __global__ void k_box_bxyz_adj(Box b, const R* __restrict__ vol, const R* __rest
     const int p[3] = {i, j, k};
     const int N[3] = {b.Ni, b.Nj, b.Nk};
     const bool inCell = i < b.Ni && j < b.Nj && k < b.Nk;
-    const DivBy<R> byV(inCell ? vol[t] : (R)1);
+    // loads first: the quotients' branches keep later loads waiting (128^3 FP64:
+    // 187 -> 175 us)
+    R gT[3] = {(R)0, (R)0, (R)0}, wT[3][3], gC[3][3], wC[3][3], vC[3] = {(R)1, (R)1, (R)1}, old[3];
+    const R vT = inCell ? vol[t] : (R)1;
+    bool below[3];
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-        bool below = p[d] >= 1;
+        below[d] = p[d] >= 1;
+#pragma unroll
         for (int a = 0; a < 3; a++)
-            if (p[a] >= N[a] + (a == d ? 1 : 0)) below = false;
-        R acc = (R)0;
-        if (below) {
+            if (p[a] >= N[a] + (a == d ? 1 : 0)) below[d] = false;
+        old[d] = dmf[d * n + t];
+        if (below[d]) {
             const long c = t - st[d];
-            const DivBy<R> byVc(vol[c]);
+            vC[d] = vol[c];
+#pragma unroll
             for (int x = 0; x < 3; x++) {
-                const R w = dxf ? dxf[(x + 3 + 6 * d) * n + c] : xfc[(x + 3 * d) * n + t] - xyzcc[x * n + c];
-                acc = acc + byVc(gB[x * n + c] * w);
+                gC[d][x] = gB[x * n + c];
+                wC[d][x] = dxf ? dxf[(x + 3 + 6 * d) * n + c] : xfc[(x + 3 * d) * n + t] - xyzcc[x * n + c];
             }
         }
         if (inCell) {
-            for (int x = 0; x < 3; x++) {
-                const R w = dxf ? dxf[(x + 6 * d) * n + t] : xfc[(x + 3 * d) * n + t] - xyzcc[x * n + t];
-                acc = acc - byV(gB[x * n + t] * w);
-            }
+#pragma unroll
+            for (int x = 0; x < 3; x++) wT[d][x] = dxf ? dxf[(x + 6 * d) * n + t] : xfc[(x + 3 * d) * n + t] - xyzcc[x * n + t];
         }
-        dmf[d * n + t] += acc;
+    }
+    if (inCell) {
+#pragma unroll
+        for (int x = 0; x < 3; x++) gT[x] = gB[x * n + t];
+    }
+    const DivBy<R> byV(vT);
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        R acc = (R)0;
+        if (below[d]) {
+            const DivBy<R> byVc(vC[d]);
+#pragma unroll
+            for (int x = 0; x < 3; x++) acc = acc + byVc(gC[d][x] * wC[d][x]);
+        }
+        if (inCell) {
+#pragma unroll
+            for (int x = 0; x < 3; x++) acc = acc - byV(gT[x] * wT[d][x]);
+        }
+        dmf[d * n + t] = old[d] + acc;
     }
 }
 
