@@ -1295,7 +1295,7 @@ __global__ void __launch_bounds__(FluxTile<R, D>::NT, MINB)
     }
     const int ii = i0 + tx, jj = D == 2 ? j0 : j0 + tn, kk = D == 2 ? k0 + tn : k0;
     const long fs = b.fs;
-    const long s = D == 0 ? 1L : (D == 1 ? (long)b.sx : b.sk);
+    [[maybe_unused]] const long s = D == 0 ? 1L : (D == 1 ? (long)b.sx : b.sk);
     // threads past the range take the range's last face (and store nothing)
     const bool in = ii <= r.i1 && jj <= r.j1 && kk <= r.k1;
     const long c = lidx(b, min(ii, r.i1), min(jj, r.j1), min(kk, r.k1));
@@ -2989,7 +2989,7 @@ template <class R, class F> void for_each_kernel(const Ctx<R>& C, int cur, cudaS
                       (unsigned)(D == 2 ? (r.k1 - r.k0 + T_::TN) / T_::TN : r.k1 - r.k0 + 1));
         const GamFluxMaps& M = C.fmaps->m[cur][D];
         // blocks per SM (registers against warps; 192^3, I/J/K sweeps): the strict
-        // form 5 (816/739/808 us; 4: 852/770/775, 7: 895/854/859), the FMA form 5
+        // form 5 (782/739/808 us; 4: 852/770/775, 7: 895/854/859), the FMA form 5
         // (598/560/563; 4: 627/576/586, 6: 648/611/636), FP32 5 of 256 threads on
         // the J and K sweeps (263/264; 4: 269/275) and 7 of 128 on the I sweep
         constexpr int MB = sizeof(R) == 8 ? 5 : (D == 0 ? 7 : 5);

@@ -151,12 +151,15 @@ struct Range {  // inclusive box-index range
 // reconstruction operands of cells -4..3 and limiter values of cells -2..1
 // along D. On the I sweep both boxes start 4 cells below the tile's first face
 // (a TMA box starts on a 16-byte boundary: an even cell in FP64, a multiple of
-// 4 in FP32; the flux ranges start at cell 4 and tiles are 16 or 32 wide).
+// 4 in FP32; the flux ranges start at cell 4 and tiles are 16 or 32 wide). The I
+// sweep's boxes are 8 cells wider than its tile; 16 x 8 faces instead of 32 x 4
+// fit a grid's odd extents better: 192^3 strict 858 -> 782 us, FP32 296 -> 280,
+// 96^3 125 -> 113 and 47 -> 43.
 template <class R, int D> struct FluxTile {
-    static constexpr int TX = D == 0 ? 32 : (sizeof(R) == 8 ? 16 : 32);
-    static constexpr int TN = D == 0 ? 4 : 8;
+    static constexpr int TX = D == 0 || sizeof(R) == 8 ? 16 : 32;
+    static constexpr int TN = 8;
     static constexpr int NT = TX * TN;
-    static constexpr int QX = D == 0 ? 40 : TX;
+    static constexpr int QX = D == 0 ? TX + 8 : TX;
     static constexpr int QN = D == 0 ? TN : TN + 7, LN = D == 0 ? TN : TN + 3;
     static constexpr unsigned BYTES = 8u * (QN + LN) * QX * sizeof(R), BYTES_GAS = 5u * (QN + LN) * QX * sizeof(R);
     static constexpr unsigned LOFF = 8u * QN * QX * sizeof(R), SMEM = BYTES;
