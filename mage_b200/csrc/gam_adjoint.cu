@@ -1981,9 +1981,9 @@ int update_call(const gam_params* p, const void* const* in, const void* const* g
     const dim3 blk(32, 4, 1);
     if (out) {
         StateBuf<R> nxt{(R*)out[0], (R*)out[1], (R*)out[2]};
-        k_update_faces<R><<<grid3(all, blk), blk, 0, s>>>(b, P, cur, nxt, w, sc, nullptr);
+        k_update_faces<R><<<grid3(all, blk), blk, 0, s>>>(b, P, cur, nxt, w, all, sc, nullptr);
         const double gamma = p->gamma, gm1 = p->gamma - 1;
-        k_update_cells<R, sizeof(R) == 8 ? 6 : 8><<<grid3(cells, blk), blk, 0, s>>>(b, P, g, cur, nxt, w, sc, gamma, gm1, 0);
+        k_update_cells<R, sizeof(R) == 8 ? 6 : 8><<<grid3(cells, blk), blk, 0, s>>>(b, P, g, cur, nxt, w, sc, gamma, gm1, cells, 0);
     } else {
         k_update_adj_cells<R><<<grid3(cells, blk), blk, 0, s>>>(b, P, g, cur, w, dt, (const R*)din[0], (R*)dst[0],
                                                                  (R*)sU, (R*)sM);

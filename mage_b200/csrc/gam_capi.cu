@@ -716,7 +716,7 @@ static int set_scalars(gam_handle* h, double time, double otime, double dt, int3
     CK(h, cudaStreamSynchronize(h->s));
     s.time = time; s.otime = otime; s.t = time; s.dt = dt; s.ts = ts;
     if (!keepOO) s.ootime = otime - dt;
-    s.status = 0; s.halted = 0; s.nbad = 0;
+    s.status = 0; s.halted = 0; s.nbad = 0; s.fixGhosts = 0;
     double hugedt = 1.0e12;
     memcpy(&s.dtmin_bits, &hugedt, 8);
     CK(h, cudaMemcpyAsync(h->sc, &s, sizeof(s), cudaMemcpyHostToDevice, h->s));

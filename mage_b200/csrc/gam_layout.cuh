@@ -51,6 +51,7 @@ struct GamScalars {
     int halted;                        // set once a step failed; later kernels return at once
     int fixedTimestep;
     int nbad;                          // cells whose dt is not a finite positive number
+    int fixGhosts;                     // the step just failed: its boundary kernel copies the ghosts of its start
     unsigned done;                     // blocks of the cell update that are through (0 between steps)
     double ootime, oodt;               // ooState time and oState - ooState spacing (doAB3)
     // bounds-check build (GAM_BOUNDS_CHECK): first failed index check

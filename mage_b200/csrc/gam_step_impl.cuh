@@ -20,9 +20,10 @@
 //   k_update_cells   Flux2Deltas, CellReynolds, bFlux2Fld, CellMaxwell, and the
 //                    per-cell CFL dt with a block min       (stress.F90:148-194,
 //                    mhdgroup.F90:79-329, gridutils.F90:49-106)
-//   k_dt_finalize    time bookkeeping + CalcDT checks       (gamapp.F90:110-111, step.F90:58-168)
-//   k_bc_periodic    EnforceBCs (periodic / none) fused with bFlux2Fld of
-//                    the cells whose faces changed          (bcs.F90:279-450, gamapp.F90:86-88)
+//   finalize_dt      time bookkeeping + CalcDT checks, in the last block of the
+//                    update where nothing comes between     (gamapp.F90:110-111, step.F90:58-168)
+//   k_bc             EnforceBCs (the kinds that copy values) fused with bFlux2Fld
+//                    of the cells whose faces changed       (bcs.F90:279-450, gamapp.F90:86-88)
 //
 // Every expression keeps the reference's evaluation order (Fortran a+b+c is
 // (a+b)+c, x**2.0 is x*x, dot_product is a sequential sum from 0), so the
@@ -725,13 +726,15 @@ __device__ __forceinline__ void predict_at(const GamBox& b, const DevParams<R>& 
 // area * flux/max(area,TINY) and flux/max(area,TINY) (EdgeLRs), flux/area (Fluxes).
 template <class R, int MINB, bool AB3 = false>
 __global__ void __launch_bounds__(256, MINB) k_predict(GamBox b, DevParams<R> P, Geo<R> g, StateBuf<R> cur,
-                                                 StateBuf<R> old, Work<R> w, const GamScalars* sc,
+                                                 StateBuf<R> old, Work<R> w, GamScalars* sc,
                                                  const R* __restrict__ oomf) {
-    if (sc->halted) return;
+    if (sc->halted) {  // the steps after a failed one leave its ghosts alone
+        if (blockIdx.x + blockIdx.y + blockIdx.z + threadIdx.x + threadIdx.y == 0) sc->fixGhosts = 0;
+        return;
+    }
     int ii, jj, kk;
     Range r{0, b.Ni, 0, b.Nj, 0, b.Nk};
     if (!thread_ijk(r, ii, jj, kk)) return;
-    const long fs = b.fs;
     const long c = lidx(b, ii, jj, kk);
     const R pdt = (R)sc->pdt, odt = (R)sc->odt;
     const bool isCell = ii < b.Ni && jj < b.Nj && kk < b.Nk;
@@ -1349,10 +1352,9 @@ __global__ void __launch_bounds__(FluxTile<R, D>::NT, MINB)
 // (CopyState(oState, ooState), mhdgroup.F90:100-102).
 template <class R>
 __global__ void __launch_bounds__(256) k_update_faces(GamBox b, DevParams<R> P, StateBuf<R> cur, StateBuf<R> nxt,
-                                                      Work<R> w, const GamScalars* sc, R* __restrict__ oomf) {
+                                                      Work<R> w, Range r, const GamScalars* sc, R* __restrict__ oomf) {
     if (sc->halted) return;
     int ii, jj, kk;
-    Range r{0, b.Ni, 0, b.Nj, 0, b.Nk};
     if (!thread_ijk(r, ii, jj, kk)) return;
     const long fs = b.fs;
     const long c = lidx(b, ii, jj, kk);
@@ -1424,6 +1426,7 @@ __device__ __forceinline__ void finalize_dt(GamScalars* sc) {
     if (isDisaster) { sc->status = 5; sc->halted = 1; }
     else if (isBad) { sc->status = 4; sc->halted = 1; }
     else step_scalars(sc);
+    sc->fixGhosts = sc->halted;
 }
 // The block's smallest dt candidate into the step's minimum, and whether one of
 // its cells has none. The minimum only falls, so a block that is not below the
@@ -1617,11 +1620,10 @@ __device__ __forceinline__ void update_cell(const GamBox& b, const DevParams<R>&
 template <class R, int MINB, bool BORIS = false>
 __global__ void __launch_bounds__(128, MINB) k_update_cells(GamBox b, DevParams<R> P, Geo<R> g, StateBuf<R> cur,
                                                       StateBuf<R> nxt, Work<R> w, GamScalars* sc, double gamma_d,
-                                                      double gm1_d, int fin) {
+                                                      double gm1_d, Range r, int fin) {
     __shared__ double smin[32];
     if (sc->halted) return;
     int ii, jj, kk;
-    Range r{0, b.Ni - 1, 0, b.Nj - 1, 0, b.Nk - 1};
     bool ok = thread_ijk(r, ii, jj, kk);
     ok = ok && GAM_BOX_OK(lidx(b, ii, jj, kk), lidx(b, ii, jj, kk) + b.sk, 12);
     double mydt = HUGE_DT;
@@ -2753,82 +2755,141 @@ __device__ __forceinline__ bool shell_ijk(const Shell& sh, unsigned t, int& ii, 
     return false;
 }
 
+// A step that failed CalcDT stops before its boundary conditions with the ghosts
+// of its start (the update's copies, mhdgroup.F90:202-256) and their field. The
+// update leaves out the layers that the boundaries fill, so they are copied here.
 template <class R>
-__global__ void __launch_bounds__(256) k_bc(GamBox b, DevParams<R> P, Geo<R> g, StateBuf<R> s, const GamScalars* sc,
-                                            int copyB, Shell sh) {
-    if (sc->halted) return;
+__device__ void failed_ghosts(const GamBox& b, const DevParams<R>& P, const Geo<R>& g, const StateBuf<R>& s,
+                              const StateBuf<R>& cur, int ii, int jj, int kk, bool isCell) {
+    const int G = GAM_NG;
+    const long fs = b.fs, c = lidx(b, ii, jj, kk);
+    auto updated = [&](int x, int y, int z) {  // a face in E2Flux's range
+        return P.doMHD && x >= G && x <= G + b.Nip && y >= G && y <= G + b.Njp && z >= G && z <= G + b.Nkp;
+    };
+    auto face = [&](int d, int x, int y, int z) {
+        const long q = d * fs + lidx(b, x, y, z);
+        return updated(x, y, z) ? s.mf[q] : cur.mf[q];
+    };
+    if (!updated(ii, jj, kk)) {
+#pragma unroll
+        for (int d = 0; d < 3; d++) s.mf[d * fs + c] = cur.mf[d * fs + c];
+    }
+    const bool active = ii >= G && ii < G + b.Nip && jj >= G && jj < G + b.Njp && kk >= G && kk < G + b.Nkp;
+    if (!isCell || active) return;
+#pragma unroll
+    for (int v = 0; v < 5; v++) s.Gas[v * fs + c] = cur.Gas[v * fs + c];
+    if (!P.doMHD) return;
+    int jb = jj, kb = kk;
+    if (P.ring.on) ring_conj_cc(b, P.ring, jb, kb);  // RingFlux2FieldFix
+    R B[3];
+    cell_bxyz(b, g, lidx(b, ii, jb, kb), face(0, ii, jb, kb), face(0, ii + 1, jb, kb), face(1, ii, jb, kb),
+              face(1, ii, jb + 1, kb), face(2, ii, jb, kb), face(2, ii, jb, kb + 1), B);
+#pragma unroll
+    for (int x = 0; x < 3; x++) s.B[x * fs + c] = B[x];
+}
+
+// Every load of a position comes before its first store: a source position is
+// an active one that no thread writes, but the compiler cannot know that, and a
+// load, store, load chain over 11 values took 25 us on a grid of 128 x 128 x 4,
+// now 17; 192^3 strict 136 -> 121 us, FP32 88 -> 82. Blocks of 128 at 6 (FP64) or 8
+// per SM: without the bound the loads held at once take 83 registers and FP64
+// 192^3 takes 170 us.
+template <class R>
+__global__ void __launch_bounds__(128, sizeof(R) == 8 ? 6 : 8)
+    k_bc(GamBox b, DevParams<R> P, Geo<R> g, StateBuf<R> s, StateBuf<R> cur, const GamScalars* sc, int copyB, Shell sh) {
+    if (sc->halted && !(sc->fixGhosts && !copyB)) return;
     int ii, jj, kk;
     if (!shell_ijk(sh, blockIdx.x * blockDim.x + threadIdx.x, ii, jj, kk)) return;
     const long fs = b.fs;
     const long c = lidx(b, ii, jj, kk);
     GAM_BOX_CHECK(c, c, 14);
+    const bool isCell = ii < b.Ni && jj < b.Nj && kk < b.Nk;
+    if (sc->halted) {
+        failed_ghosts(b, P, g, s, cur, ii, jj, kk, isCell);
+        return;
+    }
+    R fv[3], gv[5], bv[3], B[3];
+    bool fm[3], gm = false, bm = false, bnew = false;
     // faces
 #pragma unroll
     for (int d = 0; d < 3; d++) {
         int x = ii, y = jj, z = kk;
         const int sg = bc_source(b, P, d, false, x, y, z);
         GAM_BOX_CHECK(lidx(b, x, y, z), lidx(b, x, y, z), 14);
-        if (x != ii || y != jj || z != kk) {
-            const R v = s.mf[d * fs + lidx(b, x, y, z)];
-            s.mf[d * fs + c] = sg < 0 ? -v : v;
+        fm[d] = x != ii || y != jj || z != kk;
+        if (fm[d]) {
+            fv[d] = s.mf[d * fs + lidx(b, x, y, z)];
+            if (sg < 0) fv[d] = -fv[d];
         }
     }
-    if (ii >= b.Ni || jj >= b.Nj || kk >= b.Nk) return;
-    // cell
-    {
+    if (isCell) {
         int x = ii, y = jj, z = kk;
         bc_source(b, P, -1, false, x, y, z);
         GAM_BOX_CHECK(lidx(b, x, y, z), lidx(b, x, y, z), 14);
-        if (x != ii || y != jj || z != kk) {
+        gm = x != ii || y != jj || z != kk;
+        if (gm) {
             const long src = lidx(b, x, y, z);
 #pragma unroll
-            for (int v = 0; v < 5; v++) s.Gas[v * fs + c] = s.Gas[v * fs + src];
+            for (int v = 0; v < 5; v++) gv[v] = s.Gas[v * fs + src];
         }
         if (copyB) {
             int xb = ii, yb = jj, zb = kk;
             bc_source(b, P, -1, true, xb, yb, zb);
             GAM_BOX_CHECK(lidx(b, xb, yb, zb), lidx(b, xb, yb, zb), 14);
-            if (xb != ii || yb != jj || zb != kk) {
+            bm = xb != ii || yb != jj || zb != kk;
+            if (bm) {
                 const long src = lidx(b, xb, yb, zb);
 #pragma unroll
-                for (int q = 0; q < 3; q++) s.B[q * fs + c] = s.B[q * fs + src];
+                for (int q = 0; q < 3; q++) bv[q] = s.B[q * fs + src];
             }
+        } else if (P.doMHD) {
+            // the six faces of this cell after the boundary fill
+            auto srcf = [&](int d, int a0, int a1, int a2) -> long {
+                int x = a0, y = a1, z = a2;
+                bc_source(b, P, d, false, x, y, z);
+                return lidx(b, x, y, z);
+            };
+            // RingFlux2FieldFix: a cell across the LFM pole takes its conjugate's field
+            int jb = jj, kb = kk;
+            const bool conj = P.ring.on && ring_conj_cc(b, P.ring, jb, kb);
+            const long fI = srcf(0, ii, jb, kb), fIp = srcf(0, ii + 1, jb, kb);
+            const long fJ = srcf(1, ii, jb, kb), fJp = srcf(1, ii, jb + 1, kb);
+            const long fK = srcf(2, ii, jb, kb), fKp = srcf(2, ii, jb, kb + 1);
+            {
+                long lo = fI, hi = fI;
+                for (long v : {fIp, fJ, fJp, fK, fKp}) {
+                    lo = v < lo ? v : lo;
+                    hi = v > hi ? v : hi;
+                }
+                GAM_BOX_CHECK(lo, hi, 14);
+            }
+            const bool facesMapped = fI != c || fIp != c + 1 || fJ != c || fJp != c + b.sx || fK != c || fKp != c + b.sk;
+            const int G = GAM_NG;
+            const bool ghost =
+                ii < G || ii >= G + b.Nip || jj < G || jj >= G + b.Njp || kk < G || kk >= G + b.Nkp;
+            bnew = ghost || facesMapped;
+            if (bnew)
+                cell_bxyz(b, g, conj ? lidx(b, ii, jb, kb) : c, s.mf[fI], s.mf[fIp], s.mf[fs + fJ], s.mf[fs + fJp],
+                          s.mf[2 * fs + fK], s.mf[2 * fs + fKp], B);
         }
     }
-    if (!P.doMHD || copyB) return;
-    // the six faces of this cell after the boundary fill
-    auto srcf = [&](int d, int a0, int a1, int a2) -> long {
-        int x = a0, y = a1, z = a2;
-        bc_source(b, P, d, false, x, y, z);
-        return lidx(b, x, y, z);
-    };
-    // RingFlux2FieldFix: a cell across the LFM pole takes its conjugate's field
-    int jb = jj, kb = kk;
-    const bool conj = P.ring.on && ring_conj_cc(b, P.ring, jb, kb);
-    const long fI = srcf(0, ii, jb, kb), fIp = srcf(0, ii + 1, jb, kb);
-    const long fJ = srcf(1, ii, jb, kb), fJp = srcf(1, ii, jb + 1, kb);
-    const long fK = srcf(2, ii, jb, kb), fKp = srcf(2, ii, jb, kb + 1);
-    {
-        long lo = fI, hi = fI;
-        for (long v : {fIp, fJ, fJp, fK, fKp}) {
-            lo = v < lo ? v : lo;
-            hi = v > hi ? v : hi;
-        }
-        GAM_BOX_CHECK(lo, hi, 14);
-    }
-    const bool facesMapped = fI != c || fIp != c + 1 || fJ != c || fJp != c + b.sx || fK != c || fKp != c + b.sk;
-    const int G = GAM_NG;
-    const bool ghost = ii < G || ii >= G + b.Nip || jj < G || jj >= G + b.Njp || kk < G || kk >= G + b.Nkp;
-    if (!(ghost || facesMapped)) return;
-    R B[3];
-    cell_bxyz(b, g, conj ? lidx(b, ii, jb, kb) : c, s.mf[fI], s.mf[fIp], s.mf[fs + fJ], s.mf[fs + fJp],
-              s.mf[2 * fs + fK], s.mf[2 * fs + fKp], B);
 #pragma unroll
-    for (int x = 0; x < 3; x++) s.B[x * fs + c] = B[x];
+    for (int d = 0; d < 3; d++)
+        if (fm[d]) s.mf[d * fs + c] = fv[d];
+    if (gm) {
+#pragma unroll
+        for (int v = 0; v < 5; v++) s.Gas[v * fs + c] = gv[v];
+    }
+    if (bm || bnew) {
+#pragma unroll
+        for (int x = 0; x < 3; x++) s.B[x * fs + c] = bm ? bv[x] : B[x];
+    }
 }
 
 // All boundary conditions of one EnforceBCs (+ final bFlux2Fld unless copyB).
-template <class R> void launch_bcs(const Ctx<R>& C, const StateBuf<R>& S, cudaStream_t s, int copyB) {
+// S: the state to fill; cur: the step's start (a failed step's ghosts)
+template <class R>
+void launch_bcs(const Ctx<R>& C, const StateBuf<R>& S, const StateBuf<R>& cur, cudaStream_t s, int copyB) {
     const GamBox& b = C.b;
     const bool iside = C.P.bc[0] == BCK_SPHIN || C.P.bc[0] == BCK_INFLOW || C.P.bc[0] == BCK_ION ||
                        C.P.bc[1] == BCK_WIND || C.P.bc[1] == BCK_ZEROGRAD;
@@ -2848,7 +2909,7 @@ template <class R> void launch_bcs(const Ctx<R>& C, const StateBuf<R>& S, cudaSt
     }
     const Shell sh = make_shell(b);
     const long nsh = sh.nA + sh.nB + sh.nC;
-    k_bc<R><<<(unsigned)((nsh + 255) / 256), 256, 0, s>>>(b, C.P, C.g, S, C.sc, copyB, sh);
+    k_bc<R><<<(unsigned)((nsh + 127) / 128), 128, 0, s>>>(b, C.P, C.g, S, cur, C.sc, copyB, sh);
 }
 
 // CalcDT on a state without changing it (gam_calc_dt): min of CellDT over
@@ -2968,7 +3029,24 @@ template <class R, class F> void for_each_kernel(const Ctx<R>& C, int cur, cudaS
     const StateBuf<R> S = C.st[cur], O = C.st[1 - cur];
     const dim3 blk(32, 4, 1);
     const Range all{0, b.Ni, 0, b.Nj, 0, b.Nk};
-    const Range cells{0, b.Ni - 1, 0, b.Nj - 1, 0, b.Nk - 1};
+    // The update copies State n into the ghosts. Those of a periodic direction are
+    // all filled by the step's boundaries, so there only the one layer that CalcDT
+    // looks at is needed (at 128 x 128 x 4 less than half of the box, at 192^3 91 %;
+    // a step of that small grid 0.161 -> 0.149 ms with this and k_bc's loads).
+    Range cells{0, b.Ni - 1, 0, b.Nj - 1, 0, b.Nk - 1}, faces = all;
+    const int N[3] = {b.Nip, b.Njp, b.Nkp};
+    int* lim[3][4] = {{&cells.i0, &cells.i1, &faces.i0, &faces.i1}, {&cells.j0, &cells.j1, &faces.j0, &faces.j1},
+                      {&cells.k0, &cells.k1, &faces.k0, &faces.k1}};
+    for (int d = 0; d < 3; d++) {
+        if (C.P.bc[2 * d] != BCK_PERIODIC || C.P.bc[2 * d + 1] != BCK_PERIODIC || (d == 2 && C.P.do25D)) continue;
+        // rows start where the box's do: a warp's values lie in whole lines then
+        *lim[d][0] = d == 0 ? 0 : G - 1;
+        *lim[d][1] = G + N[d];
+        if (!C.oomf) {  // ooState takes the fluxes of every face
+            *lim[d][2] = *lim[d][0];
+            *lim[d][3] = G + N[d] + 1;
+        }
+    }
     const int kke = C.P.do25D ? G : G + b.Nkp - 1;  // last active k of the stress sweep
     f(0, [&] { k_step_begin<<<1, 1, 0, s>>>(C.sc); });
     const dim3 pblk(32, 8, 1);
@@ -2980,9 +3058,11 @@ template <class R, class F> void for_each_kernel(const Ctx<R>& C, int cur, cudaS
             k_predict<R, sizeof(R) == 8 ? 3 : 4><<<grid_for(all, pblk), pblk, 0, s>>>(b, C.P, C.g, S, O, C.w, C.sc, nullptr);
     });
     if (C.P.doMHD) {
-        const Range mf[3] = {{0, b.Ni - 1, G, G + b.Njp, 0, b.Nk - 1},
-                             {0, b.Ni - 1, 0, b.Nj - 1, G, G + b.Nkp},
-                             {G, G + b.Nip, 0, b.Nj - 1, 0, b.Nk - 1}};
+        // the faces whose velocities the edges' stencils (along dT2) take (the
+        // ghosts left out: 192^3 strict 375 -> 353 us for the three)
+        const Range mf[3] = {{G, G + b.Nip - 1, G, G + b.Njp, 0, b.Nk - 1},
+                             {0, b.Ni - 1, G, G + b.Njp - 1, G, G + b.Nkp},
+                             {G, G + b.Nip, 0, b.Nj - 1, G, G + b.Nkp - 1}};
         const Range ed[3] = {{G, G + b.Nip - 1, G, G + b.Njp, G, G + b.Nkp},
                              {G, G + b.Nip, G, G + b.Njp - 1, G, G + b.Nkp},
                              {G, G + b.Nip, G, G + b.Njp, G, G + b.Nkp - 1}};
@@ -3041,7 +3121,7 @@ template <class R, class F> void for_each_kernel(const Ctx<R>& C, int cur, cudaS
             const long nf = (long)ni * (b.Njp + 1);
             k_fix_e_lfm<R><<<(unsigned)((nf + 255) / 256), 256, 0, s>>>(b, C.w.E, GAM_NG, GAM_NG + b.Njp, C.sc);
         }
-        k_update_faces<R><<<grid_for(all, blk), blk, 0, s>>>(b, C.P, S, O, C.w, C.sc, C.oomf);
+        k_update_faces<R><<<grid_for(faces, blk), blk, 0, s>>>(b, C.P, S, O, C.w, faces, C.sc, C.oomf);
     });
     f(12, [&] {
         if (C.P.ring.on) {  // RingFlux (stress.F90:137-139), before the fluxes become deltas
@@ -3051,9 +3131,9 @@ template <class R, class F> void for_each_kernel(const Ctx<R>& C, int cur, cudaS
                 k_ion_flux<R><<<16, 32, C.P.ring.Np * sizeof(R), s>>>(b, C.P, C.w, C.sc);
         }
         if (C.P.doBoris)
-            k_update_cells<R, sizeof(R) == 8 ? 6 : 8, true><<<grid_for(cells, blk), blk, 0, s>>>(b, C.P, C.g, S, O, C.w, C.sc, C.gamma, C.gm1, fold);
+            k_update_cells<R, sizeof(R) == 8 ? 6 : 8, true><<<grid_for(cells, blk), blk, 0, s>>>(b, C.P, C.g, S, O, C.w, C.sc, C.gamma, C.gm1, cells, fold);
         else  // strict: 6 blocks/SM (732 us at 192^3; 8: 792, 5: 784, 4: 819); the other forms 8
-            k_update_cells<R, GAM_STRICT_KERNELS ? 6 : 8><<<grid_for(cells, blk), blk, 0, s>>>(b, C.P, C.g, S, O, C.w, C.sc, C.gamma, C.gm1, fold);
+            k_update_cells<R, GAM_STRICT_KERNELS ? 6 : 8><<<grid_for(cells, blk), blk, 0, s>>>(b, C.P, C.g, S, O, C.w, C.sc, C.gamma, C.gm1, cells, fold);
         if (C.P.ring.on) launch_ring_average(C, O, s);  // mhdgroup.F90:69-74
         if (C.P.ion.push) {  // HackStep (PerStep, earthcmi.F90:224-263): PushIon, before CalcDT
             const long np = (long)C.P.ion.nIonP * b.Njp * b.Nkp;
@@ -3079,7 +3159,7 @@ template <class R, class F> void for_each_kernel(const Ctx<R>& C, int cur, cudaS
         }
     });
     if (!fold) f(13, [&] { k_dt_finalize<<<1, 1, 0, s>>>(C.sc); });
-    f(14, [&] { launch_bcs(C, O, s, 0); });
+    f(14, [&] { launch_bcs(C, O, S, s, 0); });
 }
 
 // One step. With side streams (C.aux, C.ev) the independent kernels run as
@@ -3203,7 +3283,7 @@ template <class R> void launch_init(const Ctx<R>& C, int cur, cudaStream_t s) {
     const Range cells{0, b.Ni - 1, 0, b.Nj - 1, 0, b.Nk - 1};
     const StateBuf<R> S = C.st[cur], O = C.st[1 - cur];
     if (C.P.doMHD) k_bfield_all<R><<<grid_for(cells, blk), blk, 0, s>>>(b, C.g, S, C.sc, C.P.ring);
-    launch_bcs(C, S, s, 1);
+    launch_bcs(C, S, S, s, 1);
     cudaMemcpyAsync(O.Gas, S.Gas, 5 * b.fs * sizeof(R), cudaMemcpyDeviceToDevice, s);
     cudaMemcpyAsync(O.mf, S.mf, 3 * b.fs * sizeof(R), cudaMemcpyDeviceToDevice, s);
     cudaMemcpyAsync(O.B, S.B, 3 * b.fs * sizeof(R), cudaMemcpyDeviceToDevice, s);

@@ -1,0 +1,39 @@
+"""The update leaves out the ghosts that the step's periodic boundaries fill: the
+whole box, ghosts included, equals the CPU restatement bit for bit after steps,
+and after a step that failed CalcDT, which stops before its boundaries with the
+ghosts of its start (step.F90:143-153). With AB3 the fluxes of every face move
+on; in 2.5-D the slabs of k are not shrunk."""
+import numpy as np
+import pytest
+
+from mage_b200.gamera import GAM_EDT_BAD, GamError
+from tests.helpers import gpu_from_oracle, make_oracle
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [(16, 4, 4), (24, 9, 12), (40, 17, 1)]
+
+
+@pytest.mark.parametrize("fail", [False, True], ids=["steps", "failed"])
+@pytest.mark.parametrize("ab3", [False, True], ids=["ab2", "ab3"])
+@pytest.mark.parametrize("N", SIZES, ids=["x".join(map(str, n)) for n in SIZES])
+def test_whole_box_matches_oracle(oracle_built, N, ab3, fail):
+    o, _ = make_oracle("ot" if N[2] == 1 else "bw", N, variant="gm", doAB3=ab3)
+    assert o.step(2) == 0
+    kw = {"doAB3": ab3}
+    if fail:  # limDT0 (step.F90:117-121): dt0 recorded 1e5 times the current dt
+        kw["dt0"] = 1.0e5 * o.scalars()["dt"]
+        o.set_scalars(dt0=kw["dt0"])
+    g = gpu_from_oracle(o, strict=True, **kw)
+    if ab3:
+        g.set_oostate(o.array("oomagFlux"), o.scalars()["ootime"])
+    assert o.step(3) == (1 if fail else 0)
+    if fail:
+        with pytest.raises(GamError) as ei:
+            g.step_gamera(3)
+        assert ei.value.code == GAM_EDT_BAD
+    else:
+        g.step_gamera(3)
+    s = g.download_state()
+    for k in ("Gas", "magFlux", "Bxyz"):
+        assert np.array_equal(s[k], o.array(k)), k
