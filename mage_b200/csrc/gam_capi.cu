@@ -106,7 +106,9 @@ struct gam_handle {
     Ctx<double> cd{};
     Ctx<float> cf{};
     GamScalars* sc = nullptr;   // device
-    GamFluxMapSet fmaps;        // tensor maps of the flux kernels
+    GamFluxMapSet fmaps;        // tensor maps of the flux and edge kernels
+    char* slab = nullptr;       // what is left of the last shared allocation (dalloc)
+    size_t slabLeft = 0;
     double* staging = nullptr;  // device, Fortran-layout transfer buffer
     double* partial = nullptr;  // device, reduction partials
     double* dres = nullptr;     // device, reduction results
@@ -139,17 +141,34 @@ static int ion_wind_tables(gam_handle* h);
             return fail(h, GAM_ECUDA, std::string(#call) + ": " + cudaGetErrorString(e_));    \
     } while (0)
 
+// Device memory of the handle. Arrays below the slab size share allocations: a
+// handle has about 70 arrays, and each cudaMalloc and cudaFree costs more than
+// the memory of a small grid's (a 32 x 32 handle: 4.6 -> 1.6 ms to create). Arrays of
+// a quarter of a slab and more keep allocations of their own.
 template <class T> static T* dalloc(gam_handle* h, long n, cudaError_t* e) {
+    constexpr size_t slab = 16u << 20;
+    const size_t bytes = (sizeof(T) * (size_t)n + 511) / 512 * 512;
     void* p = nullptr;
-    *e = cudaMalloc(&p, sizeof(T) * (size_t)n);
-    if (*e == cudaSuccess) {
+    *e = cudaSuccess;
+    if (bytes > h->slabLeft) {
+        const size_t take = bytes < slab / 4 ? slab : bytes;
+        *e = cudaMalloc(&p, take);
+        if (*e != cudaSuccess) return nullptr;
         h->allocs.push_back(p);
-#ifdef GAM_BOUNDS_CHECK
-        cudaMemsetAsync(p, 0xFF, sizeof(T) * (size_t)n, h->s);  // NaN canaries
-#else
-        cudaMemsetAsync(p, 0, sizeof(T) * (size_t)n, h->s);
-#endif
+        if (take > bytes) {  // the rest serves the arrays that follow
+            h->slab = (char*)p + bytes;
+            h->slabLeft = take - bytes;
+        }
+    } else {
+        p = h->slab;
+        h->slab += bytes;
+        h->slabLeft -= bytes;
     }
+#ifdef GAM_BOUNDS_CHECK
+    cudaMemsetAsync(p, 0xFF, sizeof(T) * (size_t)n, h->s);  // NaN canaries
+#else
+    cudaMemsetAsync(p, 0, sizeof(T) * (size_t)n, h->s);
+#endif
     return (T*)p;
 }
 
