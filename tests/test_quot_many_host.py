@@ -1,7 +1,8 @@
 """QuotExact::many and the constructor that takes a ready reciprocal
 (mage_b200/csrc/gam_quot.cuh), compiled for the host: N quotients at once are
 the IEEE quotients bit for bit, also where one operand of the group is out of
-the fast range, zero of either sign, infinite or NaN."""
+the fast range, zero of either sign, infinite or NaN. QuotExact::quick is the IEEE
+quotient or says that it is not."""
 import os
 import shutil
 import subprocess
@@ -39,6 +40,13 @@ int main(int argc, char** argv) {
         if (i % 5 == 0) a[sm(s) % 5] = odd[sm(s) % 8];
         gam::QuotExact(d, 1.0 / d).many<5>(a, q);
         for (int k = 0; k < 5; k++) bad += !same(q[k], a[k] / d);
+        // quick: where it does not turn ok off it is the quotient, and it stays on in the ordinary range
+        for (int k = 0; k < 5; k++) {
+            bool ok = true;
+            const double v = gam::QuotExact(d, 1.0 / d).quick(a[k], ok);
+            bad += ok && !same(v, a[k] / d);
+            bad += !ok && std::fabs(d) > 1e-13 && std::fabs(d) < 1e13 && std::fabs(a[k]) > 1e-13 && std::fabs(a[k]) < 1e13;
+        }
     }
     printf("%ld\n", bad);
     return bad != 0;
