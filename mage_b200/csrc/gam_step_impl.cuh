@@ -1615,8 +1615,10 @@ __device__ __forceinline__ void update_cell(const GamBox& b, const DevParams<R>&
 
 // update_cell for every cell, then the CFL dt of cells in the dt range. Bound by
 // the latency of its ~85 loads per cell: the strict form's branch at each
-// quotient kept the next loads waiting (192^3: 932 -> 732 us with quick
-// quotients and one check at the end; the FMA form, which has none, 625).
+// quotient kept the next loads waiting (192^3: 932 -> 792 us with quick
+// quotients and one check at the end; the FMA form, which has none, 640). Slower:
+// the face values in shared memory by TMA (924 us, FMA 903, FP32 389 against 380),
+// E2Flux in the same kernel (FMA 800 against 641 + 104, FP32 539 against 380 + 75).
 template <class R, int MINB, bool BORIS = false>
 __global__ void __launch_bounds__(128, MINB) k_update_cells(GamBox b, DevParams<R> P, Geo<R> g, StateBuf<R> cur,
                                                       StateBuf<R> nxt, Work<R> w, GamScalars* sc, double gamma_d,
@@ -3132,8 +3134,8 @@ template <class R, class F> void for_each_kernel(const Ctx<R>& C, int cur, cudaS
         }
         if (C.P.doBoris)
             k_update_cells<R, sizeof(R) == 8 ? 6 : 8, true><<<grid_for(cells, blk), blk, 0, s>>>(b, C.P, C.g, S, O, C.w, C.sc, C.gamma, C.gm1, cells, fold);
-        else  // strict: 6 blocks/SM (732 us at 192^3; 8: 792, 5: 784, 4: 819); the other forms 8
-            k_update_cells<R, GAM_STRICT_KERNELS ? 6 : 8><<<grid_for(cells, blk), blk, 0, s>>>(b, C.P, C.g, S, O, C.w, C.sc, C.gamma, C.gm1, cells, fold);
+        else  // strict: 5 blocks/SM (792 us at 192^3; 6: 836; dipole of 1.2e6 cells 158, 6: 171); the other forms 8
+            k_update_cells<R, GAM_STRICT_KERNELS ? 5 : 8><<<grid_for(cells, blk), blk, 0, s>>>(b, C.P, C.g, S, O, C.w, C.sc, C.gamma, C.gm1, cells, fold);
         if (C.P.ring.on) launch_ring_average(C, O, s);  // mhdgroup.F90:69-74
         if (C.P.ion.push) {  // HackStep (PerStep, earthcmi.F90:224-263): PushIon, before CalcDT
             const long np = (long)C.P.ion.nIonP * b.Njp * b.Nkp;
