@@ -1613,6 +1613,14 @@ __device__ __forceinline__ void update_cell(const GamBox& b, const DevParams<R>&
     }
 }
 
+// Whether the ring average or a hook may change cell (ii, jj, .) after the
+// update: its CFL dt is then taken by k_dt_only (grids with rings)
+template <class R> __device__ __forceinline__ bool dt_after_rings(const GamBox& b, const DevParams<R>& P, int ii, int jj) {
+    const int G = GAM_NG;
+    return P.doBoris || (P.ring.doS && jj < G + P.ring.NumR) || (P.ring.doE && jj >= G + b.Njp - P.ring.NumR) ||
+           (P.ion.push && ii < G + P.ion.nIonP) || (P.ion.wind && ii >= G + b.Nip - 1);
+}
+
 // update_cell for every cell, then the CFL dt of cells in the dt range. Bound by
 // the latency of its ~85 loads per cell: the strict form's branch at each
 // quotient kept the next loads waiting (192^3: 932 -> 792 us with quick
@@ -1650,7 +1658,7 @@ __global__ void __launch_bounds__(128, MINB) k_update_cells(GamBox b, DevParams<
                           jj <= G + b.Njp - 1 + P.dtJhi && kk >= G - P.dtKlo &&
                           kk <= G + b.Nkp - 1 + P.dtKhi && !(P.ion.push && active && ii < G + P.ion.nIonP) &&
                           !(P.ion.wind && active && ii == G + b.Nip - 1);
-        if (indt && !sc->fixedTimestep && !P.ring.on) {
+        if (indt && !sc->fixedTimestep && !(P.ring.on && dt_after_rings(b, P, ii, jj))) {
             double Ud[5], Bt[3];
 #pragma unroll
             for (int v = 0; v < 5; v++) Ud[v] = (double)U[v];
@@ -2915,7 +2923,8 @@ void launch_bcs(const Ctx<R>& C, const StateBuf<R>& S, const StateBuf<R>& cur, c
 }
 
 // CalcDT on a state without changing it (gam_calc_dt): min of CellDT over
-// the dt range into sc->dtmin_bits.
+// the dt range into sc->dtmin_bits. As a part of a step (countBad): of the cells
+// that the update left to it.
 template <class R>
 __global__ void __launch_bounds__(128) k_dt_only(GamBox b, DevParams<R> P, Geo<R> g, StateBuf<R> s,
                                                  GamScalars* sc, double gamma_d, double gm1_d, int countBad) {
@@ -2926,7 +2935,8 @@ __global__ void __launch_bounds__(128) k_dt_only(GamBox b, DevParams<R> P, Geo<R
             G + b.Nkp - 1 + P.dtKhi};
     double mydt = HUGE_DT;
     bool bad = false;
-    if (thread_ijk(r, ii, jj, kk) && GAM_BOX_OK(lidx(b, ii, jj, kk), lidx(b, ii, jj, kk), 13)) {
+    if (thread_ijk(r, ii, jj, kk) && !(countBad && !dt_after_rings(b, P, ii, jj)) &&
+        GAM_BOX_OK(lidx(b, ii, jj, kk), lidx(b, ii, jj, kk), 13)) {
         const long fs = b.fs;
         const long c = lidx(b, ii, jj, kk);
         double Ud[5], Bt[3] = {0.0, 0.0, 0.0};
@@ -2986,38 +2996,42 @@ template <class R, int E> void launch_vxb(const Ctx<R>& C, const Range& r, cudaS
     k_vxb<R, E, sizeof(R) == 4 ? 5 : 3><<<gr, T_::NT, sm, s>>>(C.b, C.P, C.g, C.w, r, C.sc, C.fmaps->e[E]);
 }
 
-// RingAverage (ringav.F90:26-75) on the updated state: smoothing EMFs of both
-// poles, PoleE and FixEFieldLFM on them, E2Flux with dt = 1, CleanLoops,
-// bFlux2Fld of the cells around the rings, SmoothGas of both poles
-template <class R> void launch_ring_average(const Ctx<R>& C, const StateBuf<R>& O, cudaStream_t s) {
+// RingAverage (ringav.F90:26-75), its magnetic part on the new fluxes: smoothing
+// EMFs of both poles, PoleE and FixEFieldLFM on them, E2Flux with dt = 1, CleanLoops
+template <class R> void launch_ring_flux_average(const Ctx<R>& C, const StateBuf<R>& O, cudaStream_t s) {
     const GamBox& b = C.b;
     const RingData& Rg = C.P.ring;
     const int G = GAM_NG;
-    if (C.P.doMHD) {
-        const long nz = 2L * (Rg.NumR + 2) * b.Ni * b.Nk;
-        k_ring_zero_e<R><<<(unsigned)((nz + 255) / 256), 256, 0, s>>>(b, Rg, C.sc);
-        const long ne = 2L * (b.Nip + 1) * Rg.NumR;
-        const size_t smE = (size_t)(2 * Rg.Np + Rg.chunkStride / 5) * sizeof(R);
-        k_ring_smooth_e<R><<<(unsigned)ne, RING_NT, smE, s>>>(b, Rg, O, C.sc);
-        R* E = (R*)Rg.smoothE;
-        const int ni = b.Nip + 1;
-        k_ring_pole_e<R><<<(unsigned)(2 * ni), 32, Rg.Np * sizeof(R), s>>>(b, Rg, E, G, G + b.Nip, C.sc);
-        // FixEFieldLFM over the rows that can be nonzero (the others hold zeros)
-        const int sj1 = std::min(G + Rg.NumR + 1, G + b.Njp), ej0 = std::max(G + b.Njp - 1 - Rg.NumR, G);
-        if (Rg.doS)
-            k_fix_e_lfm<R><<<(unsigned)(((long)ni * (sj1 - G + 1) + 255) / 256), 256, 0, s>>>(b, E, G, sj1, C.sc);
-        if (Rg.doE)
-            k_fix_e_lfm<R><<<(unsigned)(((long)ni * (G + b.Njp - ej0 + 1) + 255) / 256), 256, 0, s>>>(
-                b, E, ej0, G + b.Njp, C.sc);
-        const long nf = 2L * (Rg.NumR + 1) * (b.Nip + 1) * (b.Nkp + 1);
-        k_ring_e2flux<R><<<(unsigned)((nf + 255) / 256), 256, 0, s>>>(b, Rg, O, C.sc);
-        if (Rg.clean) k_ring_clean_loops<R><<<(unsigned)(2 * ni), 32, Rg.Np * sizeof(R), s>>>(b, Rg, O, C.sc);
-        const long nb = 2L * (G + Rg.NumR + 2) * b.Ni * b.Nk;
-        k_ring_bfield<R><<<(unsigned)((nb + 127) / 128), 128, 0, s>>>(b, C.g, Rg, O, C.sc);
-    }
-    const long ng = 2L * b.Nip * Rg.NumR;
+    const long nz = 2L * (Rg.NumR + 2) * b.Ni * b.Nk;
+    k_ring_zero_e<R><<<(unsigned)((nz + 255) / 256), 256, 0, s>>>(b, Rg, C.sc);
+    const long ne = 2L * (b.Nip + 1) * Rg.NumR;
+    const size_t smE = (size_t)(2 * Rg.Np + Rg.chunkStride / 5) * sizeof(R);
+    k_ring_smooth_e<R><<<(unsigned)ne, RING_NT, smE, s>>>(b, Rg, O, C.sc);
+    R* E = (R*)Rg.smoothE;
+    const int ni = b.Nip + 1;
+    k_ring_pole_e<R><<<(unsigned)(2 * ni), 32, Rg.Np * sizeof(R), s>>>(b, Rg, E, G, G + b.Nip, C.sc);
+    // FixEFieldLFM over the rows that can be nonzero (the others hold zeros)
+    const int sj1 = std::min(G + Rg.NumR + 1, G + b.Njp), ej0 = std::max(G + b.Njp - 1 - Rg.NumR, G);
+    if (Rg.doS)
+        k_fix_e_lfm<R><<<(unsigned)(((long)ni * (sj1 - G + 1) + 255) / 256), 256, 0, s>>>(b, E, G, sj1, C.sc);
+    if (Rg.doE)
+        k_fix_e_lfm<R><<<(unsigned)(((long)ni * (G + b.Njp - ej0 + 1) + 255) / 256), 256, 0, s>>>(
+            b, E, ej0, G + b.Njp, C.sc);
+    const long nf = 2L * (Rg.NumR + 1) * (b.Nip + 1) * (b.Nkp + 1);
+    k_ring_e2flux<R><<<(unsigned)((nf + 255) / 256), 256, 0, s>>>(b, Rg, O, C.sc);
+    if (Rg.clean) k_ring_clean_loops<R><<<(unsigned)(2 * ni), 32, Rg.Np * sizeof(R), s>>>(b, Rg, O, C.sc);
+}
+// ... bFlux2Fld of the cells around the rings
+template <class R> void launch_ring_field(const Ctx<R>& C, const StateBuf<R>& O, cudaStream_t s) {
+    const long nb = 2L * (GAM_NG + C.P.ring.NumR + 2) * C.b.Ni * C.b.Nk;
+    k_ring_bfield<R><<<(unsigned)((nb + 127) / 128), 128, 0, s>>>(C.b, C.g, C.P.ring, O, C.sc);
+}
+// ... and SmoothGas of both poles on the updated state
+template <class R> void launch_ring_gas_average(const Ctx<R>& C, const StateBuf<R>& O, cudaStream_t s) {
+    const RingData& Rg = C.P.ring;
+    const long ng = 2L * C.b.Nip * Rg.NumR;
     const size_t smG = (size_t)(5 * Rg.Np + Rg.chunkStride) * sizeof(R);
-    k_ring_smooth_gas<R><<<(unsigned)ng, RING_NT, smG, s>>>(b, C.P, O, C.sc);
+    k_ring_smooth_gas<R><<<(unsigned)ng, RING_NT, smG, s>>>(C.b, C.P, O, C.sc);
 }
 
 // The kernels of one stepGamera in order, each handed to f(id, launch) with
@@ -3124,6 +3138,11 @@ template <class R, class F> void for_each_kernel(const Ctx<R>& C, int cur, cudaS
             k_fix_e_lfm<R><<<(unsigned)((nf + 255) / 256), 256, 0, s>>>(b, C.w.E, GAM_NG, GAM_NG + b.Njp, C.sc);
         }
         k_update_faces<R><<<grid_for(faces, blk), blk, 0, s>>>(b, C.P, S, O, C.w, faces, C.sc, C.oomf);
+        // RingAverage's magnetic part takes the new fluxes alone, and only CellBoris
+        // looks at the field before it: here it runs beside the flux sweeps, and the
+        // update finds the averaged fluxes (96 x 96 x 128 cells: 65 us of small launches
+        // beside the sweeps, and the field around the rings formed once, 20 us)
+        if (C.P.ring.on && C.P.doMHD && !C.P.doBoris) launch_ring_flux_average(C, O, s);
     });
     f(12, [&] {
         if (C.P.ring.on) {  // RingFlux (stress.F90:137-139), before the fluxes become deltas
@@ -3136,7 +3155,13 @@ template <class R, class F> void for_each_kernel(const Ctx<R>& C, int cur, cudaS
             k_update_cells<R, sizeof(R) == 8 ? 6 : 8, true><<<grid_for(cells, blk), blk, 0, s>>>(b, C.P, C.g, S, O, C.w, C.sc, C.gamma, C.gm1, cells, fold);
         else  // strict: 5 blocks/SM (792 us at 192^3; 6: 836; dipole of 1.2e6 cells 158, 6: 171); the other forms 8
             k_update_cells<R, GAM_STRICT_KERNELS ? 5 : 8><<<grid_for(cells, blk), blk, 0, s>>>(b, C.P, C.g, S, O, C.w, C.sc, C.gamma, C.gm1, cells, fold);
-        if (C.P.ring.on) launch_ring_average(C, O, s);  // mhdgroup.F90:69-74
+        if (C.P.ring.on) {  // RingAverage (mhdgroup.F90:69-74)
+            if (C.P.doMHD && C.P.doBoris) {
+                launch_ring_flux_average(C, O, s);
+                launch_ring_field(C, O, s);
+            }
+            launch_ring_gas_average(C, O, s);
+        }
         if (C.P.ion.push) {  // HackStep (PerStep, earthcmi.F90:224-263): PushIon, before CalcDT
             const long np = (long)C.P.ion.nIonP * b.Njp * b.Nkp;
             if (C.P.doBoris)
