@@ -2765,27 +2765,27 @@ __device__ __forceinline__ bool shell_ijk(const Shell& sh, unsigned t, int& ii, 
     return false;
 }
 
+__device__ __forceinline__ bool in_range(const Range& r, int ii, int jj, int kk) {
+    return ii >= r.i0 && ii <= r.i1 && jj >= r.j0 && jj <= r.j1 && kk >= r.k0 && kk <= r.k1;
+}
 // A step that failed CalcDT stops before its boundary conditions with the ghosts
 // of its start (the update's copies, mhdgroup.F90:202-256) and their field. The
-// update leaves out the layers that the boundaries fill, so they are copied here.
+// update's ranges uc, uf leave out the layers that the boundaries fill, so those
+// are copied here; the others may hold more than a copy (NudgeSW across the pole).
 template <class R>
 __device__ void failed_ghosts(const GamBox& b, const DevParams<R>& P, const Geo<R>& g, const StateBuf<R>& s,
-                              const StateBuf<R>& cur, int ii, int jj, int kk, bool isCell) {
-    const int G = GAM_NG;
+                              const StateBuf<R>& cur, const Range& uc, const Range& uf, int ii, int jj, int kk,
+                              bool isCell) {
     const long fs = b.fs, c = lidx(b, ii, jj, kk);
-    auto updated = [&](int x, int y, int z) {  // a face in E2Flux's range
-        return P.doMHD && x >= G && x <= G + b.Nip && y >= G && y <= G + b.Njp && z >= G && z <= G + b.Nkp;
-    };
     auto face = [&](int d, int x, int y, int z) {
         const long q = d * fs + lidx(b, x, y, z);
-        return updated(x, y, z) ? s.mf[q] : cur.mf[q];
+        return in_range(uf, x, y, z) ? s.mf[q] : cur.mf[q];
     };
-    if (!updated(ii, jj, kk)) {
+    if (!in_range(uf, ii, jj, kk)) {
 #pragma unroll
         for (int d = 0; d < 3; d++) s.mf[d * fs + c] = cur.mf[d * fs + c];
     }
-    const bool active = ii >= G && ii < G + b.Nip && jj >= G && jj < G + b.Njp && kk >= G && kk < G + b.Nkp;
-    if (!isCell || active) return;
+    if (!isCell || in_range(uc, ii, jj, kk)) return;
 #pragma unroll
     for (int v = 0; v < 5; v++) s.Gas[v * fs + c] = cur.Gas[v * fs + c];
     if (!P.doMHD) return;
@@ -2806,7 +2806,8 @@ __device__ void failed_ghosts(const GamBox& b, const DevParams<R>& P, const Geo<
 // 192^3 takes 170 us.
 template <class R>
 __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 6 : 8)
-    k_bc(GamBox b, DevParams<R> P, Geo<R> g, StateBuf<R> s, StateBuf<R> cur, const GamScalars* sc, int copyB, Shell sh) {
+    k_bc(GamBox b, DevParams<R> P, Geo<R> g, StateBuf<R> s, StateBuf<R> cur, const GamScalars* sc, int copyB, Shell sh,
+         Range uc, Range uf) {
     if (sc->halted && !(sc->fixGhosts && !copyB)) return;
     int ii, jj, kk;
     if (!shell_ijk(sh, blockIdx.x * blockDim.x + threadIdx.x, ii, jj, kk)) return;
@@ -2815,7 +2816,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 6 : 8)
     GAM_BOX_CHECK(c, c, 14);
     const bool isCell = ii < b.Ni && jj < b.Nj && kk < b.Nk;
     if (sc->halted) {
-        failed_ghosts(b, P, g, s, cur, ii, jj, kk, isCell);
+        failed_ghosts(b, P, g, s, cur, uc, uf, ii, jj, kk, isCell);
         return;
     }
     R fv[3], gv[5], bv[3], B[3];
@@ -2897,9 +2898,11 @@ __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 6 : 8)
 }
 
 // All boundary conditions of one EnforceBCs (+ final bFlux2Fld unless copyB).
-// S: the state to fill; cur: the step's start (a failed step's ghosts)
+// S: the state to fill; cur: the step's start, uc and uf: the cells and faces that
+// the update wrote (a failed step's ghosts)
 template <class R>
-void launch_bcs(const Ctx<R>& C, const StateBuf<R>& S, const StateBuf<R>& cur, cudaStream_t s, int copyB) {
+void launch_bcs(const Ctx<R>& C, const StateBuf<R>& S, const StateBuf<R>& cur, const Range& uc, const Range& uf,
+                cudaStream_t s, int copyB) {
     const GamBox& b = C.b;
     const bool iside = C.P.bc[0] == BCK_SPHIN || C.P.bc[0] == BCK_INFLOW || C.P.bc[0] == BCK_ION ||
                        C.P.bc[1] == BCK_WIND || C.P.bc[1] == BCK_ZEROGRAD;
@@ -2919,7 +2922,7 @@ void launch_bcs(const Ctx<R>& C, const StateBuf<R>& S, const StateBuf<R>& cur, c
     }
     const Shell sh = make_shell(b);
     const long nsh = sh.nA + sh.nB + sh.nC;
-    k_bc<R><<<(unsigned)((nsh + 127) / 128), 128, 0, s>>>(b, C.P, C.g, S, cur, C.sc, copyB, sh);
+    k_bc<R><<<(unsigned)((nsh + 127) / 128), 128, 0, s>>>(b, C.P, C.g, S, cur, C.sc, copyB, sh, uc, uf);
 }
 
 // CalcDT on a state without changing it (gam_calc_dt): min of CellDT over
@@ -3186,7 +3189,7 @@ template <class R, class F> void for_each_kernel(const Ctx<R>& C, int cur, cudaS
         }
     });
     if (!fold) f(13, [&] { k_dt_finalize<<<1, 1, 0, s>>>(C.sc); });
-    f(14, [&] { launch_bcs(C, O, S, s, 0); });
+    f(14, [&] { launch_bcs(C, O, S, cells, faces, s, 0); });
 }
 
 // One step. With side streams (C.aux, C.ev) the independent kernels run as
@@ -3310,7 +3313,7 @@ template <class R> void launch_init(const Ctx<R>& C, int cur, cudaStream_t s) {
     const Range cells{0, b.Ni - 1, 0, b.Nj - 1, 0, b.Nk - 1};
     const StateBuf<R> S = C.st[cur], O = C.st[1 - cur];
     if (C.P.doMHD) k_bfield_all<R><<<grid_for(cells, blk), blk, 0, s>>>(b, C.g, S, C.sc, C.P.ring);
-    launch_bcs(C, S, S, s, 1);
+    launch_bcs(C, S, S, cells, all, s, 1);
     cudaMemcpyAsync(O.Gas, S.Gas, 5 * b.fs * sizeof(R), cudaMemcpyDeviceToDevice, s);
     cudaMemcpyAsync(O.mf, S.mf, 3 * b.fs * sizeof(R), cudaMemcpyDeviceToDevice, s);
     cudaMemcpyAsync(O.B, S.B, 3 * b.fs * sizeof(R), cudaMemcpyDeviceToDevice, s);
