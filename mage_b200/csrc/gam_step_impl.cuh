@@ -2828,8 +2828,12 @@ __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 6 : 8)
         const int sg = bc_source(b, P, d, false, x, y, z);
         GAM_BOX_CHECK(lidx(b, x, y, z), lidx(b, x, y, z), 14);
         fm[d] = x != ii || y != jj || z != kk;
+        // a source that the update left out belongs to no face (it lies past the last
+        // cell across d): it has the value of the step's start, also in its own place
+        const bool left = !in_range(uf, x, y, z);
+        fm[d] = fm[d] || left;
         if (fm[d]) {
-            fv[d] = s.mf[d * fs + lidx(b, x, y, z)];
+            fv[d] = (left ? cur.mf : s.mf)[d * fs + lidx(b, x, y, z)];
             if (sg < 0) fv[d] = -fv[d];
         }
     }

@@ -37,3 +37,27 @@ def test_whole_box_matches_oracle(oracle_built, N, ab3, fail):
     s = g.download_state()
     for k in ("Gas", "magFlux", "Bxyz"):
         assert np.array_equal(s[k], o.array(k)), k
+
+
+@pytest.mark.parametrize("ab3", [False, True], ids=["ab2", "ab3"])
+@pytest.mark.parametrize("N", SIZES, ids=["x".join(map(str, n)) for n in SIZES])
+def test_slots_past_the_last_cell(oracle_built, N, ab3):
+    """magFlux has a layer past the last cell across each component's direction that
+    no face is in: what State has there stays, whatever oState has."""
+    o, _ = make_oracle("ot" if N[2] == 1 else "bw", N, variant="gm", doAB3=ab3)
+    for n, name in enumerate(("magFlux", "omagFlux")):
+        for d in range(3):
+            for a in range(3):
+                if a != d:
+                    sl = [slice(None)] * 3
+                    sl[2 - a] = -1
+                    o.array(name)[d][tuple(sl)] = 1.0 + n + 0.1 * d + 0.01 * a
+    g = gpu_from_oracle(o, strict=True, doAB3=ab3)
+    if ab3:
+        g.set_oostate(o.array("oomagFlux"), o.scalars()["ootime"])
+    for n in (1, 2):
+        assert o.step(n) == 0
+        g.step_gamera(n)
+        s = g.download_state()
+        for k in ("Gas", "magFlux", "Bxyz"):
+            assert np.array_equal(s[k], o.array(k)), (n, k)
