@@ -1403,6 +1403,26 @@ __device__ __forceinline__ void finalize_dt(GamScalars* sc) {
     sc->ootime = sc->otime;        // CopyState(oState, ooState) (mhdgroup.F90:100-102)
     sc->otime = sc->time;          // CopyState (mhdgroup.F90:255)
     sc->time = sc->time + sc->dt;  // mhdgroup.F90:106
+// magFlux has slots in the last layer of each direction that no face is in. The
+// update copies State's to the new buffer only where it copies the ghosts, so after
+// an upload they are copied here once, and both buffers hold State's from then on.
+template <class R>
+__global__ void __launch_bounds__(128) k_last_slots(GamBox b, StateBuf<R> cur, StateBuf<R> nxt, const GamScalars* sc) {
+    if (sc->halted) return;
+    long t = blockIdx.x * (long)blockDim.x + threadIdx.x, c;
+    if (t < b.sk) {
+        c = t + b.sk * b.Nk;
+    } else if ((t -= b.sk) < (long)b.sx * b.Nk) {
+        c = t % b.sx + (long)b.sx * b.Nj + b.sk * (t / b.sx);
+    } else if ((t -= (long)b.sx * b.Nk) < (long)b.Nj * b.Nk) {
+        c = b.Ni + b.sx * (t % b.Nj) + b.sk * (t / b.Nj);
+    } else {
+        return;
+    }
+    GAM_BOX_CHECK(c, c, 14);
+#pragma unroll
+    for (int d = 0; d < 3; d++) nxt.mf[d * b.fs + c] = cur.mf[d * b.fs + c];
+}
     sc->ts = sc->ts + 1;
     sc->t = sc->t + sc->dt;
     if (sc->fixedTimestep) {
@@ -2828,12 +2848,8 @@ __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 6 : 8)
         const int sg = bc_source(b, P, d, false, x, y, z);
         GAM_BOX_CHECK(lidx(b, x, y, z), lidx(b, x, y, z), 14);
         fm[d] = x != ii || y != jj || z != kk;
-        // a source that the update left out belongs to no face (it lies past the last
-        // cell across d): it has the value of the step's start, also in its own place
-        const bool left = !in_range(uf, x, y, z);
-        fm[d] = fm[d] || left;
         if (fm[d]) {
-            fv[d] = (left ? cur.mf : s.mf)[d * fs + lidx(b, x, y, z)];
+            fv[d] = s.mf[d * fs + lidx(b, x, y, z)];
             if (sg < 0) fv[d] = -fv[d];
         }
     }
@@ -3249,8 +3265,15 @@ template <class R> void launch_step(const Ctx<R>& C, int cur, cudaStream_t s) {
         L();
     }, fold);
 }
-// the scalars of the first step after the host may have set some
-template <class R> void launch_begin(const Ctx<R>& C, cudaStream_t s) { k_step_begin<<<1, 1, 0, s>>>(C.sc); }
+// Before the first step of a call: the scalars, which the host may have set, and
+// (slots) the last layers of the other state buffer
+template <class R> void launch_begin(const Ctx<R>& C, int cur, bool slots, cudaStream_t s) {
+    const GamBox& b = C.b;
+    k_step_begin<<<1, 1, 0, s>>>(C.sc);
+    if (!slots || C.oomf) return;  // with ooState the update copies every face
+    const long n = b.sk + (long)b.sx * b.Nk + (long)b.Nj * b.Nk;
+    k_last_slots<R><<<(unsigned)((n + 127) / 128), 128, 0, s>>>(b, C.st[cur], C.st[1 - cur], C.sc);
+}
 
 // Device time of each kernel of a step (ms, average of reps back-to-back
 // launches; ms[15]). The kernels after k_step_begin read their inputs and

@@ -61,3 +61,5 @@ def test_slots_past_the_last_cell(oracle_built, N, ab3):
         s = g.download_state()
         for k in ("Gas", "magFlux", "Bxyz"):
             assert np.array_equal(s[k], o.array(k)), (n, k)
+        if ab3:
+            assert np.array_equal(g.get_oostate()["oomagFlux"], o.array("oomagFlux")), n
