@@ -1396,6 +1396,32 @@ __device__ __forceinline__ void step_scalars(GamScalars* sc) {
     sc->rodt = 1.0 / sc->odt;
     sc->rdt = 1.0 / sc->dt;
 }
+// magFlux has slots in the last layer across each component's direction that no
+// face is in. The update copies State's to the new buffer only where it copies the
+// ghosts, so after an upload they are copied here once, and both buffers hold
+// State's from then on.
+template <class R>
+__global__ void __launch_bounds__(128) k_last_slots(GamBox b, StateBuf<R> cur, StateBuf<R> nxt, const GamScalars* sc) {
+    if (sc->halted) return;
+    long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    const long nI = b.Ni + 1, nK = nI * (b.Nj + 1), nJ = nI * b.Nk;  // the last layers of K, J and I
+    int ii, jj, kk;
+    if (t < nK) {
+        ii = (int)(t % nI), jj = (int)(t / nI), kk = b.Nk;
+    } else if ((t -= nK) < nJ) {
+        ii = (int)(t % nI), jj = b.Nj, kk = (int)(t / nI);
+    } else if ((t -= nJ) < (long)b.Nj * b.Nk) {
+        ii = b.Ni, jj = (int)(t % b.Nj), kk = (int)(t / b.Nj);
+    } else {
+        return;
+    }
+    const long c = lidx(b, ii, jj, kk);
+    GAM_BOX_CHECK(c, c, 14);
+    const bool last[3] = {ii == b.Ni, jj == b.Nj, kk == b.Nk};
+#pragma unroll
+    for (int d = 0; d < 3; d++)
+        if (last[(d + 1) % 3] || last[(d + 2) % 3]) nxt.mf[d * b.fs + c] = cur.mf[d * b.fs + c];
+}
 // The end of a step: time bookkeeping and CalcDT's checks (gamapp.F90:110-111,
 // step.F90:58-168), by one thread; then the scalars of the next step
 __device__ __forceinline__ void finalize_dt(GamScalars* sc) {
@@ -1403,26 +1429,6 @@ __device__ __forceinline__ void finalize_dt(GamScalars* sc) {
     sc->ootime = sc->otime;        // CopyState(oState, ooState) (mhdgroup.F90:100-102)
     sc->otime = sc->time;          // CopyState (mhdgroup.F90:255)
     sc->time = sc->time + sc->dt;  // mhdgroup.F90:106
-// magFlux has slots in the last layer of each direction that no face is in. The
-// update copies State's to the new buffer only where it copies the ghosts, so after
-// an upload they are copied here once, and both buffers hold State's from then on.
-template <class R>
-__global__ void __launch_bounds__(128) k_last_slots(GamBox b, StateBuf<R> cur, StateBuf<R> nxt, const GamScalars* sc) {
-    if (sc->halted) return;
-    long t = blockIdx.x * (long)blockDim.x + threadIdx.x, c;
-    if (t < b.sk) {
-        c = t + b.sk * b.Nk;
-    } else if ((t -= b.sk) < (long)b.sx * b.Nk) {
-        c = t % b.sx + (long)b.sx * b.Nj + b.sk * (t / b.sx);
-    } else if ((t -= (long)b.sx * b.Nk) < (long)b.Nj * b.Nk) {
-        c = b.Ni + b.sx * (t % b.Nj) + b.sk * (t / b.Nj);
-    } else {
-        return;
-    }
-    GAM_BOX_CHECK(c, c, 14);
-#pragma unroll
-    for (int d = 0; d < 3; d++) nxt.mf[d * b.fs + c] = cur.mf[d * b.fs + c];
-}
     sc->ts = sc->ts + 1;
     sc->t = sc->t + sc->dt;
     if (sc->fixedTimestep) {
@@ -3271,7 +3277,7 @@ template <class R> void launch_begin(const Ctx<R>& C, int cur, bool slots, cudaS
     const GamBox& b = C.b;
     k_step_begin<<<1, 1, 0, s>>>(C.sc);
     if (!slots || C.oomf) return;  // with ooState the update copies every face
-    const long n = b.sk + (long)b.sx * b.Nk + (long)b.Nj * b.Nk;
+    const long n = (b.Ni + 1L) * (b.Nj + 1 + b.Nk) + (long)b.Nj * b.Nk;
     k_last_slots<R><<<(unsigned)((n + 127) / 128), 128, 0, s>>>(b, C.st[cur], C.st[1 - cur], C.sc);
 }
 
