@@ -607,11 +607,12 @@ __global__ void __launch_bounds__(EdgeTile<E>::NT, MINB)
     m.fA1 = edge_area(b, g, c, dT1, dT2);
     m.fA2 = edge_area(b, g, c, dT2, dT1);
     m.detT = (R)1 / (m.xni * m.ynj - m.xnj * m.yni);
-    const Quot<R> qA1(m.fA1), qA2(m.fA2), qdt((R)sc->dt);
+    const R dt = (R)sc->dt;
+    const Quot<R> qA1(m.fA1), qA2(m.fA2), qdt(dt);
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     if (!in) return;
-    edge_emf<R, E, true>(b, P, g, w, c, sm, tx, ty, tz, m, qA1, qA2, qdt);
+    edge_emf<R, E, true>(b, P, g, w, c, sm, tx, ty, tz, m, qA1, qA2, qdt, dt);
 }
 template <class R, int E>
 void launch_vxb_box(const GamBox& b, const DevParams<R>& P, const Geo<R>& g, const Work<R>& w, const Range& r,

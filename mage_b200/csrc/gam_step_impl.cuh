@@ -110,18 +110,25 @@ template <> struct Mth<float> {
 // Quot1 is the same for a divisor with a single numerator, where QuotExact
 // would cost more than the division it replaces.
 // many<N> takes N numerators at once (one range check for all of them). The
-// two-argument form takes the divisor's rounded reciprocal from a table.
+// two-argument form takes the divisor's rounded reciprocal from a table. close is
+// rounded like a division in every form: where only the reciprocal is kept, the
+// product gets the correction by its exact remainder (gam_quot.cuh).
 template <class R> struct Quot {
 #ifdef GAM_FAST_RECIP
     R r;
     __device__ __forceinline__ explicit Quot(R d) : r((R)1 / d) {}
     __device__ __forceinline__ Quot(R, R rd) : r(rd) {}
     __device__ __forceinline__ R operator()(R a) const { return a * r; }
+    __device__ __forceinline__ R close(R a, R d) const {
+        const R q = a * r, e = fma(-d, q, a);
+        return e - e == (R)0 ? fma(e, r, q) : q;  // an infinite quotient stays infinite
+    }
 #else
     R d;
     __device__ __forceinline__ explicit Quot(R dd) : d(dd) {}
     __device__ __forceinline__ Quot(R dd, R) : d(dd) {}
     __device__ __forceinline__ R operator()(R a) const { return a / d; }
+    __device__ __forceinline__ R close(R a, R) const { return a / d; }
 #endif
     template <int N> __device__ __forceinline__ void many(const R* a, R* o) const {
 #pragma unroll
@@ -134,6 +141,7 @@ template <> struct Quot<double> {
     __device__ __forceinline__ explicit Quot(double d) : q(d) {}
     __device__ __forceinline__ Quot(double d, double rd) : q(d, rd) {}
     __device__ __forceinline__ double operator()(double a) const { return q(a); }
+    __device__ __forceinline__ double close(double a, double) const { return q(a); }
     template <int N> __device__ __forceinline__ void many(const double* a, double* o) const { q.many<N>(a, o); }
 };
 #endif
@@ -180,18 +188,12 @@ template <class R> struct Quot1 {
 #endif
 };
 
-// a/(gamma - 1) with the reciprocal from the parameters. The forms that multiply
-// by reciprocals add the correction of a division here: pressure and internal
-// energy go through gamma - 1 and back every step, and a rounded reciprocal
-// would pull the energy the same way each time (FP32: 5e-7 instead of 2e-7 off
-// after 20 steps).
+// a/(gamma - 1) with the reciprocal from the parameters, rounded like a division
+// in every form: pressure and internal energy go through gamma - 1 and back every
+// step, and a rounded reciprocal would pull the energy the same way each time
+// (FP32: 5e-7 instead of 2e-7 off after 20 steps).
 template <class R> __device__ __forceinline__ R over_gm1(const DevParams<R>& P, R a) {
-#ifdef GAM_FAST_RECIP
-    const R q = a * P.rgm1, r = fma(-P.gm1, q, a);
-    return r == r ? fma(r, P.rgm1, q) : q;  // an infinite a stays infinite
-#else
-    return Quot<R>(P.gm1, P.rgm1)(a);
-#endif
+    return Quot<R>(P.gm1, P.rgm1).close(a, P.gm1);
 }
 template <class R, bool EXACT> __device__ __forceinline__ R over_gm1(const DevParams<R>& P, R a, bool& ok) {
 #ifdef GAM_FAST_RECIP
@@ -618,7 +620,11 @@ __device__ __forceinline__ void predict_at(const GamBox& b, const DevParams<R>& 
             const R bh = qAm(hm[d], ok);
             w.abh[d * fs + c] = A * bh;
             // the area itself divides Bnf: the same quotient, but for areas below TINY
+#ifdef GAM_FAST_RECIP
+            w.Bnf[d * fs + c] = Am == A ? qAm.close(hm[d], A) : qdiv(hm[d], A);
+#else
             w.Bnf[d * fs + c] = Am == A ? bh : qdiv(hm[d], A);
+#endif
             w.bn[d * fs + c] = P.doLFMLim ? qAm(fQ[d], ok) : bh;
         }
     }
@@ -862,7 +868,7 @@ template <class R> struct EdgeMetric {
 template <class R, int E, bool SAVE>
 __device__ __forceinline__ void edge_emf(const GamBox& b, const DevParams<R>& P, const Geo<R>& g, const Work<R>& w,
                                          long c, const R* sm, int tx, int ty, int tz, const EdgeMetric<R>& m,
-                                         const Quot<R>& qA1, const Quot<R>& qA2, const Quot<R>& qdt) {
+                                         const Quot<R>& qA1, const Quot<R>& qA2, const Quot<R>& qdt, R dt) {
     using T_ = EdgeTile<E>;
     constexpr int eD = E, dT1 = T_::d1, dT2 = T_::d2;
     const long fs = b.fs;
@@ -937,7 +943,9 @@ __device__ __forceinline__ void edge_emf(const GamBox& b, const DevParams<R>& P,
     R vA = qdiv(Mth<R>::sqrt_(b1 * b1 + b2 * b2), Mth<R>::sqrt_(Dc));
     if (P.doBoris) vA = boris_speed((R)P.Ca, vA);
     vDiff = vDiff + vA;
-    vDiff = rmin(vDiff, qdt(P.CFL * m.edge));
+    // FP32 divides: 192^3, the I edges 150 us, 156 with the corrected product
+    const R vMax = sizeof(R) == 4 ? P.CFL * m.edge / dt : qdt.close(P.CFL * m.edge, dt);
+    vDiff = rmin(vDiff, vMax);
     R e = -(v1 * b2 - v2 * b1) + P.Vd0 * vDiff * Jd;
     w.E[eD * fs + c] = e * m.edge;
     if (SAVE && w.esv) {
@@ -1037,7 +1045,8 @@ __global__ void __launch_bounds__(EdgeTile<E>::NT, MINB)
     m.fA1 = g.fae[(2 * eD) * fs + c];
     m.fA2 = g.fae[(2 * eD + 1) * fs + c];
 #endif
-    const Quot<R> qA1(m.fA1, m.rA1), qA2(m.fA2, g.rfae[(2 * eD + 1) * fs + c]), qdt((R)sc->dt, (R)sc->rdt);
+    const R dt = (R)sc->dt;
+    const Quot<R> qA1(m.fA1, m.rA1), qA2(m.fA2, g.rfae[(2 * eD + 1) * fs + c]), qdt(dt, (R)sc->rdt);
     m.detT = g.rdet[eD * fs + c];
     m.edge = g.edge[eD * fs + c];
     __syncthreads();  // the barrier's initialisation
@@ -1052,7 +1061,7 @@ __global__ void __launch_bounds__(EdgeTile<E>::NT, MINB)
         [[maybe_unused]] const long lo = c - sA - sB < c - 4 * sM ? c - sA - sB : c - 4 * sM;
         GAM_BOX_CHECK(lo, c + 3 * sM, 3 + 2 * eD);
     }
-    edge_emf<R, E, false>(b, P, g, w, c, sm, tx, ty, tz, m, qA1, qA2, qdt);
+    edge_emf<R, E, false>(b, P, g, w, c, sm, tx, ty, tz, m, qA1, qA2, qdt, dt);
 }
 
 #endif  // GAM_GEO_TABLES
@@ -1497,7 +1506,7 @@ __device__ __forceinline__ double cell_dt(const DevParams<R>& P, const double* U
     double ke = 0.5 * rho * (MagV * MagV);
     double e = U[4] - ke;
     double Pr = gm1 * e;
-    double Cs = sqrt(qr(gamma * Pr));
+    double Cs = sqrt(qr.close(gamma * Pr, rho));
     double Valf = 0.0;
     if (P.doMHD) {
         double MagB = sqrt(Bt[0] * Bt[0] + Bt[1] * Bt[1] + Bt[2] * Bt[2]);
