@@ -11,6 +11,7 @@
 #include <vector>
 #include "../../include/gamgpu.h"
 #include "gam_layout.cuh"
+#include "gam_slab.h"
 #include "gam_types.cuh"
 
 // variant launchers (gam_step_strict.cu, gam_step_fast.cu)
@@ -107,8 +108,7 @@ struct gam_handle {
     Ctx<float> cf{};
     GamScalars* sc = nullptr;   // device
     GamFluxMapSet fmaps;        // tensor maps of the flux and edge kernels
-    char* slab = nullptr;       // what is left of the last shared allocation (dalloc)
-    size_t slabLeft = 0;
+    GamSlab slab;               // the small arrays' shared allocations (dalloc)
     double* staging = nullptr;  // device, Fortran-layout transfer buffer
     double* partial = nullptr;  // device, reduction partials
     double* dres = nullptr;     // device, reduction results
@@ -142,29 +142,16 @@ static int ion_wind_tables(gam_handle* h);
             return fail(h, GAM_ECUDA, std::string(#call) + ": " + cudaGetErrorString(e_));    \
     } while (0)
 
-// Device memory of the handle. Arrays below the slab size share allocations: a
+// Device memory of the handle, the small arrays out of shared allocations: a
 // handle has about 70 arrays, and each cudaMalloc and cudaFree costs more than
-// the memory of a small grid's (a 32 x 32 handle: 4.6 -> 1.6 ms to create). Arrays of
-// a quarter of a slab and more keep allocations of their own.
+// the memory of a small grid's (a 32 x 32 handle: 4.6 -> 1.6 ms to create).
 template <class T> static T* dalloc(gam_handle* h, long n, cudaError_t* e) {
-    constexpr size_t slab = 16u << 20;
-    const size_t bytes = (sizeof(T) * (size_t)n + 511) / 512 * 512;
-    void* p = nullptr;
-    *e = cudaSuccess;
-    if (bytes > h->slabLeft) {
-        const size_t take = bytes < slab / 4 ? slab : bytes;
-        *e = cudaMalloc(&p, take);
-        if (*e != cudaSuccess) return nullptr;
-        h->allocs.push_back(p);
-        if (take > bytes) {  // the rest serves the arrays that follow
-            h->slab = (char*)p + bytes;
-            h->slabLeft = take - bytes;
-        }
-    } else {
-        p = h->slab;
-        h->slab += bytes;
-        h->slabLeft -= bytes;
-    }
+    void* p = h->slab.take(sizeof(T) * (size_t)n, *e, [h](void** q, size_t bytes) {
+        const cudaError_t rc = cudaMalloc(q, bytes);
+        if (rc == cudaSuccess) h->allocs.push_back(*q);
+        return rc;
+    });
+    if (!p) return nullptr;
 #ifdef GAM_BOUNDS_CHECK
     cudaMemsetAsync(p, 0xFF, sizeof(T) * (size_t)n, h->s);  // NaN canaries
 #else
