@@ -10,6 +10,7 @@
 #include <string>
 #include <vector>
 #include "../../include/gamgpu.h"
+#include "gam_entry.h"
 #include "gam_layout.cuh"
 #include "gam_slab.h"
 #include "gam_types.cuh"
@@ -208,14 +209,15 @@ static bool encode_box(const GamBox& b, const R* base, int nc, int bx, int by, i
     typedef CUresult (*Encode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    static void* const f = [] {  // the driver's entry point, the same for every handle
+    static GamEntry entry;  // the same for every handle
+    void* const f = entry.get([] {
         void* p = nullptr;
         cudaDriverEntryPointQueryResult q;
         return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
                        q == cudaDriverEntryPointSuccess
                    ? p
                    : nullptr;
-    }();
+    });
     if (!f) return false;
     const cuuint64_t dim[4] = {(cuuint64_t)b.sx, (cuuint64_t)(b.Nj + 1), (cuuint64_t)(b.Nk + 1), (cuuint64_t)nc};
     const cuuint64_t str[3] = {b.sx * sizeof(R), b.sk * sizeof(R), b.fs * sizeof(R)};
