@@ -441,6 +441,8 @@ extern "C" int gam_create(const gam_params* p, gam_handle** out) {
     // test hook: a smaller index limit than the box makes the checks fire on
     // in-bounds indices, so the reporting path can be exercised safely
     if (const char* lim = getenv("GAM_BOUNDS_LIMIT")) s0.oobLimit = atoll(lim);
+    // test hook: a step's waits for its copies run out
+    if (getenv("GAM_COPY_STALL")) s0.copyStall = 16;
 #endif
     if (cudaMemcpyAsync(h->sc, &s0, sizeof(s0), cudaMemcpyHostToDevice, h->s) != cudaSuccess ||
         cudaStreamSynchronize(h->s) != cudaSuccess)
@@ -731,7 +733,7 @@ static int set_scalars(gam_handle* h, double time, double otime, double dt, int3
     CK(h, cudaStreamSynchronize(h->s));
     s.time = time; s.otime = otime; s.t = time; s.dt = dt; s.ts = ts;
     if (!keepOO) s.ootime = otime - dt;
-    s.status = 0; s.halted = 0; s.nbad = 0; s.fixGhosts = 0;
+    s.status = 0; s.halted = 0; s.nbad = 0; s.fixGhosts = 0; s.copyFailed = 0;
     double hugedt = 1.0e12;
     memcpy(&s.dtmin_bits, &hugedt, 8);
     CK(h, cudaMemcpyAsync(h->sc, &s, sizeof(s), cudaMemcpyHostToDevice, h->s));
@@ -880,6 +882,16 @@ static int check_bounds(gam_handle* h, const GamScalars& s) {
     return GAM_OK;
 }
 
+// The code and message of a step that stopped (s.halted); earlier: in a call before
+static int step_failure(gam_handle* h, const GamScalars& s, bool earlier) {
+    if (s.status == 6)
+        return fail(h, GAM_ECUDA, earlier ? "a previous step's copy to shared memory did not complete; upload a state"
+                                          : "a step's copy to shared memory did not complete");
+    const int code = s.status == 5 ? GAM_EDT_DISASTER : GAM_EDT_BAD;
+    if (earlier) return fail(h, code, "a previous step failed CalcDT; upload a state");
+    return fail(h, code, s.status == 5 ? "CalcDT: timestep too small or not finite" : "CalcDT: timestep dropped 10x or below limDT0");
+}
+
 extern "C" int gam_bounds_status(gam_handle* h, int32_t* fired, int32_t* kernel, int64_t* index) {
     if (!h || !fired) return GAM_EINVAL;
 #ifdef GAM_BOUNDS_CHECK
@@ -921,8 +933,7 @@ extern "C" int gam_step(gam_handle* h, int32_t nsteps, double* dt, double* t) {
     GamScalars s;
     CK(h, cudaMemcpyAsync(&s, h->sc, sizeof(s), cudaMemcpyDeviceToHost, h->s));
     CK(h, cudaStreamSynchronize(h->s));
-    if (s.halted)
-        return fail(h, s.status == 5 ? GAM_EDT_DISASTER : GAM_EDT_BAD, "a previous step failed CalcDT; upload a state");
+    if (s.halted) return step_failure(h, s, true);
     const int ts0 = s.ts, cur0 = h->cur;
     // host-side range with the reference's priority clock label (gamapp.F90:96-99)
     nvtxRangePushA("Gamera");
@@ -942,9 +953,7 @@ extern "C" int gam_step(gam_handle* h, int32_t nsteps, double* dt, double* t) {
     if (dt) *dt = s.dt;
     if (t) *t = s.t;
     if (int rcb = check_bounds(h, s)) return rcb;
-    if (s.halted)
-        return fail(h, s.status == 5 ? GAM_EDT_DISASTER : GAM_EDT_BAD,
-                    s.status == 5 ? "CalcDT: timestep too small or not finite" : "CalcDT: timestep dropped 10x or below limDT0");
+    if (s.halted) return step_failure(h, s, false);
     return GAM_OK;
 }
 
@@ -1847,7 +1856,7 @@ extern "C" int gam_step_begin(gam_handle* h) {
     GamScalars s;
     CK(h, cudaMemcpyAsync(&s, h->sc, sizeof(s), cudaMemcpyDeviceToHost, h->s));
     CK(h, cudaStreamSynchronize(h->s));
-    if (s.halted) return fail(h, s.status == 5 ? GAM_EDT_DISASTER : GAM_EDT_BAD, "a previous step failed CalcDT");
+    if (s.halted) return step_failure(h, s, true);
     if ((rc = ensure_phase_graph(h, h->cur, 0))) return rc;
     if ((rc = ensure_phase_graph(h, h->cur, 1))) return rc;
     CK(h, cudaEventRecord(h->ev0, h->s));
@@ -1886,9 +1895,7 @@ extern "C" int gam_step_end(gam_handle* h, uint64_t dtmin_bits, int32_t nbad, do
     if (dt) *dt = s.dt;
     if (t) *t = s.t;
     if (int rcb = check_bounds(h, s)) return rcb;
-    if (s.halted)
-        return fail(h, s.status == 5 ? GAM_EDT_DISASTER : GAM_EDT_BAD,
-                    s.status == 5 ? "CalcDT: timestep too small or not finite" : "CalcDT: timestep dropped 10x or below limDT0");
+    if (s.halted) return step_failure(h, s, false);
     return GAM_OK;
 }
 
@@ -1957,9 +1964,7 @@ extern "C" int gam_step_status(gam_handle* h, double* dt, double* t) {
     if (dt) *dt = s.dt;
     if (t) *t = s.t;
     if (int rcb = check_bounds(h, s)) return rcb;
-    if (s.halted)
-        return fail(h, s.status == 5 ? GAM_EDT_DISASTER : GAM_EDT_BAD,
-                    s.status == 5 ? "CalcDT: timestep too small or not finite" : "CalcDT: timestep dropped 10x or below limDT0");
+    if (s.halted) return step_failure(h, s, false);
     return GAM_OK;
 }
 

@@ -47,10 +47,11 @@ struct GamScalars {
     double rodt, rdt;                  // 1/odt and 1/dt, rounded
     unsigned long long dtmin_bits;     // running min of the cell dt (bits of a positive double)
     int ts;
-    int status;                        // 0 ok, 4 dt bad, 5 dt disaster
+    int status;                        // 0 ok, 4 dt bad, 5 dt disaster, 6 a copy to shared memory did not complete
     int halted;                        // set once a step failed; later kernels return at once
     int fixedTimestep;
     int nbad;                          // cells whose dt is not a finite positive number
+    int copyFailed;                    // a wait for such a copy ran out in this step
     int fixGhosts;                     // the step just failed: its boundary kernel copies the ghosts of its start
     unsigned done;                     // blocks of the cell update that are through (0 between steps)
     double ootime, oodt;               // ooState time and oState - ooState spacing (doAB3)
@@ -59,4 +60,5 @@ struct GamScalars {
     int oobKernel;                     // for_each_kernel id (15: halo, 16: other)
     long long oobIndex;                // the offending linear box index
     long long oobLimit;                // indices must be < this (0: the box size)
+    unsigned copyStall;                // bytes that the flux and edge kernels wait for in vain (a multiple of 16; tests)
 };

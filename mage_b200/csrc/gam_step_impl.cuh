@@ -981,10 +981,16 @@ __device__ __forceinline__ void tma_load(void* dst, const CUtensorMap* map, int 
         "[%6];" ::"r"(smem_u32(dst)), "l"(map), "r"(i), "r"(j), "r"(k), "r"(comp), "r"(smem_u32(bar))
         : "memory");
 }
-// Wait for the first phase; false when it does not complete within the limit
-// (each try waits in hardware for a while)
+__device__ __forceinline__ uint64_t device_ns() {
+    uint64_t t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+// Wait for the first phase; false when it does not complete in half a second (each
+// try waits in hardware for a while, the first ones without a look at the clock)
 __device__ __forceinline__ bool tma_wait(uint64_t* bar) {
-    for (int n = 0; n < (1 << 20); n++) {
+    uint64_t t0 = 0;
+    for (int n = 0;; n = n < 64 ? n + 1 : n) {
         uint32_t done;
         asm volatile(
             "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0; selp.b32 %0, 1, 0, p; }"
@@ -992,9 +998,27 @@ __device__ __forceinline__ bool tma_wait(uint64_t* bar) {
             : "r"(smem_u32(bar))
             : "memory");
         if (done) return true;
+        if (n < 64) continue;
+        const uint64_t t = device_ns();
+        if (t0 == 0) t0 = t;
+        if (t - t0 > 500000000u) return false;
     }
+}
+// ... in the step's kernels: a wait that ran out is noted for the end of the step
+// (finalize_dt), which stops there. It does not set halted, which other blocks look
+// at. The copies may still be under way into this block's memory, so it waits
+// once more before it gives the memory up.
+__device__ __forceinline__ bool tma_wait(uint64_t* bar, GamScalars* sc) {
+    if (tma_wait(bar)) return true;
+    sc->copyFailed = 1;
+    tma_wait(bar);
     return false;
 }
+#ifdef GAM_BOUNDS_CHECK
+#define GAM_COPY_BYTES(n) ((n) + sc->copyStall)  // test hook: bytes that never come
+#else
+#define GAM_COPY_BYTES(n) (n)
+#endif
 
 // VxB edge loop for direction E (fields.F90:184-228), one edge per thread. The
 // stencils (the two EdgeLRs with their limiters, GetCornerV's, GetCornerD's)
@@ -1017,7 +1041,7 @@ __global__ void __launch_bounds__(EdgeTile<E>::NT, MINB)
     const int i0 = r.i0 + blockIdx.x * T_::T0, j0 = r.j0 + blockIdx.y * T_::T1, k0 = r.k0 + blockIdx.z * T_::T2;
     if (threadIdx.x == 0) {
         tma_bar_init(&bar);
-        tma_expect(&bar, T_::all() * sizeof(R));
+        tma_expect(&bar, GAM_COPY_BYTES(T_::all() * sizeof(R)));
 #pragma unroll
         for (int q = 0; q < 6; q++)
             tma_load(sm + T_::off(q), &maps.m[q], i0 - T_::org(q, 0), j0 - T_::org(q, 1), k0 - T_::org(q, 2),
@@ -1050,11 +1074,7 @@ __global__ void __launch_bounds__(EdgeTile<E>::NT, MINB)
     m.detT = g.rdet[eD * fs + c];
     m.edge = g.edge[eD * fs + c];
     __syncthreads();  // the barrier's initialisation
-    if (!tma_wait(&bar)) {  // never in a sound step: stop it
-        sc->status = 5;
-        sc->halted = 1;
-        return;
-    }
+    if (!tma_wait(&bar, sc)) return;
     if (!in) return;
     {
         [[maybe_unused]] const long sA = dstride(b, dT1), sB = dstride(b, dT2), sM = sA > sB ? sA : sB;
@@ -1313,7 +1333,7 @@ __global__ void __launch_bounds__(FluxTile<R, D>::NT, MINB)
     const int k0 = r.k0 + blockIdx.z * (D == 2 ? T_::TN : 1);
     if (threadIdx.x == 0) {
         tma_bar_init(&bar);
-        tma_expect(&bar, P.doMHD ? T_::BYTES : T_::BYTES_GAS);
+        tma_expect(&bar, GAM_COPY_BYTES(P.doMHD ? T_::BYTES : T_::BYTES_GAS));
         const int qi = D == 0 ? i0 - 4 : i0, qj = D == 1 ? j0 - 4 : j0, qk = D == 2 ? k0 - 4 : k0;
         const int lj = D == 1 ? j0 - 2 : j0, lk = D == 2 ? k0 - 2 : k0;
         tma_load(sQ, &maps.QW, qi, qj, qk, 0, &bar);
@@ -1345,11 +1365,7 @@ __global__ void __launch_bounds__(FluxTile<R, D>::NT, MINB)
         }
     }
     __syncthreads();  // the barrier's initialisation
-    if (!tma_wait(&bar)) {  // never in a sound step: stop it
-        sc->status = 5;
-        sc->halted = 1;
-        return;
-    }
+    if (!tma_wait(&bar, sc)) return;
     if (!in) return;
     GAM_BOX_CHECK(c - 4 * s, c + 3 * s, 8 + D);
     flux_face<R, D, BORIS, false>(b, P, w, sc, gasN, gasO, c, sQ, sL, tx, tn, Vi, T, fa, Bn, B0, B0n);
@@ -1440,6 +1456,11 @@ __device__ __forceinline__ void finalize_dt(GamScalars* sc) {
     sc->time = sc->time + sc->dt;  // mhdgroup.F90:106
     sc->ts = sc->ts + 1;
     sc->t = sc->t + sc->dt;
+    if (sc->copyFailed) {  // its fluxes or EMFs are not those of the state
+        sc->status = 6;
+        sc->halted = sc->fixGhosts = 1;
+        return;
+    }
     if (sc->fixedTimestep) {
         step_scalars(sc);
         return;
