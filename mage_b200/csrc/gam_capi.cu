@@ -110,7 +110,8 @@ struct gam_handle {
     GamScalars* sc = nullptr;   // device
     GamFluxMapSet fmaps;        // tensor maps of the flux and edge kernels
     GamSlab slab;               // the small arrays' shared allocations (dalloc)
-    double* staging = nullptr;  // device, Fortran-layout transfer buffer
+    double* staging = nullptr;  // device, Fortran-layout transfer buffer of stagingN fields
+    int stagingN = 0;
     double* partial = nullptr;  // device, reduction partials
     double* dres = nullptr;     // device, reduction results
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
@@ -268,7 +269,9 @@ template <class R> static int alloc_bulk(gam_handle* h, Ctx<R>& C) {
         A(C.st[q].mf, 3);
         A(C.st[q].B, 3);
     }
-    A(C.w.QW, 5); A(C.w.QB, 3); A(C.w.Dh, 1); A(C.w.Wn, 5); A(C.w.Bl, 3); A(C.w.VdV, 3);
+    A(C.w.QW, 5); A(C.w.QB, 3); A(C.w.Dh, 1); A(C.w.Wn, 5); A(C.w.VdV, 3);
+    C.w.Bl = nullptr;
+    if (!h->p.doLFMLim) A(C.w.Bl, 3);  // lfmlim limits with the State's field
     A(C.w.abh, 3); A(C.w.bn, 3); A(C.w.Bnf, 3); A(C.w.AVf, 9); A(C.w.E, 3);
     A(C.w.gF, 15); A(C.w.mF, 9);
     // CalcElecField starts from E = 0 (fields.F90:88) and E2Flux
@@ -396,9 +399,10 @@ extern "C" int gam_create(const gam_params* p, gam_handle** out) {
         h->windTab = dalloc<double>(h, 7L * 4 * (h->b.Nj + 1) * (h->b.Nk + 1), &e);
         if (e != cudaSuccess) return bad(GAM_ECUDA, "cudaMalloc failed (wind tables)");
     }
-    // staging: the largest Fortran array passed through (Tf/Te: 27 face-sized comps)
-    long nface = (long)(h->b.Ni + 1) * (h->b.Nj + 1) * (h->b.Nk + 1);
-    h->staging = dalloc<double>(h, 27 * nface, &e);
+    // staging: the largest State array (Gas); the metric's pass through it in parts.
+    // FP32 holds an initial condition's fields there too (ic_fields)
+    h->stagingN = h->f32 ? 11 : 5;
+    h->staging = dalloc<double>(h, h->stagingN * fs, &e);
     if (e != cudaSuccess) return bad(GAM_ECUDA, "cudaMalloc failed (staging)");
     h->partial = dalloc<double>(h, 8 * (long)gam_diag_partials(h->b), &e);
     h->dres = dalloc<double>(h, 16, &e);
@@ -476,31 +480,46 @@ extern "C" const char* gam_last_error(gam_handle* h) { return h ? h->err.c_str()
 static long n_face(const GamBox& b) { return (long)(b.Ni + 1) * (b.Nj + 1) * (b.Nk + 1); }
 static long n_cell(const GamBox& b) { return (long)b.Ni * b.Nj * b.Nk; }
 
-// host Fortran array -> FP64 box array
-static int up_d(gam_handle* h, const double* src, double* dst, bool face, int nc) {
-    long n = (face ? n_face(h->b) : n_cell(h->b)) * nc;
-    CK(h, cudaMemcpyAsync(h->staging, src, sizeof(double) * n, cudaMemcpyHostToDevice, h->s));
-    gam_geom_fortran_to_box_d(h->b, h->staging, dst, face, nc, h->s);
+// Fortran array of nc components on the host -> box array, as many components at a
+// time as the staging buffer holds, and back
+template <class R> static int up_r(gam_handle* h, const double* src, R* dst, bool face, int nc) {
+    const long n = face ? n_face(h->b) : n_cell(h->b);
+    for (int c = 0; c < nc; c += h->stagingN) {
+        const int m = std::min(nc - c, h->stagingN);
+        CK(h, cudaMemcpyAsync(h->staging, src + c * n, sizeof(double) * n * m, cudaMemcpyHostToDevice, h->s));
+        if (sizeof(R) == sizeof(double))
+            gam_geom_fortran_to_box_d(h->b, h->staging, (double*)dst + c * h->b.fs, face, m, h->s);
+        else
+            gam_geom_fortran_to_box_f(h->b, h->staging, (float*)dst + c * h->b.fs, face, m, h->s);
+    }
     return GAM_OK;
 }
-template <class R> static int up_r(gam_handle* h, const double* src, R* dst, bool face, int nc) {
-    long n = (face ? n_face(h->b) : n_cell(h->b)) * nc;
-    CK(h, cudaMemcpyAsync(h->staging, src, sizeof(double) * n, cudaMemcpyHostToDevice, h->s));
-    if (sizeof(R) == sizeof(double))
-        gam_geom_fortran_to_box_d(h->b, h->staging, (double*)dst, face, nc, h->s);
-    else
-        gam_geom_fortran_to_box_f(h->b, h->staging, (float*)dst, face, nc, h->s);
-    return GAM_OK;
+static int up_d(gam_handle* h, const double* src, double* dst, bool face, int nc) {
+    return up_r<double>(h, src, dst, face, nc);
 }
 template <class R> static int down_r(gam_handle* h, const R* src, double* dst, bool face, int nc) {
-    long n = (face ? n_face(h->b) : n_cell(h->b)) * nc;
-    if (sizeof(R) == sizeof(double))
-        gam_geom_box_to_fortran_d(h->b, (const double*)src, h->staging, face, nc, h->s);
-    else
-        gam_geom_box_to_fortran_f(h->b, (const float*)src, h->staging, face, nc, h->s);
-    CK(h, cudaMemcpyAsync(dst, h->staging, sizeof(double) * n, cudaMemcpyDeviceToHost, h->s));
+    const long n = face ? n_face(h->b) : n_cell(h->b);
+    for (int c = 0; c < nc; c += h->stagingN) {
+        const int m = std::min(nc - c, h->stagingN);
+        if (sizeof(R) == sizeof(double))
+            gam_geom_box_to_fortran_d(h->b, (const double*)src + c * h->b.fs, h->staging, face, m, h->s);
+        else
+            gam_geom_box_to_fortran_f(h->b, (const float*)src + c * h->b.fs, h->staging, face, m, h->s);
+        CK(h, cudaMemcpyAsync(dst + c * n, h->staging, sizeof(double) * n * m, cudaMemcpyDeviceToHost, h->s));
+    }
     CK(h, cudaStreamSynchronize(h->s));
     return GAM_OK;
+}
+
+// FP64 fields of an initial condition: Gas (5), magFlux (3) and a vector potential (3).
+// The FP64 forms take the face velocities' 9 components for the latter two, which
+// every step forms anew before it reads them.
+struct IcFields {
+    double *Gas, *mf, *lA;
+};
+static IcFields ic_fields(gam_handle* h) {
+    double* mf = h->f32 ? h->staging + 5 * h->b.fs : h->cd.w.AVf;
+    return {h->staging, mf, mf + 3 * h->b.fs};
 }
 
 // FP32 form: round the FP64 metric once into the FP32 copies
@@ -1151,37 +1170,32 @@ static int init_common(gam_handle* h, double* Gas64, double* mf64) {
 extern "C" int gam_init_orszag_tang(gam_handle* h) {
     if (!h) return GAM_EINVAL;
     if (!h->haveGeo) return fail(h, GAM_ESTATE, "set the geometry first");
-    double* Gas64 = h->staging;
-    double* mf64 = h->staging + 5 * h->b.fs;
-    if (8 * h->b.fs > 27 * n_face(h->b)) return fail(h, GAM_EINVAL, "staging too small");
-    gam_geom_fill(Gas64, 8 * h->b.fs, 0.0, h->s);
-    gam_geom_ic_ot(h->b, h->gd.xyzcc, h->gd.face, Gas64, mf64, h->p.gamma, h->s);
-    return init_common(h, Gas64, mf64);
+    const IcFields f = ic_fields(h);
+    gam_geom_fill(f.Gas, 5 * h->b.fs, 0.0, h->s);
+    gam_geom_fill(f.mf, 3 * h->b.fs, 0.0, h->s);
+    gam_geom_ic_ot(h->b, h->gd.xyzcc, h->gd.face, f.Gas, f.mf, h->p.gamma, h->s);
+    return init_common(h, f.Gas, f.mf);
 }
 
 extern "C" int gam_init_test_problem(gam_handle* h, int32_t which, double a, double b) {
     if (!h || which < GAM_IC_ADV1D || which > GAM_IC_ALFVEN) return GAM_EINVAL;
     if (!h->haveXyz) return fail(h, GAM_ESTATE, "the problem set-ups integrate over cells and edges: call gam_set_geometry first");
-    if (11 * h->b.fs > 27 * n_face(h->b)) return fail(h, GAM_EINVAL, "staging too small");
-    double* Gas64 = h->staging;
-    double* mf64 = h->staging + 5 * h->b.fs;
-    double* lA = h->staging + 8 * h->b.fs;
-    gam_geom_fill(Gas64, 8 * h->b.fs, 0.0, h->s);
-    gam_geom_ic_case(h->b, h->gd.xyz, h->gd.xyzcc, h->gd.vol, Gas64, mf64, lA, h->p.gamma, which - GAM_IC_ADV1D, a, b,
+    const IcFields f = ic_fields(h);
+    gam_geom_fill(f.Gas, 5 * h->b.fs, 0.0, h->s);
+    gam_geom_fill(f.mf, 3 * h->b.fs, 0.0, h->s);
+    gam_geom_ic_case(h->b, h->gd.xyz, h->gd.xyzcc, h->gd.vol, f.Gas, f.mf, f.lA, h->p.gamma, which - GAM_IC_ADV1D, a, b,
                      h->s);
-    return init_common(h, Gas64, mf64);
+    return init_common(h, f.Gas, f.mf);
 }
 
 extern "C" int gam_init_blast_wave(gam_handle* h, const double* bw9) {
     if (!h || !bw9) return GAM_EINVAL;
     if (!h->haveXyz) return fail(h, GAM_ESTATE, "the blast-wave IC integrates over cells: call gam_set_geometry first");
-    if (11 * h->b.fs > 27 * n_face(h->b)) return fail(h, GAM_EINVAL, "staging too small");
-    double* Gas64 = h->staging;
-    double* mf64 = h->staging + 5 * h->b.fs;
-    double* lA = h->staging + 8 * h->b.fs;
-    gam_geom_fill(Gas64, 8 * h->b.fs, 0.0, h->s);
-    gam_geom_ic_bw(h->b, h->gd.xyz, h->gd.vol, Gas64, mf64, lA, h->p.gamma, bw9, h->p.doMHD != 0, h->s);
-    return init_common(h, Gas64, mf64);
+    const IcFields f = ic_fields(h);
+    gam_geom_fill(f.Gas, 5 * h->b.fs, 0.0, h->s);
+    gam_geom_fill(f.mf, 3 * h->b.fs, 0.0, h->s);
+    gam_geom_ic_bw(h->b, h->gd.xyz, h->gd.vol, f.Gas, f.mf, f.lA, h->p.gamma, bw9, h->p.doMHD != 0, h->s);
+    return init_common(h, f.Gas, f.mf);
 }
 
 // ------------------------------------------------------------ background field and solar wind
@@ -1247,10 +1261,9 @@ extern "C" int gam_set_background_dipole(gam_handle* h, double M0) {
     if (!h) return GAM_EINVAL;
     if (!h->p.doBackground) return fail(h, GAM_ESTATE, "the handle was created without doBackground");
     if (!h->haveXyz) return fail(h, GAM_ESTATE, "the dipole background integrates over cells: call gam_set_geometry first");
-    if (9 * h->b.fs > 27 * n_face(h->b)) return fail(h, GAM_EINVAL, "staging too small");
     const GeoD& g = h->gd;
     gam_geom_b0_dipole(h->b, g.xyz, g.face, g.vol, g.Te, M0, h->bg.fcB0, h->bg.bFlux0, h->bg.edgB0, h->bg.B0,
-                       h->bg.dpB0, h->staging, h->s);
+                       h->bg.dpB0, h->f32 ? h->staging : h->cd.w.AVf, h->s);
     CK(h, cudaGetLastError());
     CK(h, cudaStreamSynchronize(h->s));
     h->haveBg = true;
@@ -1682,15 +1695,13 @@ extern "C" int gam_init_dipole_wind(gam_handle* h, const double wind[8], uint64_
     if (!h || !wind) return GAM_EINVAL;
     if (!h->haveXyz) return fail(h, GAM_ESTATE, "the vector potential is integrated along edges: call gam_set_geometry first");
     if (h->p.doBackground && !h->haveBg) return fail(h, GAM_ESTATE, "set the background field first");
-    if (11 * h->b.fs > 27 * n_face(h->b)) return fail(h, GAM_EINVAL, "staging too small");
     int rc;
     if (h->p.bc[1] == GAM_BC_WIND && (rc = gam_set_wind(h, wind))) return rc;
-    double* Gas64 = h->staging;
-    double* mf64 = h->staging + 5 * h->b.fs;
-    double* lA = h->staging + 8 * h->b.fs;
-    gam_geom_fill(Gas64, 8 * h->b.fs, 0.0, h->s);
-    gam_geom_ic_wind(h->b, h->gd.xyz, Gas64, mf64, lA, h->p.gamma, h->p.dFloor, h->p.pFloor, wind, seed, amp, h->s);
-    return init_common(h, Gas64, mf64);
+    const IcFields f = ic_fields(h);
+    gam_geom_fill(f.Gas, 5 * h->b.fs, 0.0, h->s);
+    gam_geom_fill(f.mf, 3 * h->b.fs, 0.0, h->s);
+    gam_geom_ic_wind(h->b, h->gd.xyz, f.Gas, f.mf, f.lA, h->p.gamma, h->p.dFloor, h->p.pFloor, wind, seed, amp, h->s);
+    return init_common(h, f.Gas, f.mf);
 }
 
 // ------------------------------------------------------------ restart files
