@@ -1029,15 +1029,27 @@ class WholeStep:
         ts = [t.contiguous() for t in (cur["Gas"], cur["mf"], old["Gas"], old["mf"])]
         return ts, _vp([t.data_ptr() for t in ts])
 
-    def work_areas(self, n: int) -> list:
-        """Up to n work areas, the object's own first: one step's intermediates
-        each. The others take at most 16 GiB and a quarter of what is free."""
+    def areas_that_fit(self, n: int, need: int = 0) -> int:
+        """How many of n work areas a caller that takes need bytes beside them may
+        have, one at least: those after the object's own take at most 16 GiB and a
+        quarter of what need leaves free."""
         if n > 1 and self.work.is_cuda:
             dev = self.work.device
             free = (torch.cuda.mem_get_info(dev)[0] + torch.cuda.memory_reserved(dev)
                     - torch.cuda.memory_allocated(dev))
-            n = min(n, 1 + min(16 << 30, free // 4) // max(1, self.work.numel()))
-        return [self.work] + [torch.empty_like(self.work) for _ in range(n - 1)]
+            n = min(n, 1 + min(16 << 30, max(0, free - need) // 4) // max(1, self.work.numel()))
+        return n
+
+    def work_areas(self, n: int) -> list:
+        """n work areas, the object's own first: one step's intermediates each. Fewer
+        where the memory for them, free by its amount, is not there in one piece."""
+        areas = [self.work]
+        try:
+            while len(areas) < n:
+                areas.append(torch.empty_like(self.work))
+        except torch.OutOfMemoryError:
+            pass
+        return areas
 
     def forward(self, cur: dict, old: dict, dt: float, odt: float, work=None) -> dict:
         """State after the step (gam_step_fwd_save); cur/old as for step(). The
@@ -1295,34 +1307,55 @@ def loss_and_grad_c(g: Grid, Gas0, mf0, dt: float, nsteps: int, seg: int | None 
     own gradient. The adjoint of oState at step n is the adjoint of State at
     step n-1, so it seeds that step's accumulators. params = [g.inflow]
     also returns the loss's gradient w.r.t. the inflow state (the sum of
-    every step's inflow adjoints), as a fourth result."""
+    every step's inflow adjoints), as a fourth result. Some of a segment's
+    steps keep their intermediates where there is memory for it; where that
+    turns out to leave too little, the sweep runs again without (and calls
+    lossf again)."""
     params = list(params or [])
     for q in params:
         assert q is g.inflow, "loss_and_grad_c differentiates w.r.t. the inflow state only"
-    dw = torch.zeros(8, dtype=g.dtype, device=Gas0.device) if params else None
     ws = WholeStep(g)
     seg = seg or max(1, int(round(nsteps ** 0.5)))
-    # the last steps of a segment keep their intermediates for their adjoints, as
-    # many as have a work area: with one for each, a step runs forward twice (the
-    # last segment's once) instead of three times (64^3, 20 steps: 42.3 -> 35.4 ms)
-    areas = ws.work_areas(min(seg, nsteps))
+    # what the sweep holds itself: the checkpoints' pairs, a segment's states, adjoints
+    state = 11 * Gas0[0].numel() * Gas0.element_size()
+    areas = ws.work_areas(ws.areas_that_fit(min(seg, nsteps), (2 * (nsteps // seg + 1) + seg + 8) * state))
+    try:
+        return _sweep_c(ws, areas, g, Gas0, mf0, dt, nsteps, seg, lossf, bool(params))
+    except torch.OutOfMemoryError:
+        pass
+    # the loss or what else lives on the device left no room for the kept areas
+    del areas
+    torch.cuda.empty_cache()
+    return _sweep_c(ws, [], g, Gas0, mf0, dt, nsteps, seg, lossf, bool(params))
 
-    def run(c, o, m):
-        """m steps from (c, o): the pair each starts from, and the last pair"""
+
+def _sweep_c(ws: WholeStep, areas: list, g: Grid, Gas0, mf0, dt: float, nsteps: int, seg: int, lossf, inflow: bool):
+    """The sweep of loss_and_grad_c. The last steps of a segment keep their
+    intermediates in areas for their adjoints: with an area for each, a step runs
+    forward twice (the last segment's once) instead of three times (64^3, 20 steps:
+    42.3 -> 35.4 ms); without areas none is kept."""
+    dw = torch.zeros(8, dtype=g.dtype, device=Gas0.device) if inflow else None
+
+    def area(w):
+        return areas[max(0, w)] if areas else None
+
+    def run(c, o, m, keep):
+        """m steps from (c, o): the pair each starts from (keep), and the last pair"""
         sts = []
         for q in range(m):
-            sts.append((c, o))
-            c, o = ws.forward(c, o, dt, dt, areas[max(0, q - m + len(areas))]), c
+            if keep:
+                sts.append((c, o))
+            c, o = ws.forward(c, o, dt, dt, area(q - m + len(areas))), c
         return sts, c, o
 
     with torch.no_grad():
         cur = {"Gas": Gas0.contiguous(), "mf": mf0.contiguous(), "B": g.bxyz(mf0)}
         old = cur
         ckpt = []
+        sts = []  # the pairs of a segment whose intermediates the areas hold: the last one
         for n in range(0, nsteps, seg):
             ckpt.append((n, cur, old))
-            sts = []  # the states of the segment before
-            sts, cur, old = run(cur, old, min(seg, nsteps - n))
+            sts, cur, old = run(cur, old, min(seg, nsteps - n), bool(areas) and n + seg >= nsteps)
         fin = {k: v.detach().clone().requires_grad_(True) for k, v in cur.items()}
     with torch.enable_grad():
         L = lossf(g, fin)
@@ -1331,20 +1364,23 @@ def loss_and_grad_c(g: Grid, Gas0, mf0, dt: float, nsteps: int, seg: int | None 
     carry = None  # adjoint of the oState of the step after the current one
     with torch.no_grad():
         for n0, c0, o0 in reversed(ckpt):
-            if sts is None:
-                sts = run(c0, o0, min(seg, nsteps - n0))[0]
-            m = len(sts)
+            m = min(seg, nsteps - n0)
+            if not sts and areas:
+                sts = run(c0, o0, m, True)[0]
+            elif not sts:
+                sts, c, o = run(c0, o0, m - 1, True)
+                sts.append((c, o))
             for q in range(m - 1, -1, -1):
                 c, o = sts[q]
                 w = q - m + len(areas)
                 # its own adjoints start from those of the next step's oState
                 acc = list(carry) if carry is not None else [torch.zeros_like(c["Gas"]), torch.zeros_like(c["mf"])]
                 acc += [torch.zeros_like(o["Gas"]), torch.zeros_like(o["mf"])]
-                d = ws.adjoint(c, o, dt, dt, lam, acc, saved=w >= 0, dinflow=dw, work=areas[max(0, w)])
+                d = ws.adjoint(c, o, dt, dt, lam, acc, saved=w >= 0, dinflow=dw, work=area(w))
                 lam = {"Gas": d[0], "mf": d[1]}
                 carry = (d[2], d[3])
-            sts = None
+            sts = []
     # step 0 starts from State = oState = (Gas0, mf0)
-    if params:
+    if inflow:
         return float(L.detach()), lam["Gas"] + carry[0], lam["mf"] + carry[1], [dw]
     return float(L.detach()), lam["Gas"] + carry[0], lam["mf"] + carry[1]
