@@ -151,6 +151,7 @@ template <class T> static T* dalloc(gam_handle* h, long n, cudaError_t* e) {
     void* p = h->slab.take(sizeof(T) * (size_t)n, *e, [h](void** q, size_t bytes) {
         const cudaError_t rc = cudaMalloc(q, bytes);
         if (rc == cudaSuccess) h->allocs.push_back(*q);
+        else cudaGetLastError();  // reported here, not by a later call's check
         return rc;
     });
     if (!p) return nullptr;

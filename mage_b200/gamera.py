@@ -14,6 +14,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import sys
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -250,11 +251,23 @@ class GameraGPU:
         self._lib_path = lib_path
         self.params = params
         self._cp = params.to_c()
+        rc = self._create()
+        if rc == GAM_ECUDA and b"cudaMalloc failed" in self.L.gam_last_error(self.h):
+            # memory that PyTorch's allocator keeps after its tensors are gone (a gradient
+            # sweep's work areas, up to 16 GiB) is free for the handle
+            torch = sys.modules.get("torch")
+            if torch is not None and torch.cuda.is_initialized():
+                torch.cuda.empty_cache()
+                self.close()
+                rc = self._create()
+        self._check(rc)
+        self.Ni, self.Nj, self.Nk = params.dims
+
+    def _create(self) -> int:
         h = C.c_void_p()
         rc = self.L.gam_create(C.byref(self._cp), C.byref(h))
         self.h = h
-        self._check(rc)
-        self.Ni, self.Nj, self.Nk = params.dims
+        return rc
 
     def __del__(self):
         h = getattr(self, "h", None)
