@@ -515,13 +515,6 @@ __global__ void __launch_bounds__(FluxTile<R, D>::NT, MINB)
     if (!in) return;
     flux_face<R, D, false, true>(b, P, w, sc, nullptr, nullptr, c, sQ, sL, tx, tn, Vi, T, fa, Bn, B0, B0n);
 }
-// the grid of FluxTile's blocks over the faces r of direction D
-template <class R, int D> dim3 flux_grid(const Range& r) {
-    using T_ = FluxTile<R, D>;
-    return dim3((unsigned)((r.i1 - r.i0 + T_::TX) / T_::TX),
-                (unsigned)(D == 2 ? r.j1 - r.j0 + 1 : (r.j1 - r.j0 + T_::TN) / T_::TN),
-                (unsigned)(D == 2 ? (r.k1 - r.k0 + T_::TN) / T_::TN : r.k1 - r.k0 + 1));
-}
 template <class R, int D>
 void launch_stress_box(const GamBox& b, const DevParams<R>& P, const Geo<R>& g, const R* Bl, const Work<R>& w,
                        const Range& r, const GamScalars* sc, cudaStream_t s) {
@@ -618,8 +611,7 @@ template <class R, int E>
 void launch_vxb_box(const GamBox& b, const DevParams<R>& P, const Geo<R>& g, const Work<R>& w, const Range& r,
                     const GamScalars* sc, cudaStream_t s) {
     using T_ = EdgeTile<E>;
-    const dim3 gr((unsigned)((r.i1 - r.i0 + T_::T0) / T_::T0), (unsigned)((r.j1 - r.j0 + T_::T1) / T_::T1),
-                  (unsigned)((r.k1 - r.k0 + T_::T2) / T_::T2));
+    const dim3 gr = edge_grid<E>(r);
     const unsigned sm = T_::all() * sizeof(R);
     constexpr int MB = sizeof(R) == 8 ? 2 : 4;
     k_vxb_box<R, E, MB><<<gr, T_::NT, sm, s>>>(b, P, g, w, r, sc);
@@ -1018,7 +1010,7 @@ __device__ void p2c_adj(A dF, A pF, A gm1, const A* W, const A* aU, A* aW) {
     aW[4] += (W[4] < pF) ? (A)0.0 : aU[4] / gm1;
     aW[0] += (W[0] < dF) ? (A)0.0 : a_rho;
 }
-// reverse of block_c2p (BlockCon2Prim): aW (5) -> aU (5)
+// reverse of BlockCon2Prim: aW (5) -> aU (5)
 template <class A>
 __device__ void bc2p_adj(A dF, A pF, A gm1, const A* U, const A* aW, A* aU) {
     const A D = U[0] < dF ? dF : U[0], rD = (A)1.0 / D;
@@ -1714,11 +1706,6 @@ int flux_call(const gam_params* p, const void* QW, const void* Wn, const void* Q
     const Range fr[3] = {{G, G + b.Nip, G, G + b.Njp - 1, G, G + b.Nkp - 1},
                          {G, G + b.Nip - 1, G, G + b.Njp, G, G + b.Nkp - 1},
                          {G, G + b.Nip - 1, G, G + b.Njp - 1, G, G + b.Nkp}};
-    const dim3 blk(16, 8, 1);
-    auto grid = [&](const Range& r) {
-        return dim3((unsigned)((r.i1 - r.i0 + 1 + blk.x - 1) / blk.x), (unsigned)((r.j1 - r.j0 + 1 + blk.y - 1) / blk.y),
-                    (unsigned)((r.k1 - r.k0 + 1 + blk.z - 1) / blk.z));
-    };
     const R* Bl = (const R*)Blim;
     if (!dgF) {
         launch_stress_box<R, 0>(b, P, g, Bl, w, fr[0], sc, s);

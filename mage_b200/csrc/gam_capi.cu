@@ -523,8 +523,8 @@ static IcFields ic_fields(gam_handle* h) {
     return {h->staging, mf, mf + 3 * h->b.fs};
 }
 
-// FP32 form: round the FP64 metric once into the FP32 copies
-// the compute form's copies and tables of a geometry just set
+// The compute form's tables of a geometry just set and, in FP32, its copies of the
+// metric, rounded once
 static void sync_geo(gam_handle* h) {
     if (!h->f32) {
         gam_geom_tables(h->b, h->gd.vol, h->gd.face, h->gd.Teb, h->cd.g, h->s);

@@ -308,23 +308,6 @@ __device__ __forceinline__ void lrs_from_qdv(const DevParams<R>& P, const R* QdV
 }
 
 // ----------------------------------------------------------------- EOS
-// BlockCon2Prim (recon.F90:62-91)
-template <class R>
-__device__ __forceinline__ void block_c2p(const DevParams<R>& P, const R* U, R* W) {
-    R D = rmax(U[0], P.dFloor);
-    const Quot<R> qD(D);
-    R Mx = U[1], My = U[2], Mz = U[3], E = U[4];
-    const R num[4] = {Mx, My, Mz, (R)0.5 * (Mx * Mx + My * My + Mz * Mz)};
-    R quo[4];
-    qD.template many<4>(num, quo);
-    R KinE = quo[3];
-    R Pr = rmax(P.gm1 * (E - KinE), P.pFloor);
-    W[0] = D;
-    W[1] = quo[0];
-    W[2] = quo[1];
-    W[3] = quo[2];
-    W[4] = Pr;
-}
 // CellC2P (gamutils.F90:301-321)
 template <class R>
 __device__ __forceinline__ void cell_c2p(const DevParams<R>& P, const R* U, R* W) {
@@ -471,11 +454,6 @@ template <class R>
 __device__ __forceinline__ void cell_bxyz(const GamBox& b, const Geo<R>& g, long c, R fI, R fIp, R fJ, R fJp, R fK,
                                           R fKp, R* B) {
     cell_bxyz_q(b, g, c, fI, fIp, fJ, fJp, fK, fKp, Quot<R>(g.vol[c]), B);
-}
-template <class R>
-__device__ __forceinline__ void cell_bxyz(const GamBox& b, const Geo<R>& g, long c, R fI, R fIp, R fJ, R fJp, R fK,
-                                          R fKp, const Quot<R>& qV, R* B) {
-    cell_bxyz_q(b, g, c, fI, fIp, fJ, fJp, fK, fKp, qV, B);
 }
 
 // ----------------------------------------------------------------- bounds checks
@@ -3037,8 +3015,21 @@ __global__ void __launch_bounds__(128) k_bfield_all(GamBox b, Geo<R> g, StateBuf
     for (int x = 0; x < 3; x++) s.B[x * fs + c] = B[x];
 }
 
-#ifdef GAM_GEO_TABLES  // the builds that hold the step
 // ----------------------------------------------------------------- launches
+// The grids of FluxTile's blocks over the faces r of direction D, and of EdgeTile's
+// over the edges r of direction E
+template <class R, int D> dim3 flux_grid(const Range& r) {
+    using T_ = FluxTile<R, D>;
+    return dim3((unsigned)((r.i1 - r.i0 + T_::TX) / T_::TX),
+                (unsigned)(D == 2 ? r.j1 - r.j0 + 1 : (r.j1 - r.j0 + T_::TN) / T_::TN),
+                (unsigned)(D == 2 ? (r.k1 - r.k0 + T_::TN) / T_::TN : r.k1 - r.k0 + 1));
+}
+template <int E> dim3 edge_grid(const Range& r) {
+    using T_ = EdgeTile<E>;
+    return dim3((unsigned)((r.i1 - r.i0 + T_::T0) / T_::T0), (unsigned)((r.j1 - r.j0 + T_::T1) / T_::T1),
+                (unsigned)((r.k1 - r.k0 + T_::T2) / T_::T2));
+}
+#ifdef GAM_GEO_TABLES  // the builds that hold the step
 static inline dim3 grid_for(const Range& r, dim3 blk) {
     return dim3((unsigned)((r.i1 - r.i0 + 1 + blk.x - 1) / blk.x), (unsigned)((r.j1 - r.j0 + 1 + blk.y - 1) / blk.y),
                 (unsigned)((r.k1 - r.k0 + 1 + blk.z - 1) / blk.z));
@@ -3046,8 +3037,7 @@ static inline dim3 grid_for(const Range& r, dim3 blk) {
 
 template <class R, int E> void launch_vxb(const Ctx<R>& C, const Range& r, cudaStream_t s) {
     using T_ = EdgeTile<E>;
-    const dim3 gr((unsigned)((r.i1 - r.i0 + T_::T0) / T_::T0), (unsigned)((r.j1 - r.j0 + T_::T1) / T_::T1),
-                  (unsigned)((r.k1 - r.k0 + T_::T2) / T_::T2));
+    const dim3 gr = edge_grid<E>(r);
     const unsigned sm = T_::all() * sizeof(R);
     // blocks of 256 per SM: 3 in FP64 (strict 289/299/299 us for the three
     // directions at 192^3; 2: 372/376/377, 4: 305/313/325), 5 in FP32
@@ -3157,9 +3147,7 @@ template <class R, class F> void for_each_kernel(const Ctx<R>& C, int cur, cudaS
         constexpr int D = decltype(Dc)::value;
         const Range& r = fr[D];
         using T_ = FluxTile<R, D>;
-        const dim3 sg((unsigned)((r.i1 - r.i0 + T_::TX) / T_::TX),
-                      (unsigned)(D == 2 ? r.j1 - r.j0 + 1 : (r.j1 - r.j0 + T_::TN) / T_::TN),
-                      (unsigned)(D == 2 ? (r.k1 - r.k0 + T_::TN) / T_::TN : r.k1 - r.k0 + 1));
+        const dim3 sg = flux_grid<R, D>(r);
         const GamFluxMaps& M = C.fmaps->m[cur][D];
         // blocks per SM (registers against warps; 192^3, I/J/K sweeps): the strict
         // form 5 (782/739/808 us; 4: 852/770/775, 7: 895/854/859), the FMA form 5

@@ -1,4 +1,4 @@
-"""The flux kernels' shared-memory tiles (16 or 32 faces by 4 or 8) at sizes
+"""The flux kernels' shared-memory tiles (16 or 32 faces by 8) at sizes
 around them: one tile and less, whole tiles, remainders in every direction, a
 2.5-D grid; both reconstructions, the limiter on either state, no field. The
 strict build equals the CPU restatement bit for bit; FP32 stays within its
