@@ -43,7 +43,9 @@ sys.path.insert(0, ROOT)
 # with a background field 24 more values, FP64 in both forms.
 BYTES_PER_CELL = {"f64": 8 * (27 + 79), "f32": 4 * (27 + 79)}
 BYTES_PER_CELL_B0 = {"f64": 8 * (27 + 79 + 24), "f32": 4 * (27 + 79) + 8 * 24}
-KERNELS_PER_STEP = 15  # begin, predict, 3x(mom2face, vxb), 3x stress, faces, cells, dt, bc
+# Kernels of a step: predict, 3 x (mom2face, vxb), 3 x stress, faces, cells, bc, and with the wind, the rings and the
+# hooks the launch lists in profiles/; a call of step_gamera starts with one more
+KERNELS_PER_STEP = {"bw": 13, "ot": 13, "dipole": 14, "magsphere": 35}
 DIPOLE_WORKLOAD, DIPOLE_STEPS = "dipole96", 500
 MAGSPHERE_WORKLOAD, MAGSPHERE_STEPS = "lfm96", 100
 
@@ -134,15 +136,13 @@ def measured_peak():
     return 6650.0, "fallback"
 
 
-# Instructions per active cell-update of the FP64 drop-in step, from the
-# single-kernel ncu captures of the 96^3 step (profiles/
-# blast96_fp64_strict_kernels.md; the I-face flux kernel counted for all three
-# directions), scaled to 192^3 by the ratio of ghosted to active cells
-# ((200/192)^3 / (104/96)^3): warp instructions x 32 (issue slots) and the FP64
-# arithmetic instructions of active threads (DADD + DMUL + DFMA).
-_SCALE_96_TO_192 = (200 / 192) ** 3 / (104 / 96) ** 3
-INST_PER_CELL_F64 = (3 * 544 + 2208 + 3 * 3182 + 1759 + 3 * 1168) * _SCALE_96_TO_192
-FP64_OPS_PER_CELL = (3 * 110 + 545 + 3 * 1027 + 334 + 3 * 322) * _SCALE_96_TO_192
+# Instructions per active cell-update of the FP64 drop-in step at 192^3: the
+# counts of its kernels at 96^3 (profiles/blast96_step_kernels.md), each
+# scaled to 192^3 by its number of blocks (issue slots: warp instructions x 32)
+# or of cells, faces or edges (FP64 arithmetic instructions of active threads:
+# DADD + DMUL + DFMA).
+INST_PER_CELL_F64 = 13895
+FP64_OPS_PER_CELL = 4381
 
 
 def committed_traffic(workload, dtype):
@@ -599,7 +599,7 @@ def main():
                             "note": "issue: 148 SMs x 4 schedulers x 1 warp-instruction (32 lanes) per clock; FP64 "
                                     "pipe: 148 SMs x 64 FP64 lanes per clock (a DFMA counts once); both at the median "
                                     "SM clock sampled in the timed region; instruction counts of the drop-in (strict) "
-                                    "kernels"} if (w["problem"] == "bw" and args.strict) else None,
+                                    "kernels at 192^3"} if (w["problem"] == "bw" and args.strict) else None,
             "e2e": {"value": e2e_value, "unit": "cell-updates/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                     "steps": args.e2e_steps,
                     "what": "per step: gam_upload_state of State%Gas and State%magFlux from pinned host memory "
@@ -614,7 +614,7 @@ def main():
             "adjoint": adj,
             "cpu_baseline": cpu,
             "clocks": clocks,
-            "gpu_launches": KERNELS_PER_STEP * args.steps,
+            "gpu_launches": KERNELS_PER_STEP[w["problem"]] * args.steps + 1,
         }
         print(json.dumps(line), flush=True)
     if dist is not None:
