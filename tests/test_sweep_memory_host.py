@@ -96,3 +96,8 @@ def test_areas_leave_the_sweeps_own_memory(monkeypatch):
     assert ws.areas_that_fit(99, 64 << 30) == 11       # a quarter of 40 GiB
     assert ws.areas_that_fit(99, 200 << 30) == 1
     assert ws.areas_that_fit(3) == 3
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda d: (0, 180 << 30))
+    assert ws.areas_that_fit(3) == 2                   # (8 - 4) / 4 GiB, of the allocator's own
+    ws.work.numel = lambda: 1 << 28
+    assert ws.areas_that_fit(5, 99 << 30) == 5         # 1 GiB: not looked at
+    assert ws.areas_that_fit(6, 99 << 30) == 1
