@@ -118,7 +118,6 @@ struct gam_handle {
     cudaGraphExec_t pgraph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // [parity][phase] (tile steps)
     int cur = 0;
     bool haveGeo = false, haveState = false, haveXyz = false;
-    bool newState = false;  // a State has been uploaded since the last step
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaStream_t aux[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     cudaEvent_t evs[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -792,7 +791,6 @@ extern "C" int gam_upload_state(gam_handle* h, const double* Gas, const double* 
     if ((rc = set_scalars(h, time, otime, dt, ts, !oGas))) return rc;
     CK(h, cudaStreamSynchronize(h->s));
     h->haveState = true;
-    h->newState = true;
     return GAM_OK;
 }
 
@@ -854,17 +852,16 @@ extern "C" int gam_download_state(gam_handle* h, double* Gas, double* magFlux, d
     return GAM_OK;
 }
 
-void gam_strict_begin_f64(const Ctx<double>& C, int cur, bool slots, cudaStream_t s);
-void gam_fast_begin_f64(const Ctx<double>& C, int cur, bool slots, cudaStream_t s);
-void gam_fast_begin_f32(const Ctx<float>& C, int cur, bool slots, cudaStream_t s);
+void gam_strict_begin_f64(const Ctx<double>& C, cudaStream_t s);
+void gam_fast_begin_f64(const Ctx<double>& C, cudaStream_t s);
+void gam_fast_begin_f32(const Ctx<float>& C, cudaStream_t s);
 static void launch_begin(gam_handle* h) {
     if (h->f32)
-        gam_fast_begin_f32(h->cf, h->cur, h->newState, h->s);
+        gam_fast_begin_f32(h->cf, h->s);
     else if (h->p.strict)
-        gam_strict_begin_f64(h->cd, h->cur, h->newState, h->s);
+        gam_strict_begin_f64(h->cd, h->s);
     else
-        gam_fast_begin_f64(h->cd, h->cur, h->newState, h->s);
-    h->newState = false;
+        gam_fast_begin_f64(h->cd, h->s);
 }
 static void launch_one(gam_handle* h, int cur) {
     if (h->f32)
@@ -1872,7 +1869,6 @@ extern "C" int gam_step_begin(gam_handle* h) {
     if ((rc = ensure_phase_graph(h, h->cur, 0))) return rc;
     if ((rc = ensure_phase_graph(h, h->cur, 1))) return rc;
     CK(h, cudaEventRecord(h->ev0, h->s));
-    if (h->newState) launch_begin(h);
     CK(h, cudaGraphLaunch(h->pgraph[h->cur][0], h->s));
     return GAM_OK;
 }
@@ -1937,7 +1933,6 @@ extern "C" int gam_step_begin_dev(gam_handle* h) {
     if ((rc = ensure_phase_graph(h, h->cur, 0))) return rc;
     if ((rc = ensure_phase_graph(h, h->cur, 1))) return rc;
     if (h->nasync == 0) CK(h, cudaEventRecord(h->ev0, h->s));
-    if (h->newState) launch_begin(h);
     CK(h, cudaGraphLaunch(h->pgraph[h->cur][0], h->s));
     return GAM_OK;
 }

@@ -22,5 +22,5 @@ void gam_fast_phase_f64(const Ctx<double>& C, int cur, cudaStream_t s, int phase
 void gam_fast_halo_f64(const Ctx<double>& C, int cur, cudaStream_t s, int dside, int unpack, int copyB, void* buf) { gam_fast::launch_halo<double>(C, cur, s, dside, unpack, copyB, buf); }
 void gam_fast_phase_f32(const Ctx<float>& C, int cur, cudaStream_t s, int phase) { gam_fast::launch_step_phase<float>(C, cur, s, phase); }
 void gam_fast_halo_f32(const Ctx<float>& C, int cur, cudaStream_t s, int dside, int unpack, int copyB, void* buf) { gam_fast::launch_halo<float>(C, cur, s, dside, unpack, copyB, buf); }
-void gam_fast_begin_f64(const Ctx<double>& C, int cur, bool slots, cudaStream_t s) { gam_fast::launch_begin<double>(C, cur, slots, s); }
-void gam_fast_begin_f32(const Ctx<float>& C, int cur, bool slots, cudaStream_t s) { gam_fast::launch_begin<float>(C, cur, slots, s); }
+void gam_fast_begin_f64(const Ctx<double>& C, cudaStream_t s) { gam_fast::launch_begin<double>(C, s); }
+void gam_fast_begin_f32(const Ctx<float>& C, cudaStream_t s) { gam_fast::launch_begin<float>(C, s); }

@@ -1353,12 +1353,18 @@ __global__ void __launch_bounds__(FluxTile<R, D>::NT, MINB)
 // E2Flux into the new buffer; faces outside its range are copied. With
 // doAB3 the buffer's old content (oState, n-1) first moves to ooState
 // (CopyState(oState, ooState), mhdgroup.F90:100-102).
+// Where r ends before the box, its last index stands for the box's last layer: the
+// slots there of the other directions' components belong to no face, no boundary
+// fills them, and they keep State's values.
 template <class R>
 __global__ void __launch_bounds__(256) k_update_faces(GamBox b, DevParams<R> P, StateBuf<R> cur, StateBuf<R> nxt,
                                                       Work<R> w, Range r, const GamScalars* sc, R* __restrict__ oomf) {
     if (sc->halted) return;
     int ii, jj, kk;
     if (!thread_ijk(r, ii, jj, kk)) return;
+    if (ii == r.i1) ii = b.Ni;
+    if (jj == r.j1) jj = b.Nj;
+    if (kk == r.k1) kk = b.Nk;
     const long fs = b.fs;
     const long c = lidx(b, ii, jj, kk);
     const int G = GAM_NG;
@@ -1398,32 +1404,6 @@ __device__ __forceinline__ void step_scalars(GamScalars* sc) {
     sc->pdt = 0.5 * sc->dt;
     sc->rodt = 1.0 / sc->odt;
     sc->rdt = 1.0 / sc->dt;
-}
-// magFlux has slots in the last layer across each component's direction that no
-// face is in. The update copies State's to the new buffer only where it copies the
-// ghosts, so after an upload they are copied here once, and both buffers hold
-// State's from then on.
-template <class R>
-__global__ void __launch_bounds__(128) k_last_slots(GamBox b, StateBuf<R> cur, StateBuf<R> nxt, const GamScalars* sc) {
-    if (sc->halted) return;
-    long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    const long nI = b.Ni + 1, nK = nI * (b.Nj + 1), nJ = nI * b.Nk;  // the last layers of K, J and I
-    int ii, jj, kk;
-    if (t < nK) {
-        ii = (int)(t % nI), jj = (int)(t / nI), kk = b.Nk;
-    } else if ((t -= nK) < nJ) {
-        ii = (int)(t % nI), jj = b.Nj, kk = (int)(t / nI);
-    } else if ((t -= nJ) < (long)b.Nj * b.Nk) {
-        ii = b.Ni, jj = (int)(t % b.Nj), kk = (int)(t / b.Nj);
-    } else {
-        return;
-    }
-    const long c = lidx(b, ii, jj, kk);
-    GAM_BOX_CHECK(c, c, 14);
-    const bool last[3] = {ii == b.Ni, jj == b.Nj, kk == b.Nk};
-#pragma unroll
-    for (int d = 0; d < 3; d++)
-        if (last[(d + 1) % 3] || last[(d + 2) % 3]) nxt.mf[d * b.fs + c] = cur.mf[d * b.fs + c];
 }
 // The end of a step: time bookkeeping and CalcDT's checks (gamapp.F90:110-111,
 // step.F90:58-168), by one thread; then the scalars of the next step
@@ -3184,7 +3164,11 @@ template <class R, class F> void for_each_kernel(const Ctx<R>& C, int cur, cudaS
             const long nf = (long)ni * (b.Njp + 1);
             k_fix_e_lfm<R><<<(unsigned)((nf + 255) / 256), 256, 0, s>>>(b, C.w.E, GAM_NG, GAM_NG + b.Njp, C.sc);
         }
-        k_update_faces<R><<<grid_for(faces, blk), blk, 0, s>>>(b, C.P, S, O, C.w, faces, C.sc, C.oomf);
+        Range fl = faces;  // with the last layers
+        fl.i1 += fl.i1 < b.Ni;
+        fl.j1 += fl.j1 < b.Nj;
+        fl.k1 += fl.k1 < b.Nk;
+        k_update_faces<R><<<grid_for(fl, blk), blk, 0, s>>>(b, C.P, S, O, C.w, fl, C.sc, C.oomf);
         // RingAverage's magnetic part takes the new fluxes alone, and only CellBoris
         // looks at the field before it: here it runs beside the flux sweeps, and the
         // update finds the averaged fluxes (96 x 96 x 128 cells: 65 us of small launches
@@ -3289,15 +3273,8 @@ template <class R> void launch_step(const Ctx<R>& C, int cur, cudaStream_t s) {
         L();
     }, fold);
 }
-// Before the first step of a call: the scalars, which the host may have set, and
-// (slots) the last layers of the other state buffer
-template <class R> void launch_begin(const Ctx<R>& C, int cur, bool slots, cudaStream_t s) {
-    const GamBox& b = C.b;
-    k_step_begin<<<1, 1, 0, s>>>(C.sc);
-    if (!slots || C.oomf) return;  // with ooState the update copies every face
-    const long n = (b.Ni + 1L) * (b.Nj + 1 + b.Nk) + (long)b.Nj * b.Nk;
-    k_last_slots<R><<<(unsigned)((n + 127) / 128), 128, 0, s>>>(b, C.st[cur], C.st[1 - cur], C.sc);
-}
+// the scalars of the first step after the host may have set some
+template <class R> void launch_begin(const Ctx<R>& C, cudaStream_t s) { k_step_begin<<<1, 1, 0, s>>>(C.sc); }
 
 // Device time of each kernel of a step (ms, average of reps back-to-back
 // launches; ms[15]). The kernels after k_step_begin read their inputs and

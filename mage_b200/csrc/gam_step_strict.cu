@@ -14,4 +14,4 @@ void gam_strict_prepare_f64() { gam_strict::prepare<double>(); }
 void gam_strict_profile_f64(const Ctx<double>& C, int cur, cudaStream_t s, int reps, double* ms) { gam_strict::profile_step<double>(C, cur, s, reps, ms); }
 void gam_strict_phase_f64(const Ctx<double>& C, int cur, cudaStream_t s, int phase) { gam_strict::launch_step_phase<double>(C, cur, s, phase); }
 void gam_strict_halo_f64(const Ctx<double>& C, int cur, cudaStream_t s, int dside, int unpack, int copyB, void* buf) { gam_strict::launch_halo<double>(C, cur, s, dside, unpack, copyB, buf); }
-void gam_strict_begin_f64(const Ctx<double>& C, int cur, bool slots, cudaStream_t s) { gam_strict::launch_begin<double>(C, cur, slots, s); }
+void gam_strict_begin_f64(const Ctx<double>& C, cudaStream_t s) { gam_strict::launch_begin<double>(C, s); }
