@@ -1049,8 +1049,11 @@ __device__ __forceinline__ R dbdf(const GamBox& b, const Geo<R>& g, long c, int 
 }
 
 // predictor adjoint, cells: dQW, dWn, dDh, dVdV, dQB -> dGas, doGas; writes
-// aB = volume * dQB (the adjoint of the half-state Bxyz) for the face pass
-template <class R>
+// aB = volume * dQB (the adjoint of the half-state Bxyz) for the face pass. ONE:
+// the two are one array, as a caller whose State is its oState too may have it (a
+// kernel of its own: the choice at run time costs the face kernel 15 registers and
+// half of its warps)
+template <class R, bool ONE>
 __global__ void __launch_bounds__(128) k_predict_adj_cells(GamBox b, DevParams<R> P, Geo<R> g, StateBuf<R> cur,
                                                            StateBuf<R> old, double pdt, double odt, Work<R> dw,
                                                            R* dGas, R* doGas, R* aB) {
@@ -1126,16 +1129,17 @@ __global__ void __launch_bounds__(128) k_predict_adj_cells(GamBox b, DevParams<R
     for (int v = 0; v < 5; v++) aWn[v] = dWn[v];
     bc2p_adj(dF, pF, gm1, Q, aWn, aQ);
     for (int v = 0; v < 5; v++) {
-        dGas[v * fs + c] = (R)gQ[v] + (R)aQ[v];
-        doGas[v * fs + c] = (R)goQ[v] + (R)aoQ[v];
+        const R n = (R)gQ[v] + (R)aQ[v];
+        dGas[v * fs + c] = n;
+        doGas[v * fs + c] = (ONE ? n : (R)goQ[v]) + (R)aoQ[v];
     }
     if (P.doMHD)
         for (int x = 0; x < 3; x++) aB[x * fs + c] = (R)(vol * dB[x]);
 }
 
 // predictor adjoint, faces: dabh, dBnf, dbn and the Bxyz adjoints of the two
-// cells sharing the face -> dmf, domf
-template <class R>
+// cells sharing the face -> dmf, domf (ONE: see k_predict_adj_cells)
+template <class R, bool ONE>
 __global__ void __launch_bounds__(256) k_predict_adj_faces(GamBox b, DevParams<R> P, Geo<R> g, double pdt, double odt,
                                                            Work<R> dw, const R* __restrict__ aB, R* dmf, R* domf) {
     using A = R;
@@ -1199,8 +1203,9 @@ __global__ void __launch_bounds__(256) k_predict_adj_faces(GamBox b, DevParams<R
         const A rvu = (A)1.0 / rvol[d];
 #pragma unroll
         for (int x = 0; x < 3; x++) ahm += aUp[d][x] * rvu * wUp[d][x];
-        dmf[d * fs + c] = (R)gm[d] + (R)(ahm + ahm * pr + bl[d] * rAm);
-        domf[d * fs + c] = (R)gom[d] + (R)(-ahm * pr);
+        const R nm = (R)gm[d] + (R)(ahm + ahm * pr + bl[d] * rAm);
+        dmf[d * fs + c] = nm;
+        domf[d * fs + c] = (ONE ? nm : (R)gom[d]) + (R)(-ahm * pr);
     }
 }
 
@@ -1943,10 +1948,10 @@ int predict_call(const gam_params* p, const void* const* st, const void* const* 
         dw.QW = (R*)din[0]; dw.Wn = (R*)din[1]; dw.Dh = (R*)din[2]; dw.VdV = (R*)din[3]; dw.QB = (R*)din[4];
         dw.abh = (R*)din[5]; dw.Bnf = (R*)din[6]; dw.bn = (R*)din[7];
         const dim3 blk(32, 4, 1);
-        k_predict_adj_cells<R><<<grid3(cells, blk), blk, 0, s>>>(b, P, g, cur, old, pdt, odt, dw, (R*)dst[0],
-                                                                  (R*)dst[2], (R*)aB);
-        k_predict_adj_faces<R><<<grid3(all, blk), blk, 0, s>>>(b, P, g, pdt, odt, dw, (const R*)aB, (R*)dst[1],
-                                                                (R*)dst[3]);
+        auto cellsAdj = dst[0] == dst[2] ? k_predict_adj_cells<R, true> : k_predict_adj_cells<R, false>;
+        auto facesAdj = dst[1] == dst[3] ? k_predict_adj_faces<R, true> : k_predict_adj_faces<R, false>;
+        cellsAdj<<<grid3(cells, blk), blk, 0, s>>>(b, P, g, cur, old, pdt, odt, dw, (R*)dst[0], (R*)dst[2], (R*)aB);
+        facesAdj<<<grid3(all, blk), blk, 0, s>>>(b, P, g, pdt, odt, dw, (const R*)aB, (R*)dst[1], (R*)dst[3]);
     }
     return cudaGetLastError() == cudaSuccess ? GAM_OK : GAM_ECUDA;
 }

@@ -51,3 +51,25 @@ def test_ragged_whole_step(N, dtype, tol):
     assert num <= tol * den, num / den
     for a, b in zip(kept, again):
         assert torch.equal(a, b), float((a - b).abs().max())
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32], ids=["fp64", "fp32"])
+def test_one_array_for_both_adjoints(dtype):
+    """A start whose State is its oState: with one array given for both adjoints, the
+    adjoint adds both into it."""
+    N = (24, 9, 13)
+    gpu = GameraGPU(GamParams(*N))
+    gpu.set_geometry(grids.warped_periodic_corners(*N))
+    gpu.init_blast_wave()
+    st = gpu.download_state(old=False)
+    g = Grid(DiffParams(*N), gpu.get_geometry_arrays(), dtype=dtype, device="cuda")
+    gas, mf = g.cell_box(st["Gas"]), g.face_box(st["magFlux"])
+    cur = {"Gas": gas, "mf": mf, "B": g.bxyz(mf)}
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    dn = {k: torch.randn(cur[k].shape, generator=gen, dtype=dtype, device="cuda") for k in ("Gas", "mf")}
+    ws = WholeStep(g)
+    ws.forward(cur, cur, DT, DT)
+    d = ws.adjoint(cur, cur, DT, DT, dn, saved=True)
+    zG, zM = torch.zeros_like(gas), torch.zeros_like(mf)
+    both = ws.adjoint(cur, cur, DT, DT, dn, [zG, zM, zG, zM], saved=True)
+    assert torch.equal(both[0], d[0] + d[2]) and torch.equal(both[1], d[1] + d[3])
