@@ -89,15 +89,21 @@ def test_sweep_within_its_memory(monkeypatch, nsteps, seg, fit, room):
 def test_areas_leave_the_sweeps_own_memory(monkeypatch):
     ws = WholeStep.__new__(WholeStep)
     ws.work = types.SimpleNamespace(is_cuda=True, device="cuda:0", numel=lambda: 1 << 30)
-    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda d: (100 << 30, 180 << 30))
-    monkeypatch.setattr(torch.cuda, "memory_reserved", lambda d: 8 << 30)
-    monkeypatch.setattr(torch.cuda, "memory_allocated", lambda d: 4 << 30)
+    free, held, asked = [100 << 30], [4 << 30], []
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda d: asked.append(1) or (free[0], 180 << 30))
+    monkeypatch.setattr(torch.cuda, "memory_stats_as_nested_dict", lambda d: {
+        "reserved_bytes": {"all": {"current": held[0] + (3 << 30)}}, "allocated_bytes": {"all": {"current": 3 << 30}}})
     assert ws.areas_that_fit(99) == 17                 # 16 GiB
     assert ws.areas_that_fit(99, 64 << 30) == 11       # a quarter of 40 GiB
     assert ws.areas_that_fit(99, 200 << 30) == 1
-    assert ws.areas_that_fit(3) == 3
-    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda d: (0, 180 << 30))
-    assert ws.areas_that_fit(3) == 2                   # (8 - 4) / 4 GiB, of the allocator's own
+    assert ws.areas_that_fit(6) == 6 and len(asked) == 4
+    assert ws.areas_that_fit(5) == 5 and len(asked) == 4   # what the allocator holds
+    free[0] = 0
+    assert ws.areas_that_fit(6) == 2                   # a quarter of 4 GiB, of the allocator's own
+    assert ws.areas_that_fit(5, 1) == 1
+    held[0] = 30 << 30
+    assert ws.areas_that_fit(99, 14 << 30) == 17 and len(asked) == 6
+    held[0] = 0
     ws.work.numel = lambda: 1 << 28
-    assert ws.areas_that_fit(5, 99 << 30) == 5         # 1 GiB: not looked at
+    assert ws.areas_that_fit(5, 99 << 30) == 5 and len(asked) == 6  # 1 GiB: not looked at
     assert ws.areas_that_fit(6, 99 << 30) == 1
