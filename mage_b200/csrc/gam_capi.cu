@@ -955,7 +955,7 @@ extern "C" int gam_step(gam_handle* h, int32_t nsteps, double* dt, double* t) {
     // host-side range with the reference's priority clock label (gamapp.F90:96-99)
     nvtxRangePushA("Gamera");
     CK(h, cudaEventRecord(h->ev0, h->s));
-    launch_begin(h);
+    if (nsteps > 0) launch_begin(h);
     for (int n = 0; n < nsteps; n++) CK(h, cudaGraphLaunch(h->graph[(cur0 + n) & 1], h->s));
     CK(h, cudaEventRecord(h->ev1, h->s));
     nvtxRangePop();

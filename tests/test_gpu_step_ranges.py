@@ -63,3 +63,16 @@ def test_slots_past_the_last_cell(oracle_built, N, ab3):
             assert np.array_equal(s[k], o.array(k)), (n, k)
         if ab3:
             assert np.array_equal(g.get_oostate()["oomagFlux"], o.array("oomagFlux")), n
+
+
+def test_no_steps_change_nothing(oracle_built):
+    """A call for no steps leaves the times alone, also where a step would first move
+    oState's time one dt back (mhdgroup.F90:25-31)."""
+    o, _ = make_oracle("ot", (16, 4, 4), variant="gm")
+    g = gpu_from_oracle(o, strict=True)
+    gas, mf, dt = o.array("Gas"), o.array("magFlux"), o.scalars()["dt"]
+    g.upload_state(gas, mf, o.array("Bxyz"), gas, mf, 1.0, 1.0, dt, 5)
+    g.step_gamera(0)
+    s = g.download_state()
+    assert (s["time"], s["otime"], s["dt"], s["ts"]) == (1.0, 1.0, dt, 5)
+    assert np.array_equal(s["Gas"], gas) and np.array_equal(s["omagFlux"], mf)
