@@ -123,12 +123,18 @@ template <class R> struct Quot {
         const R q = a * r, e = fma(-d, q, a);
         return e - e == (R)0 ? fma(e, r, q) : q;  // an infinite quotient stays infinite
     }
+    // the same for a finite quotient; NaN for another
+    __device__ __forceinline__ R close_finite(R a, R d) const {
+        const R q = a * r;
+        return fma(fma(-d, q, a), r, q);
+    }
 #else
     R d;
     __device__ __forceinline__ explicit Quot(R dd) : d(dd) {}
     __device__ __forceinline__ Quot(R dd, R) : d(dd) {}
     __device__ __forceinline__ R operator()(R a) const { return a / d; }
     __device__ __forceinline__ R close(R a, R) const { return a / d; }
+    __device__ __forceinline__ R close_finite(R a, R) const { return a / d; }
 #endif
     template <int N> __device__ __forceinline__ void many(const R* a, R* o) const {
 #pragma unroll
@@ -142,6 +148,7 @@ template <> struct Quot<double> {
     __device__ __forceinline__ Quot(double d, double rd) : q(d, rd) {}
     __device__ __forceinline__ double operator()(double a) const { return q(a); }
     __device__ __forceinline__ double close(double a, double) const { return q(a); }
+    __device__ __forceinline__ double close_finite(double a, double) const { return q(a); }
     template <int N> __device__ __forceinline__ void many(const double* a, double* o) const { q.many<N>(a, o); }
 };
 #endif
@@ -245,10 +252,11 @@ __device__ __forceinline__ R pdm1(R pdmb, R q0, R q1, R q2, R qI) {
     R dqL = qN - q1;
     return qN - s1 * rmax((R)0, fabs(dqL) - s01 * fabs(dq0));
 }
-// PDM on both sides of a face between the cells v1 and v2, for the
-// interpolants QL and QR (the same one in 8CENT): the values of pdm1, which are
-// pdmLR's too (its right state is its left one with the stencil mirrored; where
-// mirroring a zero difference changes its sign, the term it selects is zero).
+// PDM on both sides of a face between the cells v1 and v2, for the interpolants QL
+// and QR: pdmLR's states with QL in 8CENT, in Up7LRs pdm1's and its from the other
+// side. The right state is the left one with the stencil mirrored; where mirroring a
+// zero difference changes its sign, the term it selects is zero. The two differ
+// beside a cell that is not a number: pdmLR's bounds are then v1, mirrored ones v2.
 // FP64: the signs of the differences are taken from their bits and twice the
 // limiter difference enters by one fma (exact, since 2|x| is): 15 FP64
 // instructions instead of 22.
@@ -261,19 +269,23 @@ __device__ __forceinline__ double pdm_cut(double pd, double v, double qN, double
     return qN - __hiloint2double(__double2hiint(m) ^ (sv & (int)0x80000000), __double2loint(m));
 }
 __device__ __forceinline__ void pdm_both(double pdmb, double v0, double v1, double v2, double v3, double QL, double QR,
-                                         double& L, double& U) {
+                                         bool up7, double& L, double& U) {
     const double d1 = v2 - v1, pd0 = pdmb * (v1 - v0), pd2 = pdmb * (v2 - v3);
-    const bool dn = __double2hiint(d1) < 0;
+    const bool dn = ((unsigned)__double2hiint(d1) ^ 0x80000000u) < 0x7ff00001u;  // negative, and a number
     const double hi = dn ? v1 : v2, lo = dn ? v2 : v1;
-    const double qL = rmax(lo, rmin(QL, hi)), qR = rmax(lo, rmin(QR, hi));
+    const double qL = rmax(lo, rmin(QL, hi)), q7 = rmin(hi, rmax(lo, QR)), qR = up7 ? q7 : qL;
     const double vd = pdmb * d1;
     L = pdm_cut(pd0, v1, qL, vd);
     U = pdm_cut(pd2, v2, qR, -vd);
 }
 __device__ __forceinline__ void pdm_both(float pdmb, float v0, float v1, float v2, float v3, float QL, float QR,
-                                         float& L, float& U) {
-    L = pdm1(pdmb, v0, v1, v2, QL);
-    U = pdm1(pdmb, v3, v2, v1, QR);
+                                         bool up7, float& L, float& U) {
+    const float hi = rmax(v1, v2), lo = rmin(v1, v2);
+    const float qL = rmax(lo, rmin(QL, hi)), q7 = rmax(rmin(v2, v1), rmin(QR, rmax(v2, v1))), qR = up7 ? q7 : qL;
+    const float d0 = pdmb * (v1 - v0), d1 = pdmb * (v2 - v1), d2 = pdmb * (v3 - v2);
+    const float s0 = sgn1(d0), s1 = sgn1(d1), s2 = sgn1(d2);
+    L = qL - s1 * rmax(0.0f, fabs(qL - v1) - fabs(s0 + s1) * fabs(d0));
+    U = qR + s1 * rmax(0.0f, fabs(v2 - qR) - fabs(s1 + s2) * fabs(d2));
 }
 template <class R> __device__ __forceinline__ R central8(const R* q) {
     R s = (R)0;
@@ -882,16 +894,17 @@ __device__ __forceinline__ void edge_emf(const GamBox& b, const DevParams<R>& P,
         for (int x = 0; x < 3; x++) VC[x] = num[2 + x] / (R)TINY;
     }
     R bT1L, bT1R, bT2L, bT2R;
-    {
-        const R* p = sm + T_::at(3, tx, ty, tz);
-        constexpr int s = T_::str(3, dT2);
-        pdm_both(P.pdmb, p[-2 * s], p[-s], p[0], p[s], quo[0], quo[1], bT1L, bT1R);
-    }
-    {
-        const R* p = sm + T_::at(4, tx, ty, tz);
-        constexpr int s = T_::str(4, dT1);
-        pdm_both(P.pdmb, p[-2 * s], p[-s], p[0], p[s], q2[0], q2[1], bT2L, bT2R);
-    }
+    auto limit = [&](bool up7) {
+        const R *p1 = sm + T_::at(3, tx, ty, tz), *p2 = sm + T_::at(4, tx, ty, tz);
+        constexpr int r1 = T_::str(3, dT2), r2 = T_::str(4, dT1);
+        pdm_both(P.pdmb, p1[-2 * r1], p1[-r1], p1[0], p1[r1], quo[0], quo[1], up7, bT1L, bT1R);
+        pdm_both(P.pdmb, p2[-2 * r2], p2[-r2], p2[0], p2[r2], q2[0], q2[1], up7, bT2L, bT2R);
+    };
+    // each with its own code: a choice inside costs the FMA form's edges 6 us of 250 (192^3)
+    if (P.up7)
+        limit(true);
+    else
+        limit(false);
     R v1 = VC[0] * m.t1[0] + VC[1] * m.t1[1] + VC[2] * m.t1[2];
     R v2 = VC[0] * m.t2[0] + VC[1] * m.t2[1] + VC[2] * m.t2[2];
     R vDiff = Mth<R>::sqrt_(v1 * v1 + v2 * v2);
@@ -921,8 +934,9 @@ __device__ __forceinline__ void edge_emf(const GamBox& b, const DevParams<R>& P,
     R vA = qdiv(Mth<R>::sqrt_(b1 * b1 + b2 * b2), Mth<R>::sqrt_(Dc));
     if (P.doBoris) vA = boris_speed((R)P.Ca, vA);
     vDiff = vDiff + vA;
-    // FP32 divides: 192^3, the I edges 150 us, 156 with the corrected product
-    const R vMax = sizeof(R) == 4 ? P.CFL * m.edge / dt : qdt.close(P.CFL * m.edge, dt);
+    // FP32 divides: 192^3, the I edges 150 us, 156 with the corrected product. (A bound
+    // that is infinite, or not a number, bounds nothing.)
+    const R vMax = sizeof(R) == 4 ? P.CFL * m.edge / dt : qdt.close_finite(P.CFL * m.edge, dt);
     vDiff = rmin(vDiff, vMax);
     R e = -(v1 * b2 - v2 * b1) + P.Vd0 * vDiff * Jd;
     w.E[eD * fs + c] = e * m.edge;
@@ -1201,7 +1215,7 @@ __device__ __forceinline__ void flux_face(const GamBox& b, const DevParams<R>& P
             const int v = n0 + n;
             const R* p = pL + v * T_::LN * T_::QX;
             R l, u;
-            pdm_both(P.pdmb, p[0], p[st], p[2 * st], p[3 * st], Qi[n], Qi[GRP + n], l, u);
+            pdm_both(P.pdmb, p[0], p[st], p[2 * st], p[3 * st], Qi[n], Qi[GRP + n], P.up7, l, u);
             if (v < 5) {
                 WL[v] = l;
                 WR[v] = u;
