@@ -3198,7 +3198,7 @@ template <class R, class F> void for_each_kernel(const Ctx<R>& C, int cur, cudaS
         }
         if (C.P.doBoris)
             k_update_cells<R, sizeof(R) == 8 ? 6 : 8, true><<<grid_for(cells, blk), blk, 0, s>>>(b, C.P, C.g, S, O, C.w, C.sc, C.gamma, C.gm1, cells, fold);
-        else  // strict: 5 blocks/SM (792 us at 192^3; 6: 836; dipole of 1.2e6 cells 158, 6: 171); the other forms 8
+        else  // strict: 5 blocks/SM (792 us at 192^3; 6: 836; dipole of 1.2e6 cells 158, 6: 171); the other forms 8 (FMA: 643 us; 7: 650, 6: 710)
             k_update_cells<R, GAM_STRICT_KERNELS ? 5 : 8><<<grid_for(cells, blk), blk, 0, s>>>(b, C.P, C.g, S, O, C.w, C.sc, C.gamma, C.gm1, cells, fold);
         if (C.P.ring.on) {  // RingAverage (mhdgroup.F90:69-74)
             if (C.P.doMHD && C.P.doBoris) {
